@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OUT = os.path.join(LIBDIR, "libqmc2d.so")
 
-SOURCES = ["input.cpp", "system.cpp", "io.cpp", "kernels.cu", "capi.cu", "rmc.cu", "noalloc.cu",
+SOURCES = ["input.cpp", "system.cpp", "io.cpp", "kernels.cu", "real.cu", "capi.cu", "rmc.cu", "noalloc.cu",
            "batch.cu", "estimators.cpp", "single.cu", "comb.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -93,6 +93,19 @@ cudaError_t dalloc(T **p, size_t n) {
 }
 
 
+// The orbitals of every spin as real combinations (DevSys::real_orb): an odd
+// number of plane waves, k = 0 and exact pairs +-k.
+bool real_orbitals(const qmc2d_system *sys) {
+  if (!sys->gvec || sys->gvec[0] != 0.0 || sys->gvec[1] != 0.0) return false;
+  for (int t = 0; t < sys->ntypes; t++) {
+    if (sys->np[t] > sys->ngvec) return false;
+    for (int k = 1; k + 1 < sys->np[t]; k += 2)
+      for (int d = 0; d < 2; d++)
+        if (sys->gvec[2 * k + d] != -sys->gvec[2 * (k + 1) + d]) return false;
+  }
+  return true;
+}
+
 int build_devsys(const qmc2d_system *sys, q2d::DevSys *hs, std::vector<double> *coef) {
   q2d::DevSys s{};
   s.N = sys->nptot;
@@ -166,6 +179,10 @@ int build_devsys(const qmc2d_system *sys, q2d::DevSys *hs, std::vector<double> *
   s.has_u3 = s.iu3[0][0] >= 0;
   s.has_bf = s.iub[0][0] >= 0;
   s.has_v2 = s.iv2[0][0] >= 0;
+  s.real_room = s.has_bf;
+  for (int t = 0; t < sys->ntypes; t++)
+    if (sys->np[t] % 2 == 0 || sys->np[t] > 164) s.real_room = 0;
+  s.real_orb = s.real_room && real_orbitals(sys);
   coef->clear();
   for (int t = 0; t < sys->ntables; t++) {
     const qmc2d_table &tb = sys->tables[t];
@@ -245,18 +262,19 @@ size_t handle_bytes(const qmc2d_system *sys, const q2d::DevSys &hs, size_t ncoef
   b += al(c * np, 8) + al(c, 8) + al(c * 4, 8) + al(c, 8) + al(c, 4);  // blk norm cnt wate status
   b += al(c, 8) * 2 + al(c, 4) * 4 + al(1, 4);                           // branch scratch
   b += al(c * 2 * N, 8) * 2 + al(c * nt, 8) + al(c * np, 8) + al(c, 8);  // staging
-  b += al(c * q2d::move_scratch_doubles(hs), 8) + al(np + 1, 8);
+  b += al(np + 1, 8);
   b += al(c, 8);  // inverse drift of the single-electron sweeps
   // determinants beyond shared memory: qmc2d_create moves them to HBM when
   // the walker exceeds the device's opt-in shared memory per block; this
   // count is made without a device, at the B200's 227 KB
   constexpr size_t kSmemOptinB200 = 232448;
   const size_t smem = std::max(q2d::move_smem_bytes(hs), q2d::eval_smem_bytes(hs));
+  q2d::DevSys g = hs;
   if (hs.gmat || (hs.has_bf && smem + sizeof(q2d::DevSys) > kSmemOptinB200)) {
-    q2d::DevSys g = hs;
     g.gmat = 1;
     b += al(c * q2d::gmat_doubles(g), 8);
   }
+  b += al(c * q2d::move_scratch_doubles(g), 8);
   return b;
 }
 
@@ -349,6 +367,15 @@ extern "C" int qmc2d_create(const qmc2d_system *sys, const qmc2d_options *opt,
   if ((e = dalloc(&h->ds, 1)) != cudaSuccess) return fail(cuda_fail(e, "alloc"));
   cudaMemcpy(h->ds, &h->hs, sizeof(q2d::DevSys), cudaMemcpyHostToDevice);
   int cap = h->cap, N = h->N, nt = h->nt, np = h->nprops;
+  // the move scratch, without room for real orbitals when that does not fit
+  // beside what is allocated
+  e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
+  if (e == cudaErrorMemoryAllocation && h->hs.real_room && !h->hs.gmat) {
+    cudaGetLastError();
+    h->hs.real_room = h->hs.real_orb = 0;
+    e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
+  }
+  if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
   for (int k = 0; k < 2; k++)
     if ((st = alloc_pop(&h->pop[k], cap, N, nt, np))) return fail(st);
   if ((e = dalloc(&h->d_blk, (size_t)cap * np)) != cudaSuccess ||
@@ -368,7 +395,6 @@ extern "C" int qmc2d_create(const qmc2d_system *sys, const qmc2d_options *opt,
       (e = dalloc(&h->d_h, (size_t)cap * nt)) != cudaSuccess ||
       (e = dalloc(&h->d_p, (size_t)cap * np)) != cudaSuccess ||
       (e = dalloc(&h->d_s, (size_t)cap)) != cudaSuccess ||
-      (e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs))) != cudaSuccess ||
       (e = dalloc(&h->d_blksum, (size_t)np + 1)) != cudaSuccess ||
       (e = dalloc(&h->d_sdrift, (size_t)cap)) != cudaSuccess)
     return fail(cuda_fail(e, "cudaMalloc"));
@@ -484,6 +510,7 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   CK(join_side(h));
   q2d::MoveArgs a{};
   a.nw = h->nw;
+  a.real = move_real(h) ? 1 : 0;
   a.scr = h->d_mscr;
   a.delta = h->hs.delta > 0.0 ? h->hs.delta : 0.01;
   a.seed = h->seed;
@@ -545,7 +572,9 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   // inversion layout of the determinant section, timed on the evaluation
   // kernel over the population's configurations (into the staging buffers;
   // the population is not changed)
-  if ((h->tune_scope & 4) && h->hs.has_bf && !h->hs.gmat) {
+  if ((h->tune_scope & 4) && h->hs.real_orb) {
+    h->hs.tune_inv = 0;  // the real-orbital route, which has no layouts
+  } else if ((h->tune_scope & 4) && h->hs.has_bf && !h->hs.gmat) {
     double best_inv = 1e300;
     int bi = 0;
     for (int layout = 0; layout < 3; layout++) {
@@ -611,6 +640,7 @@ extern "C" int qmc2d_update_twist(qmc2d_handle *h, const qmc2d_system *sys) {
   CK(cudaMemcpyAsync(h->d_gvec, sys->gvec, sizeof(double) * 2 * sys->ngvec,
                      cudaMemcpyHostToDevice, h->stream));
   h->hs.ngvec = sys->ngvec;
+  h->hs.real_orb = h->hs.real_room && real_orbitals(sys);
   CK(cudaMemcpyAsync(h->ds, &h->hs, sizeof(q2d::DevSys), cudaMemcpyHostToDevice, h->stream));
   // sys->gvec is replaced by the next qmc2d_system_set_twist: finish reading it
   CK(cudaStreamSynchronize(h->stream));
@@ -916,7 +946,8 @@ static int run_moves(qmc2d_handle *h, int nstp, int dmc, double delta, double et
   a.cnt = h->d_cnt;
   a.wate = dmc ? h->d_wate : nullptr;
   a.status = h->d_status;
-  a.orb_inv = move_orb_inv(h) ? 1 : 0;
+  a.real = move_real(h) ? 1 : 0;
+  a.orb_inv = !a.real && move_orb_inv(h) ? 1 : 0;
   if (h->hs.delta != delta && h->hs.adrift != 0.0) {
     h->hs.delta = delta;
     CK(cudaMemcpyAsync(h->ds, &h->hs, sizeof(q2d::DevSys), cudaMemcpyHostToDevice, h->stream));
@@ -928,7 +959,7 @@ static int run_moves(qmc2d_handle *h, int nstp, int dmc, double delta, double et
       ProfScope ps(h, QMC2D_KERNEL_PAIRS, h->stream);
       CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));
     }
-    if (a.orb_inv) {
+    if (a.orb_inv || a.real) {
       ProfScope ps(h, QMC2D_KERNEL_ORB_INV, h->stream);
       CK(q2d::launch_orb_inv(h->hs, h->ds, a, h->stream));
     }

@@ -75,6 +75,15 @@ struct DevSys {
   // terms and the determinant's drift and Laplacian come from the diagonals
   // of F and D2 without the cross-term GEMM.
   int bf_zero;
+  // Real orbitals (set by the handle): backflow determinants of an odd number
+  // of plane waves per spin that are k = 0 and pairs +-k, gvec rows 2 p + 1
+  // and 2 p + 2 exact negatives (the Gamma point). Moves and evaluations
+  // then take the real-orbital kernels (real_det.cuh) unless the caller has
+  // chosen a complex layout (qmc2d_set_inversion, qmc2d_set_move_inversion).
+  int real_orb;
+  // The scratch has room for them (odd spins, fixed at create time: a twist
+  // can be set and taken back later).
+  int real_room;
   // Every Ewald k vector on the reciprocal lattice, k = 2 pi (n1 / Lx,
   // n2 / Ly) to 1e-14 (set by the handle; |n1| <= rk_p1, |n2| <= rk_p2): the
   // pair kernels form rho_k from per-particle tables of exp(2 pi i p x / L)

@@ -79,6 +79,13 @@ inline bool move_orb_inv(const qmc2d_handle *h) {
   return q2d::orb_inv_pays(h->hs, h->nw, h->nsm, need);
 }
 
+// Whether this handle's moves take the real-orbital route (real_det.cuh): at
+// every population size it is the faster one; an inversion layout or a move
+// inversion mode chosen by the caller keeps the complex kernels.
+inline bool move_real(const qmc2d_handle *h) {
+  return h->hs.real_orb && h->hs.tune_inv == 0 && h->move_inv_mode == 1;
+}
+
 // Orders the handle's stream after the side copies of the last
 // qmc2d_population_load_async (nothing when none are pending). Every entry
 // point that touches the population calls it first; a move calls it after

@@ -13,6 +13,7 @@
 #include <utility>
 
 #include "kernels.cuh"
+#include "real_det.cuh"
 #include "walker_eval.cuh"
 
 namespace q2d {
@@ -91,7 +92,8 @@ size_t gmat_doubles(const DevSys &s) {
   if (!s.gmat) return 0;
   size_t g = 0;
   eval_carve(s, nullptr, nullptr, nullptr, &g);
-  return ((g + 7) / 8 + 31) & ~size_t(31);
+  const size_t d = ((g + 7) / 8 + 31) & ~size_t(31);
+  return s.real_room ? std::max(d, (real_layout(s).end + 31) & ~size_t(31)) : d;
 }
 
 // ------------------------------------------------------------- the move
@@ -168,10 +170,13 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 //
 // R is the precision of the u2 and v2 pair terms (qmc2d_set_precision), LG
 // the lanes per particle of the pair passes (4, 8 or 16: a launch choice,
-// DevSys::tune_lanes).
-template <class R, int G, int LG>
+// DevSys::tune_lanes). kJ: the Jacobian blocks of the real-orbital route
+// (real_det.cuh) instead of the pairs' spline values; xe (kJ only) the
+// configurations to evaluate instead of a proposal.
+template <class R, int G, int LG, bool kJ>
 __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(const DevSys *sp, DevPop pop,
-                                                                    MoveArgs a, int stage_rows) {
+                                                                    MoveArgs a, int stage_rows,
+                                                                    const double *xe) {
   constexpr int kPairGroups = G, kPairThreads = G * kThreads;
   __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
@@ -204,6 +209,10 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(const DevSys
     long long tph = clock64();
     double wo = 0.0;
     for (int j = tid; j < N2; j += kThreads) {
+      if (kJ && xe) {
+        m.x[j] = xe[(size_t)w * N2 + j];
+        continue;
+      }
       int ti = type_of(S, j >> 1);
       double var = 2.0 * S.hbs2m[ti] * a.delta, vari = 1.0 / var;
       double2 u = uniform2(a.seed, (uint32_t)j, (uint32_t)w, step, 0u);
@@ -214,12 +223,16 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(const DevSys
     const double wold = block_sum_t<kThreads>(wo, m.red, sync, tid);
     phase_mark(S, PH_PROPOSE, tph, tid == 0);
     double *o = a.scr + (size_t)w * L.stride;
-    double *pout = S.has_bf ? o + L.pair : nullptr;
+    double *pout = !S.has_bf ? nullptr
+                   : !kJ     ? o + L.pair
+                   : S.bf_zero ? nullptr
+                   : S.gmat    ? S.gmat_base + (size_t)w * S.gmat_stride
+                               : o + L.pair;  // as real_base()
     if (stage_rows)
-      eval_pairs<kThreads, true, R, GroupSync, LG>(S, m, tph, pout, (const R *)rows_s, sync,
-                                                   tid);
+      eval_pairs<kThreads, true, R, GroupSync, LG, kJ>(S, m, tph, pout, (const R *)rows_s, sync,
+                                                       tid);
     else
-      eval_pairs<kThreads, false, R, GroupSync, LG>(S, m, tph, pout, rows_g, sync, tid);
+      eval_pairs<kThreads, false, R, GroupSync, LG, kJ>(S, m, tph, pout, rows_g, sync, tid);
     pair_rhok<LG>(S, m, tid, kThreads, sync);
     sync();
     for (int j = tid; j < 4 * S.nk; j += kThreads) o[L.rhok + j] = m.rhok[j];
@@ -569,6 +582,170 @@ __global__ void __launch_bounds__(kThreads, kSeq ? 3 : 2) move_kernel(const DevS
   }
 }
 
+// --------------------------------------------------- real orbitals
+// The pair passes' sums of walker w into shared memory, the determinant sums
+// zeroed (asynchronous 8-byte copies; the caller waits).
+__device__ __forceinline__ void load_real_sums(const DevSys &S, const EvalSmem &m,
+                                               const double *o, const MoveScratch &L) {
+  const int N = S.N, tid = threadIdx.x;
+  for (int j = tid; j < 2 * N; j += kThreads) {
+    cp_async8(m.x + j, o + L.x + j);
+    cp_async8(m.g + j, o + L.g + j);
+  }
+  for (int j = tid; j < N; j += kThreads) {
+    cp_async8(m.lap + j, o + L.lap + j);
+    cp_async8(m.ltf + j, o + L.ltf + j);
+    cp_async8(m.vp + j, o + L.vp + j);
+    m.lapd[j] = 0.0;
+    m.ph2[j] = 0.0;
+    m.ph2d[j] = 0.0;
+  }
+}
+
+// What move_real_kernel keeps beside the evaluation: the old positions and
+// drift, the new properties, -lap per type, the sign.
+struct MoveRealSmem {
+  double *xo, *go, *pn, *hn, *sc;
+};
+__host__ __device__ inline size_t move_real_carve(const DevSys &s, char *base, MoveRealSmem *m) {
+  size_t off = 0;
+  auto take = [&](size_t doubles) -> double * {
+    char *p = base ? base + off : nullptr;
+    off += align16(sizeof(double) * doubles);
+    return (double *)p;
+  };
+  MoveRealSmem t;
+  t.xo = take(2 * s.N);
+  t.go = take(2 * s.N);
+  t.pn = take(s.nprops);
+  t.hn = take(2);
+  t.sc = take(2);
+  if (m) *m = t;
+  return off;
+}
+size_t move_real_smem_bytes(const DevSys &s) {
+  return real_carve(s, nullptr, nullptr) + move_real_carve(s, nullptr, nullptr);
+}
+size_t eval_real_smem_bytes(const DevSys &s) {
+  return real_carve(s, nullptr, nullptr) + align16(sizeof(double) * (s.nprops + 4));
+}
+
+// The rest of a move after launch_real_det: the assembly, the reverse move,
+// Metropolis, the averages. Latency-bound (reductions, transcendentals, the
+// records' reads and writes); four CTAs per SM overlap it.
+__global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const DevSys *sp, DevPop pop,
+                                                                MoveArgs a, RealArgs ra,
+                                                                MoveScratch L) {
+  __shared__ DevSys S;
+  extern __shared__ __align__(16) char smem[];
+  load_sys(S, sp);
+  EvalSmem m;
+  const size_t off = real_carve(S, smem, &m);
+  MoveRealSmem v;
+  move_real_carve(S, smem + off, &v);
+  const int w = blockIdx.x, tid = threadIdx.x;
+  if (w >= a.nw) return;
+  const int N2 = 2 * S.N, np = S.nprops, nt = S.nt;
+  const double *o = a.scr + (size_t)w * L.stride;
+  load_real_sums(S, m, o, L);
+  for (int j = tid; j < N2; j += kThreads) {
+    cp_async8(v.xo + j, pop.x + (size_t)w * N2 + j);
+    cp_async8(v.go + j, pop.g + (size_t)w * N2 + j);
+  }
+  const double wold = o[L.wold];
+  const double po_ltf = pop.p[(size_t)w * np + QMC2D_JLTF];
+  const double po_et = pop.p[(size_t)w * np + QMC2D_JETOT];
+  const double age0 = pop.age[w];
+  double wate = (a.dmc && !a.first) ? a.wate[w] : 1.0;
+  long long tph = clock64();
+  const int status = eval_det_real(S, m, v.hn, v.pn, &v.sc[0], tph, o, L, ra,
+                                   real_base(ra, w));
+  // reverse move (reptation.f:4660-4674)
+  double wn = 0.0;
+  for (int j = tid; j < N2; j += kThreads) {
+    int ti = type_of(S, j >> 1);
+    double var = 2.0 * S.hbs2m[ti] * a.delta, vari = 1.0 / var;
+    double chi = v.xo[j] - m.x[j] - (-var * m.g[j]);
+    wn -= chi * chi * vari;
+  }
+  const double wnew = block_sum(wn, m.red);
+  const bool forced = age0 == a.mage;
+  double p = 1.0;
+  if (!forced) {
+    p = (po_ltf - v.pn[QMC2D_JLTF]) * 2.0 + 0.5 * (wnew - wold);
+    p = exp(fmin(0.0, fmax(-50.0, p)));
+  }
+  // metropolis_test (reptation.f:2622-2659)
+  const uint32_t step = a.step0 + (a.ctr ? a.ctr[0] : 0u);
+  double xr = 1.0;
+  if (p < 1.0) xr = uniform2(a.seed, 0xFFFFFFFEu, (uint32_t)w, step, 0u).x;
+  const bool acc = p >= xr;
+  double wgt = 1.0;
+  if (a.dmc) {
+    // dmc weight (reptation.f:898-903), as in move_kernel
+    double el = acc ? 0.5 * (v.pn[QMC2D_JETOT] + po_et) : po_et;
+    if (a.ecut > 0.0) el = fmin(fmax(el, a.etrial - a.ecut), a.etrial + a.ecut);
+    double peso = exp(-S.npnorm * (el - a.etrial) * a.delta);
+    if (peso > a.mmult) peso = a.mmult;
+    wate *= peso;
+    wgt = wate;
+  }
+  phase_mark(S, PH_ACCEPT, tph);
+  if (acc)
+    for (int j = tid; j < N2; j += kThreads) {
+      pop.x[(size_t)w * N2 + j] = m.x[j];
+      pop.g[(size_t)w * N2 + j] = m.g[j];
+    }
+  // the walker's properties, the new ones if accepted, with the acceptance
+  // probability; the block sums
+  for (int j = tid; j < np; j += kThreads) {
+    const size_t i = (size_t)w * np + j;
+    double val = acc ? v.pn[j] : pop.p[i];
+    if (j == QMC2D_JACC) val = p;
+    a.blk[i] += val * wgt;
+    if (acc || j == QMC2D_JACC) pop.p[i] = val;
+  }
+  if (acc && tid < nt) pop.h[(size_t)w * nt + tid] = v.hn[tid];
+  if (tid == 0) {
+    if (acc) pop.s[w] = v.sc[0];
+    pop.age[w] = acc ? 0.0 : age0 + 1.0;
+    a.blk_norm[w] += wgt;
+    a.cnt[4 * w + 0] += acc ? 1.0 : 0.0;
+    a.cnt[4 * w + 1] += 1.0;
+    a.cnt[4 * w + 2] += forced ? 1.0 : 0.0;
+    if (status) a.cnt[4 * w + 3] += 1.0;
+    if (a.wate) a.wate[w] = wate;
+    a.status[w] |= status;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 4) eval_real_kernel(const DevSys *sp, int nw,
+                                                                RealArgs ra, MoveScratch L,
+                                                                double *g, double *hl,
+                                                                double *props, double *s,
+                                                                int *status) {
+  __shared__ DevSys S;
+  extern __shared__ __align__(16) char smem[];
+  load_sys(S, sp);
+  EvalSmem m;
+  const size_t off = real_carve(S, smem, &m);
+  double *pn = reinterpret_cast<double *>(smem + off);
+  double *hn = pn + S.nprops, *sn = hn + 2;
+  const int w = blockIdx.x;
+  if (w >= nw) return;
+  const double *o = ra.scr + (size_t)w * L.stride;
+  load_real_sums(S, m, o, L);
+  long long tph = clock64();
+  const int st = eval_det_real(S, m, hn, pn, sn, tph, o, L, ra, real_base(ra, w));
+  for (int j = threadIdx.x; j < 2 * S.N; j += kThreads) g[(size_t)w * 2 * S.N + j] = m.g[j];
+  for (int j = threadIdx.x; j < S.nprops; j += kThreads) props[(size_t)w * S.nprops + j] = pn[j];
+  if (threadIdx.x < S.nt) hl[(size_t)w * S.nt + threadIdx.x] = hn[threadIdx.x];
+  if (threadIdx.x == 0) {
+    s[w] = *sn;
+    status[w] = st;
+  }
+}
+
 // ------------------------------------------------------------- branch2
 // One block. Population-wide steps of branch2 (reptation.f:2174-2212) and
 // prov_dest's in-rank assignment (reptation.f:2260-2271) on global scratch.
@@ -812,10 +989,11 @@ cudaError_t launch_eval(const DevSys &hs, const DevSys *ds, int nw, const double
   return cudaGetLastError();
 }
 
-template <class R, int G, int LG>
+template <class R, int G, int LG, bool kJ>
 static cudaError_t launch_pairs_t(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin) {
-  const void *k = (const void *)pairs_kernel<R, G, LG>;
+                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
+                                  const double *xe) {
+  const void *k = (const void *)pairs_kernel<R, G, LG, kJ>;
   const size_t carve = G * ((pair_carve(hs, nullptr, nullptr, kThreads) + 127) & ~size_t(127));
   const size_t rows =
       sizeof(R) * RowLayout<R>::sstride * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
@@ -832,29 +1010,31 @@ static cudaError_t launch_pairs_t(const DevSys &hs, const DevSys *ds, DevPop pop
   const int need = (a.nw + G - 1) / G;
   const int cap = nsm * (per_sm > 0 ? per_sm : 1);
   const int grid = need < cap ? need : cap;
-  pairs_kernel<R, G, LG><<<grid, G * kThreads, sm, st>>>(ds, pop, a, stage);
+  pairs_kernel<R, G, LG, kJ><<<grid, G * kThreads, sm, st>>>(ds, pop, a, stage, xe);
   return cudaGetLastError();
 }
 
-template <class R, int LG>
+template <class R, int LG, bool kJ>
 static cudaError_t launch_pairs_g(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin) {
-  return hs.tune_groups == 1 ? launch_pairs_t<R, 1, LG>(hs, ds, pop, a, st, nsm, optin)
-                             : launch_pairs_t<R, 2, LG>(hs, ds, pop, a, st, nsm, optin);
+                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
+                                  const double *xe) {
+  return hs.tune_groups == 1 ? launch_pairs_t<R, 1, LG, kJ>(hs, ds, pop, a, st, nsm, optin, xe)
+                             : launch_pairs_t<R, 2, LG, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
 }
 
-template <class R>
+template <class R, bool kJ>
 static cudaError_t launch_pairs_r(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin) {
+                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
+                                  const double *xe) {
   switch (hs.tune_lanes) {
-    case 4: return launch_pairs_g<R, 4>(hs, ds, pop, a, st, nsm, optin);
-    case 16: return launch_pairs_g<R, 16>(hs, ds, pop, a, st, nsm, optin);
-    default: return launch_pairs_g<R, 8>(hs, ds, pop, a, st, nsm, optin);
+    case 4: return launch_pairs_g<R, 4, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
+    case 16: return launch_pairs_g<R, 16, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
+    default: return launch_pairs_g<R, 8, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
   }
 }
 
-cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
-                         cudaStream_t st) {
+static cudaError_t launch_pairs_x(const DevSys &hs, const DevSys *ds, DevPop pop,
+                                  const MoveArgs &a, cudaStream_t st, const double *xe) {
   if (a.nw <= 0) return cudaSuccess;
   int dev = 0, nsm = 0, optin = 0;
   cudaError_t e;
@@ -864,8 +1044,34 @@ cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const M
   if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
       cudaSuccess)
     return e;
-  return hs.pair_f32 ? launch_pairs_r<float>(hs, ds, pop, a, st, nsm, optin)
-                     : launch_pairs_r<double>(hs, ds, pop, a, st, nsm, optin);
+  if (a.real)
+    return hs.pair_f32 ? launch_pairs_r<float, true>(hs, ds, pop, a, st, nsm, optin, xe)
+                       : launch_pairs_r<double, true>(hs, ds, pop, a, st, nsm, optin, xe);
+  return hs.pair_f32 ? launch_pairs_r<float, false>(hs, ds, pop, a, st, nsm, optin, nullptr)
+                     : launch_pairs_r<double, false>(hs, ds, pop, a, st, nsm, optin, nullptr);
+}
+
+cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
+                         cudaStream_t st) {
+  return launch_pairs_x(hs, ds, pop, a, st, nullptr);
+}
+
+cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const double *x,
+                             double *g, double *hl, double *props, double *s, int *status,
+                             double *scr, cudaStream_t st) {
+  if (nw <= 0) return cudaSuccess;
+  MoveArgs a{};
+  a.nw = nw;
+  a.real = 1;
+  a.scr = scr;
+  cudaError_t e;
+  if ((e = launch_pairs_x(hs, ds, DevPop{}, a, st, x)) != cudaSuccess) return e;
+  if ((e = launch_real_det(hs, ds, nw, scr, st)) != cudaSuccess) return e;
+  const size_t sm = eval_real_smem_bytes(hs);
+  if ((e = set_smem((const void *)eval_real_kernel, sm)) != cudaSuccess) return e;
+  eval_real_kernel<<<nw, kThreads, sm, st>>>(ds, nw, real_args(hs, scr), move_scratch(hs), g, hl,
+                                             props, s, status);
+  return cudaGetLastError();
 }
 
 bool orb_inv_applies(const DevSys &hs) { return hs.split_inv && orb_inv_fits(hs); }
@@ -875,6 +1081,7 @@ bool orb_inv_pays(const DevSys &hs, int nw, int nsm, int min_per_sm) {
 
 cudaError_t launch_orb_inv(const DevSys &hs, const DevSys *ds, const MoveArgs &a,
                            cudaStream_t st) {
+  if (a.real) return launch_real_det(hs, ds, a.nw, a.scr, st);
   if (a.nw <= 0 || !a.orb_inv || !orb_inv_applies(hs)) return cudaSuccess;
   size_t wd = 0;
   for (int t = 0; t < hs.nt; t++) wd = std::max(wd, orb_inv_warp_doubles(hs.np[t]));
@@ -898,6 +1105,14 @@ cudaError_t launch_orb_inv(const DevSys &hs, const DevSys *ds, const MoveArgs &a
 cudaError_t launch_move(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
                         cudaStream_t st) {
   if (a.nw <= 0) return cudaSuccess;
+  if (a.real) {
+    const size_t sm = move_real_smem_bytes(hs);
+    cudaError_t e = set_smem((const void *)move_real_kernel, sm);
+    if (e != cudaSuccess) return e;
+    move_real_kernel<<<a.nw, kThreads, sm, st>>>(ds, pop, a, real_args(hs, a.scr),
+                                                 move_scratch(hs));
+    return cudaGetLastError();
+  }
   const bool seq = !hs.gmat && a.orb_inv && orb_inv_applies(hs) && props_buf_fits(hs);
   size_t sm = seq ? move_smem_bytes_seq(hs) : move_smem_bytes(hs);
   auto k = hs.gmat ? move_kernel<true, false>

@@ -27,6 +27,7 @@ struct MoveArgs {
   double *wate;       // nw DMC weights (product over the generation's moves)
   int *status;        // nw status words (OR-ed)
   int orb_inv;        // 1: orb_inv_kernel ran before the move kernel (its output is in scr)
+  int real;           // 1: real orbitals (launch_real_det between the pair and the move kernel)
   // Device counters {move, generation} added to step0 (and to the comb's
   // generation) when non-null: a CUDA graph replays its launches with the
   // same arguments, so the Philox counters that must advance are read here.
@@ -40,6 +41,12 @@ cudaError_t raise_smem_limit(const void *fn, size_t bytes);
 // Evaluate nw configurations x (2N each) -> g, hl, props, s.
 cudaError_t launch_eval(const DevSys &hs, const DevSys *ds, int nw, const double *x, double *g,
                         double *hl, double *props, double *s, int *status, cudaStream_t st);
+
+// The same evaluations with real orbitals through the move's kernels: the
+// pair passes into scr (nw move scratch blocks), launch_real_det, the rest.
+cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const double *x,
+                             double *g, double *hl, double *props, double *s, int *status,
+                             double *scr, cudaStream_t st);
 
 // One move of a resident population: the proposal and pair passes into the
 // move scratch (launch_pairs), the orbitals and their inversion into the

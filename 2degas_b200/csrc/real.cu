@@ -1,0 +1,962 @@
+// real.cu - determinants over real orbitals (real_det.cuh) between the pair
+// passes and the evaluation's end: orbitals, inverse and F matrices of every
+// (walker, spin), then the sums over its Jacobian blocks.
+//
+// F_a = D^-1 d_a D with D(o, j) the orbitals sqrt(2) cos(g.q_j),
+// sqrt(2) sin(g.q_j) of the pairs +-g and the constant (paho_orbitals,
+// reptation.f:10268; zgefa/zgedi :9227, :9338; slater_excitations
+// :10189-10200). Orbital o < n - 1 is the cosine (even) or sine (odd) of
+// pair o / 2, whose wave vector is gvec row o | 1; orbital n - 1 is the
+// constant 1. The derivative of a cosine is -g times its sine, of a sine g
+// times its cosine, so
+//   F_a(l, j) = sum_o Dinv(l, o) s_o g_a D(o ^ 1, j), s_o = -1 for a cosine.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "real_det.cuh"
+
+namespace q2d {
+
+namespace {
+
+// The pivot key of |x|: the top word of the double with its low byte
+// replaced by 255 - r, so ties within 2^-12 go to the lowest row; every
+// unused row's key is nonzero, a zero or NaN column included.
+__device__ __forceinline__ unsigned pivot_key(double x, int r, bool on) {
+  return on ? ((unsigned)__double2hiint(fabs(x)) & ~0xFFu) | (unsigned)(255 - r) : 0u;
+}
+
+constexpr double kSqrt2 = 1.4142135623730951;
+
+__host__ __device__ inline int odd4(int c) {  // smallest odd multiple of 4 that holds c
+  return ((c + 3) / 4 | 1) * 4;
+}
+
+// (s_o g_x, s_o g_y) of orbital o of n.
+__device__ __forceinline__ double2 orbital_g(const double *gvec, int o, int n) {
+  if (o >= n - 1) return make_double2(0.0, 0.0);
+  const double s = o & 1 ? 1.0 : -1.0;
+  return make_double2(s * __ldg(gvec + 2 * (o | 1)), s * __ldg(gvec + 2 * (o | 1) + 1));
+}
+
+// Orbital rows of a spin (row o at at(o, j)) by threads t, t + nthr, ...: one
+// sincos for the two rows of a pair.
+template <class At>
+__device__ __forceinline__ void orbital_rows(const RealArgs &a, const double *q, int n, int t,
+                                             int nthr, At at) {
+  for (int e = t; e < (n - 1) / 2 * n; e += nthr) {
+    const int p = e / n, j = e - p * n;
+    const double2 x = *reinterpret_cast<const double2 *>(q + 2 * j);
+    double sv, cv;
+    sincos(x.x * __ldg(a.gvec + 4 * p + 2) + x.y * __ldg(a.gvec + 4 * p + 3), &sv, &cv);
+    at(2 * p, j) = kSqrt2 * cv;
+    at(2 * p + 1, j) = kSqrt2 * sv;
+  }
+  for (int j = t; j < n; j += nthr) at(n - 1, j) = 1.0;
+}
+
+// F_x and F_y of kR row tiles (from l0) and kT column tiles (from j0) of 8 x 8
+// entries on the FP64 tensor cores (mma.m8n8k4): the A fragment is
+// Dinv(l, o) s_o g_a, the B fragment D(o ^ 1, j). wt(o, l) and b(o, j) read the
+// transposed inverse and the orbitals, sg[o] the scaled wave vectors (zeros
+// from orbital n - 1 on). Entries outside n x n are computed from whatever
+// finite values stand there and not stored.
+template <int kR, int kT, class Wt, class Bm>
+__device__ __forceinline__ void f_products(double (&acc)[kR][kT][2][2], int n, int l0, int j0,
+                                           const double2 *sg, Wt wt, Bm b) {
+  const int lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
+#pragma unroll 2
+  for (int ob = 0; ob < n; ob += 4) {
+    const int o = ob + lt;
+    const double2 g = sg[o];
+    double ax[kR], ay[kR];
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+      const double w = wt(o, l0 + 8 * r + lg);
+      ax[r] = w * g.x;
+      ay[r] = w * g.y;
+    }
+#pragma unroll
+    for (int t = 0; t < kT; t++) {
+      const double v = b(o ^ 1, j0 + 8 * t + lg);
+#pragma unroll
+      for (int r = 0; r < kR; r++) {
+        dmma_m8n8k4(acc[r][t][0], ax[r], v);
+        dmma_m8n8k4(acc[r][t][1], ay[r], v);
+      }
+    }
+  }
+}
+template <int kR, int kT>
+__device__ __forceinline__ void f_store(const double (&acc)[kR][kT][2][2], double *F, int n,
+                                        int l0, int j0) {
+  const int lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
+#pragma unroll
+  for (int r = 0; r < kR; r++)
+#pragma unroll
+    for (int t = 0; t < kT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int l = l0 + 8 * r + lg, j = j0 + 8 * t + 2 * lt + e;
+        if (l < n && j < n) {
+          F[l + j * n] = acc[r][t][0][e];
+          F[n * n + l + j * n] = acc[r][t][1][e];
+        }
+      }
+}
+
+// ------------------------------------------------ spins of at most 32 orbitals
+// One warp per (walker, spin), as orb_inv_kernel: lane r holds row r of the
+// Gauss-Jordan matrix, rotated so that the pivot column is always register 0
+// and the step loop stays rolled; the pivot row reaches the other lanes
+// through shared memory. The inverse then goes to shared memory and F comes
+// from the FP64 tensor cores: 450 instructions per matrix of 29 where lanes
+// holding a row of the inverse and 8 columns of F took 3200 (0.177 ms per
+// 4096 walkers at 29 + 29). Both matrices have rows of LD doubles, columns
+// XOR-swizzled by 4 (row mod 4): the fragments' half-warp reads (four rows,
+// four columns) and the lanes' column writes fall on distinct banks.
+constexpr int kRealWarps = 4;
+__host__ __device__ constexpr int real_ld(int nm) { return nm <= 16 ? 16 : 32; }
+__host__ __device__ constexpr size_t real_warp_doubles(int nm) {
+  // orbitals, transposed inverse, two pivot rows, (s g) and pivots per orbital
+  return (size_t)2 * nm * real_ld(nm) + 2 * 32 + 2 * 36 + 16;
+}
+
+template <int NM>
+__global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs a, int nw) {
+  static_assert(NM <= 32, "one lane per row");
+  extern __shared__ __align__(16) char smem[];
+  constexpr int LD = real_ld(NM), TT = (NM + 7) / 8;
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int item = blockIdx.x * kRealWarps + wl;
+  const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
+  const int n = spn ? a.np[1] : a.np[0], r = lane;
+  if (w >= nw || n > NM) return;  // whole warps; nothing below waits on other warps
+  double *Bs = reinterpret_cast<double *>(smem) + wl * real_warp_doubles(NM);
+  double *Wt = Bs + NM * LD, *prow = Wt + NM * LD;
+  double2 *sg = reinterpret_cast<double2 *>(prow + 64);
+  int *perm = reinterpret_cast<int *>(sg + 36);
+  auto at = [](double *m, int o, int j) -> double & { return m[o * LD + (j ^ (4 * (o & 3)))]; };
+  double *F = real_base(a, w) + (spn ? a.f[1] : a.f[0]);
+  // finite values wherever the tiles' padding reads
+  for (int e = lane; e < (NM - n + 1) * LD; e += 32) {
+    const int k = n - 1 + e / LD;
+    Bs[k * LD + e % LD] = 0.0;
+    Wt[k * LD + e % LD] = 0.0;
+  }
+  for (int e = lane; e < n * (LD - n); e += 32) {
+    const int k = e / (LD - n), j = n + e - k * (LD - n);
+    at(Bs, k, j) = 0.0;
+    at(Wt, k, j) = 0.0;
+  }
+  prow[lane] = prow[32 + lane] = 0.0;
+  for (int o = lane; o < 36; o += 32) sg[o] = orbital_g(a.gvec, o, n);
+  __syncwarp();
+  orbital_rows(a, a.scr + w * a.stride + a.l_q + 2 * (spn ? a.f0[1] : a.f0[0]), n, lane, 32,
+               [&](int o, int j) -> double & { return at(Bs, o, j); });
+  __syncwarp();
+  double v[NM];
+#pragma unroll
+  for (int j = 0; j < NM; j++) v[j] = r < n && j < n ? at(Bs, r, j) : (r == j ? 1.0 : 0.0);
+  bool used = r >= n;
+  double my_inv = 1.0, my_d = 1.0;
+  int my_l = r, sing = 0;
+#pragma unroll 1
+  for (int k = 0; k < NM; k++) {
+    int p = k;  // an identity row's own step
+    if (k < n) {
+      const unsigned best = __reduce_max_sync(0xffffffffu, pivot_key(v[0], r, !used));
+      p = 255 - (int)(best & 0xFFu);
+      sing |= (best >> 8) == 0u;
+    }
+    double2 *pr = reinterpret_cast<double2 *>(prow + (k & 1) * 32);
+    if (r == p)
+#pragma unroll
+      for (int c = 0; c < NM; c += 2) pr[c / 2] = make_double2(v[c], c + 1 < NM ? v[c + 1] : 0.0);
+    __syncwarp();
+    const double2 b0 = pr[0];
+    const double inv = rcp_newton(b0.x);
+    const bool isp = r == p;
+    used = used || isp;
+    if (isp) {
+      my_inv = inv;
+      my_d = fabs(b0.x);
+      my_l = k;
+    }
+    const double fac = isp || r >= n ? 0.0 : v[0] * inv;
+    v[0] = fma(-fac, b0.y, v[1]);
+#pragma unroll
+    for (int j = 2; j < NM; j += 2) {
+      const double2 b = pr[j / 2];
+      v[j - 1] = fma(-fac, b.x, v[j]);
+      if (j + 1 < NM) v[j] = fma(-fac, b.y, v[j + 1]);
+    }
+    v[NM - 1] = isp ? 1.0 : -fac;
+  }
+  // step c's pivot row is the orbital of the inverse's column c
+  if (r < n) perm[my_l] = r;
+  double ld = r < n ? log(my_d) : 0.0;
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, q);
+  __syncwarp();
+  if (r < n)
+#pragma unroll
+    for (int c = 0; c < NM; c++)
+      if (c < n) at(Wt, perm[c], my_l) = v[c] * my_inv;
+  __syncwarp();
+  // D2_l = -sum_o Dinv(l, o) g_a g_b D(o, l)
+  if (r < n) {
+    double xx = 0.0, xy = 0.0, yy = 0.0;
+    for (int o = 0; o < n - 1; o++) {
+      const double t = at(Wt, o, r) * at(Bs, o, r);
+      const double2 g = sg[o];
+      xx -= t * (g.x * g.x);
+      xy -= t * (g.x * g.y);
+      yy -= t * (g.y * g.y);
+    }
+    double *d2 = F + 2 * n * n + 2;
+    d2[3 * r] = xx;
+    d2[3 * r + 1] = xy;
+    d2[3 * r + 2] = yy;
+  }
+#pragma unroll 1
+  for (int lt2 = 0; lt2 < TT; lt2 += 2) {
+    if (8 * lt2 >= n) break;
+    double acc[2][TT][2][2] = {};
+    f_products<2, TT>(acc, n, 8 * lt2, 0, sg,
+                      [&](int o, int l) { return at(Wt, min(o, NM - 1), min(l, LD - 1)); },
+                      [&](int o, int j) { return at(Bs, min(o, NM - 1), j); });
+    f_store<2, TT>(acc, F, n, 8 * lt2, 0);
+  }
+  if (lane == 0) {
+    F[2 * n * n] = ld;
+    F[2 * n * n + 1] = (double)sing;
+  }
+}
+
+// ------------------------------------------------- spins above 32 orbitals
+// One CTA per (walker, spin), four lanes per row: lane s of a row holds the
+// columns 4 j + s in C registers, rotated by one register every four steps
+// so that the pivot column of step k is register 0 of lane k mod 4. As
+// gj_invert_reg a step is one barrier: before it every warp publishes its
+// best candidate row (key, reciprocal, columns), after it every thread takes
+// the best key's row. The whole matrix stays in registers, so a step moves
+// only the pivot row through shared memory: C / 2 16-byte reads for C FP64
+// instructions. Above 128 orbitals the last CS of a lane's C columns, which
+// the registers of one SM cannot hold, live in shared memory as a ring that
+// the rotation feeds from. When both spins have at most kRealFused orbitals the
+// transposed inverse and the orbitals then share the CTA's memory and F
+// comes from the FP64 tensor cores here; else both go to device memory for
+// real_f_kernel.
+template <int C>
+__host__ __device__ constexpr int gjc_lane_stride() {  // doubles between the lanes' columns
+  return (C + 1) / 2 * 2 + 2;
+}
+template <int C>
+__host__ __device__ constexpr int gjc_slot() {  // a published row: four lanes' columns, 1 / pivot, |pivot|
+  return 4 * gjc_lane_stride<C>() + 2;
+}
+template <int C, int NT, int CS>
+constexpr size_t inv_cta_doubles(int n, bool fused) {
+  // candidate rows and ring; fused: the transposed inverse in their place (the
+  // ring is empty there), the orbitals, the scaled wave vectors
+  const size_t gj = (size_t)2 * (NT / 32) * gjc_slot<C>() + (size_t)CS * NT;
+  if (!fused) return gj;
+  const size_t m = (size_t)(n + 3) * odd4(n);
+  return (gj > m ? gj : m) + m + 2 * (n + 8);
+}
+
+template <int C, int NT, int MB, int CS, bool kFused>
+__global__ void __launch_bounds__(NT, MB) real_inv_cta_kernel(RealArgs a, int nw) {
+  constexpr int CR = C - CS, G = NT / 32, LS = gjc_lane_stride<C>(), SL = gjc_slot<C>();
+  static_assert(!kFused || CS == 0, "the ring would share its place");
+  __shared__ unsigned keys[2][32];
+  __shared__ double red[G];
+  __shared__ int perm[NT / 4];
+  __shared__ int singular;
+  extern __shared__ __align__(16) char smem[];
+  const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
+  const int n = spn ? a.np[1] : a.np[0];
+  if (w >= nw || n <= 32) return;  // whole CTAs
+  const int t = threadIdx.x, lane = t & 31, wp = t >> 5, r = t >> 2, s = t & 3;
+  double *slots = reinterpret_cast<double *>(smem);  // [2][G][SL]
+  // logical column CR + i of this thread at xs[((hd + i) mod CS) NT]
+  double *xs = slots + (size_t)2 * G * SL + t;
+  int hd = 0;
+  auto xcol = [&](int i) -> double & {
+    const int q = hd + i;
+    return xs[(q >= CS ? q - CS : q) * NT];
+  };
+  double *base = real_base(a, w);
+  const int ldw = spn ? a.ldw[1] : a.ldw[0], ld = odd4(n);
+  double *Wg = base + (spn ? a.w[1] : a.w[0]), *Bg = Wg + n * ldw;  // !kFused
+  double *F = base + (spn ? a.f[1] : a.f[0]);
+  // kFused: the inverse over the candidate rows, the orbitals behind it
+  const size_t gj = (size_t)2 * G * SL, mat = (size_t)(n + 3) * ld;
+  double *Wt = slots, *Bs = slots + (gj > mat ? gj : mat);
+  double2 *sg = reinterpret_cast<double2 *>(Bs + mat);
+  auto bat = [&](int o, int j) -> double & {
+    return kFused ? Bs[o * ld + j] : Bg[o * ldw + j];
+  };
+  if (t == 0) singular = 0;
+  if (t < 64) keys[t >> 5][t & 31] = 0u;
+  orbital_rows(a, a.scr + w * a.stride + a.l_q + 2 * (spn ? a.f0[1] : a.f0[0]), n, t, NT, bat);
+  if (kFused) {
+    for (int o = t; o < n + 8; o += NT) sg[o] = orbital_g(a.gvec, o, n);
+    for (int e = t; e < 3 * ld; e += NT) Bs[n * ld + e] = 0.0;  // read past the last row
+    for (int e = t; e < n * (ld - n); e += NT) {
+      const int k = e / (ld - n);
+      Bs[k * ld + n + e - k * (ld - n)] = 0.0;
+    }
+  }
+  __syncthreads();
+  const bool row = r < n;
+  auto first_col = [&](int j) { return row && 4 * j + s < n ? bat(r, 4 * j + s) : 0.0; };
+  double v[CR];
+#pragma unroll
+  for (int j = 0; j < CR; j++) v[j] = first_col(j);
+  for (int i = 0; i < CS; i++) xcol(i) = first_col(CR + i);
+  bool used = !row;
+  double my_inv = 1.0, my_d = 1.0;
+  int my_l = 0;
+  // step k's candidate of this warp: own is the lane that holds column k in x
+  auto publish = [&](int k, unsigned wk, bool own, double x, double rx) {
+    double *sl = slots + (size_t)((k & 1) * G + wp) * SL;
+    if (wk != 0u && r == 255 - (int)(wk & 0xFFu)) {
+#pragma unroll
+      for (int j = 0; j < CR; j += 2)
+        *reinterpret_cast<double2 *>(sl + s * LS + j) =
+            make_double2(v[j], j + 1 < CR ? v[j + 1] : 0.0);
+      for (int i = 0; i < CS; i++) sl[s * LS + CR + i] = xcol(i);
+      if (own) *reinterpret_cast<double2 *>(sl + 4 * LS) = make_double2(rx, fabs(x));
+    }
+    if (lane == 0) keys[k & 1][wp] = wk;
+  };
+  double f;  // this row's entry of the pivot column
+  {
+    const bool own = s == 0;
+    const unsigned wk = __reduce_max_sync(0xffffffffu, pivot_key(v[0], r, own && !used));
+    publish(0, wk, own, v[0], rcp_newton(v[0]));
+    f = __shfl_sync(0xffffffffu, v[0], 0, 4);
+  }
+  const int macros = (n + 3) / 4;
+#pragma unroll 1
+  for (int m = 0; m < macros; m++) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = 4 * m + u;
+      if (k < n) {
+        __syncthreads();
+        const unsigned best = __reduce_max_sync(0xffffffffu, keys[k & 1][lane]);
+        const int p = 255 - (int)(best & 0xFFu);
+        const double *ps = slots + (size_t)((k & 1) * G + (p >> 3)) * SL;
+        const double inv = ps[4 * LS];
+        if (t == 0) {
+          perm[k] = p;
+          if ((best >> 8) == 0u) singular = 1;
+        }
+        const bool piv = r == p;
+        used = used || piv;
+        if (piv) {
+          my_inv = inv;
+          my_d = ps[4 * LS + 1];
+          my_l = k;
+        }
+        const double fac = piv ? 0.0 : f * inv;
+        const double *pc = ps + s * LS;
+        // the register of column k + 1 first: the next key needs it
+        const int jn = u == 3 ? 1 : 0;  // before the rotation
+        const double xn = fma(-fac, pc[jn], v[jn]);
+        const bool ownn = s == ((u + 1) & 3);
+        const unsigned wk = __reduce_max_sync(0xffffffffu, pivot_key(xn, r, ownn && !used));
+        const double rx = rcp_newton(xn);
+        const double2 *b = reinterpret_cast<const double2 *>(pc);
+        const double done = piv ? 1.0 : -fac;  // the eliminated column
+        if (u < 3) {
+#pragma unroll
+          for (int j = 0; j < CR; j += 2) {
+            const double2 bb = b[j / 2];
+            v[j] = fma(-fac, bb.x, v[j]);
+            if (j + 1 < CR) v[j + 1] = fma(-fac, bb.y, v[j + 1]);
+          }
+#pragma unroll 4
+          for (int i = 0; i < CS; i++) xcol(i) = fma(-fac, pc[CR + i], xcol(i));
+          if (s == u) v[0] = done;
+        } else {
+          const double first = s == u ? done : fma(-fac, pc[0], v[0]);
+#pragma unroll
+          for (int j = 0; j < CR; j += 2) {
+            const double2 bb = b[j / 2];
+            if (j) v[j - 1] = fma(-fac, bb.x, v[j]);
+            if (j + 1 < CR) v[j] = fma(-fac, bb.y, v[j + 1]);
+          }
+          if constexpr (CS > 0) {
+            v[CR - 1] = fma(-fac, pc[CR], xcol(0));
+#pragma unroll 4
+            for (int i = 1; i < CS; i++) xcol(i) = fma(-fac, pc[CR + i], xcol(i));
+            xcol(0) = first;
+            hd = hd + 1 == CS ? 0 : hd + 1;
+          } else {
+            v[CR - 1] = first;
+          }
+        }
+        if (k + 1 < n) {
+          publish(k + 1, wk, ownn, xn, rx);
+          f = __shfl_sync(0xffffffffu, v[0], (u + 1) & 3, 4);
+        }
+      } else if (u == 3) {
+        // past the last step: the rotation alone
+        const double first = v[0];
+#pragma unroll
+        for (int j = 1; j < CR; j++) v[j - 1] = v[j];
+        if constexpr (CS > 0) {
+          v[CR - 1] = xcol(0);
+          xcol(0) = first;
+          hd = hd + 1 == CS ? 0 : hd + 1;
+        } else {
+          v[CR - 1] = first;
+        }
+      }
+    }
+  }
+  __syncthreads();  // perm; the last step's candidates are read
+  // rows normalised by their own pivot, transposed and in orbital order;
+  // register j holds column 4 ((macros + j) mod C) + s
+  auto store = [&](int j, double x) {
+    const int m = macros + j, c = 4 * (m >= C ? m - C : m) + s;
+    if (row && c < n) (kFused ? Wt + perm[c] * ld : Wg + perm[c] * ldw)[my_l] = x * my_inv;
+  };
+#pragma unroll
+  for (int j = 0; j < CR; j++) store(j, v[j]);
+  for (int i = 0; i < CS; i++) store(CR + i, xcol(i));
+  if (kFused) {
+    for (int e = t; e < 3 * ld; e += NT) Wt[n * ld + e] = 0.0;
+    for (int e = t; e < n * (ld - n); e += NT) {
+      const int k = e / (ld - n);
+      Wt[k * ld + n + e - k * (ld - n)] = 0.0;
+    }
+  }
+  double lg = row && s == 0 ? log(my_d) : 0.0;
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, q);
+  if (lane == 0) red[wp] = lg;
+  __syncthreads();
+  if (t == 0) {
+    double sum = 0.0;
+    for (int q = 0; q < G; q++) sum += red[q];
+    F[2 * n * n] = sum;
+    F[2 * n * n + 1] = (double)singular;
+  }
+  if constexpr (kFused) {
+    if (t < n) {
+      double xx = 0.0, xy = 0.0, yy = 0.0;
+      for (int o = 0; o < n - 1; o++) {
+        const double x = Wt[o * ld + t] * Bs[o * ld + t];
+        const double2 g = sg[o];
+        xx -= x * (g.x * g.x);
+        xy -= x * (g.x * g.y);
+        yy -= x * (g.y * g.y);
+      }
+      double *d2 = F + 2 * n * n + 2;
+      d2[3 * t] = xx;
+      d2[3 * t + 1] = xy;
+      d2[3 * t + 2] = yy;
+    }
+    // items of one row tile and up to four column tiles
+    const int T = (n + 7) / 8, TC = (T + 3) / 4;
+    for (int it = wp; it < T * TC; it += G) {
+      const int l0 = 8 * (it / TC), j0 = 32 * (it % TC);
+      double acc[1][4][2][2] = {};
+      f_products<1, 4>(acc, n, l0, j0, sg,
+                       [&](int o, int l) { return Wt[o * ld + min(l, ld - 1)]; },
+                       [&](int o, int j) { return Bs[o * ld + min(j, ld - 1)]; });
+      f_store<1, 4>(acc, F, n, l0, j0);
+    }
+  }
+}
+
+// F and D2 when the larger spin has more than kRealFused orbitals: a CTA takes every row and 32
+// columns of F; the 32 orbital columns are resident, the transposed inverse
+// streams through two buffers of kFK orbitals. A warp holds two row tiles
+// and four column tiles of F_x and F_y.
+constexpr int kFK = 16, kFLd = 36, kFThreads = 352;
+
+inline size_t real_f_doubles(int n, int ldw) {
+  return (size_t)(n + 15) / 16 * 16 * kFLd + (size_t)2 * kFK * odd4(ldw) + 2 * (n + 16);
+}
+
+__global__ void __launch_bounds__(kFThreads, 1) real_f_kernel(RealArgs a, int nw, int blocks) {
+  extern __shared__ __align__(16) char smem[];
+  const int bj = blockIdx.x % blocks, item = blockIdx.x / blocks;
+  const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
+  const int n = spn ? a.np[1] : a.np[0], j0 = 32 * bj;
+  if (w >= nw || n <= 32 || j0 >= n) return;  // whole CTAs
+  const int t = threadIdx.x, wp = t >> 5, lane = t & 31, lg = lane >> 2, lt = lane & 3;
+  double *base = real_base(a, w);
+  const int ldw = spn ? a.ldw[1] : a.ldw[0], ld = odd4(ldw), rows = (n + 15) / 16 * 16;
+  const double *Wg = base + (spn ? a.w[1] : a.w[0]), *Bg = Wg + n * ldw;
+  double *F = base + (spn ? a.f[1] : a.f[0]);
+  double *Bs = reinterpret_cast<double *>(smem), *Wb = Bs + (size_t)rows * kFLd;
+  double2 *sg = reinterpret_cast<double2 *>(Wb + (size_t)2 * kFK * ld);
+  auto stage = [&](int c) {  // orbitals c kFK ..: rows of ldw doubles, 16-byte copies
+    double *dst = Wb + (c & 1) * kFK * ld;
+    const int q = ldw / 2;
+    for (int e = t; e < kFK * q; e += kFThreads) {
+      const int o = e / q, x = e - o * q;
+      if (c * kFK + o < n)
+        cp_async16(dst + o * ld + 2 * x, Wg + (size_t)(c * kFK + o) * ldw + 2 * x);
+      else
+        *reinterpret_cast<double2 *>(dst + o * ld + 2 * x) = make_double2(0.0, 0.0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(0);
+  for (int o = t; o < n + 16; o += kFThreads) sg[o] = orbital_g(a.gvec, o, n);
+  for (int e = t; e < rows * 32; e += kFThreads) {
+    const int o = e >> 5, j = e & 31;
+    Bs[o * kFLd + j] = o < n && j0 + j < n ? Bg[o * ldw + j0 + j] : 0.0;
+  }
+  double acc[2][4][2][2] = {};
+  double d2[3] = {0.0, 0.0, 0.0};
+  const int l0 = 16 * wp, nc = rows / kFK;
+  for (int c = 0; c < nc; c++) {
+    if (c + 1 < nc) stage(c + 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const double *W = Wb + (c & 1) * kFK * ld;
+    if (l0 < n)
+#pragma unroll
+      for (int k = 0; k < kFK; k += 4) {
+        const int o = c * kFK + k + lt;
+        const double2 g = sg[o];
+        double ax[2], ay[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          const double x = W[(k + lt) * ld + min(l0 + 8 * r + lg, ldw - 1)];
+          ax[r] = x * g.x;
+          ay[r] = x * g.y;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const double v = Bs[(o ^ 1) * kFLd + 8 * q + lg];
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            dmma_m8n8k4(acc[r][q][0], ax[r], v);
+            dmma_m8n8k4(acc[r][q][1], ay[r], v);
+          }
+        }
+      }
+    if (t < 32 && j0 + t < n)  // D2 of these 32 electrons
+      for (int k = 0; k < kFK; k++) {
+        const double2 g = sg[c * kFK + k];
+        const double x = W[k * ld + j0 + t] * Bs[(c * kFK + k) * kFLd + t];
+        d2[0] -= x * (g.x * g.x);
+        d2[1] -= x * (g.x * g.y);
+        d2[2] -= x * (g.y * g.y);
+      }
+    __syncthreads();  // this buffer may be refilled
+  }
+  if (l0 < n) f_store<2, 4>(acc, F, n, l0, j0);
+  if (t < 32 && j0 + t < n)
+    for (int q = 0; q < 3; q++) F[2 * n * n + 2 + 3 * (j0 + t) + q] = d2[q];
+}
+
+// ------------------------------------------------- S, drift and Laplacian
+// S_jk[a][c] = sum_i sum_b J_ji[a][b] J_ki[c][b] of one (walker, spin) on the
+// FP64 tensor cores (mma.m8n8k4): in shared memory the Jacobian planes (xx,
+// xy, yy) are matrices of rows j and columns i, so for 8 x 8 tiles of (j, k)
+// and four electrons a warp loads three fragments per tile and issues eight
+// products ((a, c) pairs times b; J is symmetric in (a, b)). The columns hold
+// type 0's electrons, then type 1's, each padded with zeros to a multiple of
+// four, and their stride is an odd multiple of four: the fragments' reads
+// fall on distinct banks. At the end every lane multiplies its S entries by
+// F_a(k,j) F_c(j,k) (and D2_j on the diagonal) and the CTA sums them. Bound by
+// the FP64 pipe (one product of 256 FMAs per 16 cycles and sub-partition).
+//
+// kB: tiles per side of a warp's item. kB = 1 keeps every column resident
+// (spins of at most 61 orbitals) and takes both types of a tile pair in one
+// item; kB = 2 streams chunks of columns through two buffers, one type after
+// the other.
+__host__ __device__ inline int s_chunk(int n) {  // columns per chunk: two buffers in 176 KB
+  const int c = (int)(88 * 1024 / (sizeof(double) * 3 * n)) / 4;
+  return (c & 1 ? c : c - 1) * 4;
+}
+
+// Jacobian columns c0 .. c1-1 (padded numbering) of the n electrons j from
+// f0 on into dst[p][j][c - c0] (asynchronous 8-byte copies, zeros in the
+// padding): from row j of the triangle for i >= j (lanes on consecutive i),
+// from row i for i < j (lanes on consecutive j).
+__device__ inline void stage_cols(const RealArgs &a, double *dst, int ld, const double *jg, int f0,
+                                  int n, int c0, int c1) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int n0 = a.np[0], n1 = a.np[1], pad0 = a.pad0, jp = a.jp, pl = n * ld;
+  for (int jl = warp; jl < n; jl += nw) {
+    const int j = f0 + jl;
+    const double *src = jg + jac_row(a.N, j);
+    double *d = dst + jl * ld - c0;
+    for (int c = c0 + lane; c < c1; c += 32) {
+      const int x = c < pad0 ? c : c - pad0, i = c < pad0 ? c : n0 + x;
+      if (x >= (c < pad0 ? n0 : n1)) {
+        d[c] = d[c + pl] = d[c + 2 * pl] = 0.0;
+      } else if (i >= j) {
+        const double *e = src + i;
+        cp_async8(d + c, e);
+        cp_async8(d + c + pl, e + jp);
+        cp_async8(d + c + 2 * pl, e + 2 * jp);
+      }
+    }
+  }
+  for (int c = c0 + warp; c < c1; c += nw) {
+    const int x = c < pad0 ? c : c - pad0, i = c < pad0 ? c : n0 + x;
+    if (x >= (c < pad0 ? n0 : n1)) continue;
+    const double *src = jg + jac_row(a.N, i) + f0;
+    double *d = dst + (c - c0);
+    for (int jl = max(0, i + 1 - f0) + lane; jl < n; jl += 32) {
+      const double *e = src + jl;
+      double *q = d + jl * ld;
+      cp_async8(q, e);
+      cp_async8(q + pl, e + jp);
+      cp_async8(q + 2 * pl, e + 2 * jp);
+    }
+  }
+}
+
+// Products of kB x kB tile pairs over the columns [k0, k1) of a buffer.
+template <int kB>
+__device__ __forceinline__ void s_products(double (&acc)[kB][kB][4][2], const double *buf, int ld,
+                                           int n, int tj, int tk, int k0, int k1) {
+  const int lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
+  const int pl = n * ld;
+  const double *pj[kB], *pk[kB];
+#pragma unroll
+  for (int a = 0; a < kB; a++) {
+    pj[a] = buf + min(8 * (kB * tj + a) + lg, n - 1) * ld + lt;
+    pk[a] = buf + min(8 * (kB * tk + a) + lg, n - 1) * ld + lt;
+  }
+#pragma unroll 2
+  for (int c = k0; c < k1; c += 4) {
+    double j[kB][3], k[kB][3];
+#pragma unroll
+    for (int a = 0; a < kB; a++)
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        j[a][p] = pj[a][p * pl + c];
+        k[a][p] = pk[a][p * pl + c];
+      }
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+      for (int a = 0; a < kB; a++)
+#pragma unroll
+        for (int d = 0; d < kB; d++)
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+            dmma_m8n8k4(acc[a][d][q], j[a][(q >> 1) + b], k[d][(q & 1) + b]);
+  }
+}
+
+// The shares lt[0 .. kN) of the Laplacian of one item's kN sets of sums: S times
+// F_a(k,j) F_c(j,k), unordered pairs of tiles twice, and D2 on the diagonal.
+template <int kB, int kN>
+__device__ __forceinline__ void s_contract(const double (&acc)[kN][kB][kB][4][2], const double *FX,
+                                           const double *d2, int n, int tj, int tk, double *lt) {
+  const int lane = threadIdx.x & 31, lg = lane >> 2, lq = lane & 3;
+  const double *FY = FX + n * n;
+#pragma unroll
+  for (int a = 0; a < kB; a++)
+#pragma unroll
+    for (int d = 0; d < kB; d++) {
+      const int jt = kB * tj + a, kt = kB * tk + d;
+      if (kB > 1 && jt > kt) continue;  // inside a diagonal item: the other order counts
+      const double wgt = jt == kt ? 1.0 : 2.0;
+      const int j = 8 * jt + lg;
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int k = 8 * kt + 2 * lq + e;
+        if (j < n && k < n) {
+          const int kj = k + j * n, jk = j + k * n;
+          const double xkj = wgt * __ldg(FX + kj), xjk = __ldg(FX + jk);
+          const double ykj = wgt * __ldg(FY + kj), yjk = __ldg(FY + jk);
+          double m0 = xkj * xjk, m1 = xkj * yjk, m2 = ykj * xjk, m3 = ykj * yjk;
+          if (j == k) {
+            m0 -= d2[3 * j];
+            m1 -= d2[3 * j + 1];
+            m2 -= d2[3 * j + 1];
+            m3 -= d2[3 * j + 2];
+          }
+#pragma unroll
+          for (int q = 0; q < kN; q++)
+            lt[q] += m0 * acc[q][a][d][0][e] + m1 * acc[q][a][d][1][e] +
+                     m2 * acc[q][a][d][2][e] + m3 * acc[q][a][d][3][e];
+        }
+      }
+    }
+}
+
+// tile pair (tj <= tk) of index tp in the row-major lower triangle
+__device__ __forceinline__ void tile_pair(int tp, int *tj, int *tk) {
+  int k = (int)((sqrtf(8.0f * (float)tp + 1.0f) - 1.0f) * 0.5f);
+  if (k * (k + 1) / 2 > tp) k--;
+  if ((k + 1) * (k + 2) / 2 <= tp) k++;
+  *tk = k;
+  *tj = tp - k * (k + 1) / 2;
+}
+
+inline size_t s_smem_doubles(int n, int cols, bool resident) {
+  // f, D2, warp sums, then the columns
+  const size_t head = 2 * (size_t)n + ((3 * (size_t)n + 1) & ~size_t(1)) + 2 * 32;
+  return head + (resident ? (size_t)3 * n * odd4(cols) : (size_t)2 * 3 * n * s_chunk(n));
+}
+
+constexpr int kSMaxThreads = 640;  // kB = 1
+
+template <int kB>
+__global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
+    real_s_kernel(RealArgs a, const DevSys *ds, int nw) {
+  extern __shared__ __align__(16) char smem[];
+  const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
+  if (w >= nw) return;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x, NW = nthr >> 5;
+  const int nt = a.nt, n = spn ? a.np[1] : a.np[0], f0 = spn ? a.f0[1] : a.f0[0];
+  double *base = real_base(a, w);
+  const double *FX = base + (spn ? a.f[1] : a.f[0]);
+  double *out = base + (spn ? a.s[1] : a.s[0]);
+  double *fd = reinterpret_cast<double *>(smem), *d2 = fd + 2 * n;
+  double *red = d2 + ((3 * n + 1) & ~1), *jac = red + 2 * 32;
+  const bool timed = ds->phase != nullptr;
+  long long tph = timed ? clock64() : 0;
+  auto mark = [&](int k) {
+    if (timed) phase_mark(*ds, k, tph, t == 0);
+  };
+  const int pad0 = a.pad0, cols = a.cols, n0 = a.np[0];
+  const int ic = kB == 1 ? cols : s_chunk(n), ld = kB == 1 ? odd4(cols) : ic;
+  const size_t bufd = (size_t)3 * n * ld;
+  // kB = 2: chunks never span both types
+  const int nch0 = kB == 1 ? 1 : (pad0 + ic - 1) / ic;
+  const int nch = kB == 1 ? 1 : nch0 + (nt > 1 ? (cols - pad0 + ic - 1) / ic : 0);
+  auto chunk = [&](int ch, int *c0, int *c1) {
+    if (kB == 1) {
+      *c0 = 0;
+      *c1 = cols;
+    } else if (ch < nch0) {
+      *c0 = ch * ic;
+      *c1 = min(pad0, *c0 + ic);
+    } else {
+      *c0 = pad0 + (ch - nch0) * ic;
+      *c1 = min(cols, *c0 + ic);
+    }
+  };
+  auto stage = [&](int ch, int buf) {
+    int c0, c1;
+    chunk(ch, &c0, &c1);
+    stage_cols(a, jac + buf * bufd, ld, base, f0, n, c0, c1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(0, 0);
+  for (int e = t; e < 2 * n; e += nthr)
+    fd[e] = __ldg(FX + (e & 1 ? n * n : 0) + (e >> 1) * (n + 1));
+  for (int e = t; e < 3 * n; e += nthr) d2[e] = __ldg(FX + 2 * n * n + 2 + e);
+  double lt[2] = {0.0, 0.0};
+  // drift of the columns of a buffer: four lanes per electron
+  auto drift = [&](const double *buf, int c0, int c1) {
+    const int l4 = t & 3, pl = n * ld;
+    for (int cb = c0; cb < c1; cb += nthr / 4) {
+      const int c = cb + (t >> 2), x = c < pad0 ? c : c - pad0;
+      const bool on = c < c1 && x < (c < pad0 ? n0 : a.np[1]);
+      double gx = 0.0, gy = 0.0;
+      if (on)
+        for (int j = l4; j < n; j += 4) {
+          const double *r = buf + j * ld + (c - c0);
+          const double xx = r[0], xy = r[pl], yy = r[2 * pl];
+          const double2 f = *reinterpret_cast<const double2 *>(fd + 2 * j);
+          gx += xx * f.x + xy * f.y;
+          gy += xy * f.x + yy * f.y;
+        }
+      gx = group_sum<4>(gx);
+      gy = group_sum<4>(gy);
+      if (on && l4 < 2) out[2 * (c < pad0 ? c : n0 + x) + l4] = l4 ? -gy : -gx;
+    }
+  };
+  const int T = ((n + 7) / 8 + kB - 1) / kB, pairs = T * (T + 1) / 2;
+  if constexpr (kB == 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    mark(PH_DRIFT);
+    drift(jac, 0, cols);
+    for (int it = warp; it < pairs; it += NW) {
+      int tj, tk;
+      tile_pair(it, &tj, &tk);
+      double acc[2][1][1][4][2] = {};
+      s_products<1>(acc[0], jac, ld, n, tj, tk, 0, pad0);
+      if (nt > 1) s_products<1>(acc[1], jac, ld, n, tj, tk, pad0, cols);
+      s_contract<1, 2>(acc, FX, d2, n, tj, tk, lt);
+    }
+  } else {
+    const int rounds = (pairs + NW - 1) / NW;
+    for (int round = 0; round < rounds; round++) {
+      const int it = round * NW + warp;
+      const bool on = it < pairs;
+      int tj = 0, tk = 0;
+      if (on) tile_pair(it, &tj, &tk);
+      double acc[1][kB][kB][4][2];
+      for (int ch = 0; ch < nch; ch++) {
+        if (ch == 0 || ch == nch0)
+#pragma unroll
+          for (int q = 0; q < kB * kB * 8; q++) (&acc[0][0][0][0][0])[q] = 0.0;
+        // this chunk is in flight; the next one (of this round or the
+        // first of the next) goes to the other buffer
+        const int seq = round * nch + ch;
+        if (ch + 1 < nch || round + 1 < rounds)
+          stage(ch + 1 < nch ? ch + 1 : 0, (seq + 1) & 1);
+        else
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        int c0, c1;
+        chunk(ch, &c0, &c1);
+        const double *buf = jac + (seq & 1) * bufd;
+        if (round == 0) drift(buf, c0, c1);
+        if (on) s_products<kB>(acc[0], buf, ld, n, tj, tk, 0, c1 - c0);
+        if (on && (ch + 1 == nch0 || ch + 1 == nch)) {
+          double s = 0.0;
+          s_contract<kB, 1>(acc, FX, d2, n, tj, tk, &s);
+          lt[0] += ch < nch0 ? s : 0.0;
+          lt[1] += ch < nch0 ? 0.0 : s;
+        }
+        __syncthreads();  // this chunk's buffer may be refilled
+      }
+    }
+  }
+  // - sum_j f_j . L_j
+  const double *o = a.scr + w * a.stride;
+  for (int e = t; e < 2 * n; e += nthr) {
+    lt[0] -= fd[e] * __ldg(o + a.l_qbd + 2 * f0 + e);
+    if (nt > 1) lt[1] -= fd[e] * __ldg(o + a.l_sb + 2 * f0 + e);
+  }
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) {
+    lt[0] += __shfl_xor_sync(0xffffffffu, lt[0], q);
+    lt[1] += __shfl_xor_sync(0xffffffffu, lt[1], q);
+  }
+  if (lane == 0) {
+    red[2 * warp] = lt[0];
+    red[2 * warp + 1] = lt[1];
+  }
+  __syncthreads();
+  if (t < 2) {
+    double s = 0.0;
+    for (int q = 0; q < NW; q++) s += red[2 * q + t];
+    out[2 * a.N + t] = s;
+  }
+  mark(PH_CROSS);
+}
+
+// Warps per CTA of the resident form: whole rounds of tile pairs, and about
+// 20 warps on an SM with the CTAs that its shared memory holds.
+int s_warps(int n, size_t smem) {
+  const int T = (n + 7) / 8, pairs = T * (T + 1) / 2, ctas = std::max<int>(1, 227 * 1024 / (int)(smem + 1024));
+  double best = 0.0;
+  int nw = 1;
+  for (int k = 2; k <= kSMaxThreads / 32; k++) {
+    const double fill = (double)pairs / ((pairs + k - 1) / k * k);
+    const int res = std::min(ctas * k, 64);
+    const double score = fill * std::min(1.0, res / 20.0) - 0.002 * k;
+    if (score > best) {
+      best = score;
+      nw = k;
+    }
+  }
+  return nw;
+}
+
+cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int nw,
+                     cudaStream_t st) {
+  size_t d = 0;
+  for (int t = 0; t < hs.nt; t++) d = std::max(d, s_smem_doubles(hs.np[t], a.cols, true));
+  const bool resident = sizeof(double) * d <= 226 * 1024;
+  if (!resident) {
+    d = 0;
+    for (int t = 0; t < hs.nt; t++) d = std::max(d, s_smem_doubles(hs.np[t], a.cols, false));
+  }
+  const size_t sm = sizeof(double) * d;
+  const void *k = resident ? (const void *)real_s_kernel<1> : (const void *)real_s_kernel<2>;
+  cudaError_t e = raise_smem_limit(k, sm);
+  if (e != cudaSuccess) return e;
+  if (resident)
+    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st>>>(a, ds, nw);
+  else
+    real_s_kernel<2><<<nw * hs.nt, 512, sm, st>>>(a, ds, nw);
+  return cudaGetLastError();
+}
+
+template <int C, int NT, int MB, int CS = 0>
+cudaError_t launch_inv_cta(const RealArgs &a, int n, int items, int nw, cudaStream_t st) {
+  constexpr bool fused = CS == 0 && NT <= 480;
+  const size_t sm = sizeof(double) * inv_cta_doubles<C, NT, CS>(n, fused);
+  const void *k = (const void *)real_inv_cta_kernel<C, NT, MB, CS, fused>;
+  cudaError_t e = raise_smem_limit(k, sm);
+  if (e != cudaSuccess) return e;
+  real_inv_cta_kernel<C, NT, MB, CS, fused><<<items, NT, sm, st>>>(a, nw);
+  return cudaGetLastError();
+}
+
+template <int NM>
+cudaError_t launch_det_warp(const RealArgs &a, int items, int nw, cudaStream_t st) {
+  const size_t sm = sizeof(double) * kRealWarps * real_warp_doubles(NM);
+  const void *k = (const void *)real_det_warp_kernel<NM>;
+  cudaError_t e = raise_smem_limit(k, sm);
+  if (e != cudaSuccess) return e;
+  real_det_warp_kernel<NM>
+      <<<(items + kRealWarps - 1) / kRealWarps, 32 * kRealWarps, sm, st>>>(a, nw);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_orbitals_f(const DevSys &hs, const RealArgs &a, int nw, cudaStream_t st) {
+  const int items = nw * hs.nt, nm = hs.nmax;
+  // registers for the rows: the closed shells' sizes 13, 21, 25 and 29
+  // exactly, others padded to 16 or 32 columns
+  if (nm <= 13) return launch_det_warp<13>(a, items, nw, st);
+  if (nm <= 16) return launch_det_warp<16>(a, items, nw, st);
+  if (nm <= 21) return launch_det_warp<21>(a, items, nw, st);
+  if (nm <= 25) return launch_det_warp<25>(a, items, nw, st);
+  if (nm <= 29) return launch_det_warp<29>(a, items, nw, st);
+  if (nm <= 32) return launch_det_warp<32>(a, items, nw, st);
+  cudaError_t e;
+  if (hs.nt > 1 && std::min(hs.np[0], hs.np[1]) <= 32) {
+    // spins on both sides of 32: the warp kernel takes the smaller one
+    if ((e = launch_det_warp<32>(a, items, nw, st)) != cudaSuccess) return e;
+  }
+  // columns per lane, threads (four lanes per row, rows <= NT / 4), CTAs per
+  // SM that the registers are kept for, columns in shared memory
+  e = nm <= 40            ? launch_inv_cta<10, 160, 6>(a, nm, items, nw, st)
+      : nm <= 48          ? launch_inv_cta<12, 192, 5>(a, nm, items, nw, st)
+      : nm <= 64          ? launch_inv_cta<16, 256, 3>(a, nm, items, nw, st)
+      : nm <= 84          ? launch_inv_cta<21, 352, 2>(a, nm, items, nw, st)
+      : nm <= 104         ? launch_inv_cta<26, 416, 1>(a, nm, items, nw, st)
+      : nm <= kRealFused  ? launch_inv_cta<29, 480, 1>(a, nm, items, nw, st)
+      : nm <= 128         ? launch_inv_cta<32, 512, 1, 4>(a, nm, items, nw, st)
+      : nm <= 152         ? launch_inv_cta<38, 608, 1, 12>(a, nm, items, nw, st)
+                          : launch_inv_cta<41, 672, 1, 21>(a, nm, items, nw, st);
+  if (e != cudaSuccess || nm <= kRealFused) return e;
+  const int blocks = (nm + 31) / 32;
+  const size_t sm = sizeof(double) * real_f_doubles(nm, (nm + 3) & ~3);
+  if ((e = raise_smem_limit((const void *)real_f_kernel, sm)) != cudaSuccess) return e;
+  real_f_kernel<<<items * blocks, kFThreads, sm, st>>>(a, nw, blocks);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_real_det(const DevSys &hs, const DevSys *ds, int nw, double *scr,
+                            cudaStream_t st) {
+  if (nw <= 0) return cudaSuccess;
+  const RealArgs a = real_args(hs, scr);
+  const cudaError_t e = launch_orbitals_f(hs, a, nw, st);
+  // a backflow of zeros needs no sums over Jacobian blocks (eval_det_real)
+  if (e != cudaSuccess || hs.bf_zero) return e;
+  return launch_s(hs, ds, a, nw, st);
+}
+
+}  // namespace q2d

@@ -284,9 +284,45 @@ __host__ __device__ inline size_t inv_spin_doubles(int n) {
 __host__ __device__ inline bool orb_inv_fits(const DevSys &s) {
   return s.has_bf && !s.gmat && s.nmax > 0 && s.nmax <= 32;
 }
+// Doubles of a walker's real-orbital region, from its base:
+//   Jacobian blocks dq_j/dx_i of the pairs i <= j (they are symmetric in
+//     (i, j)), the upper triangle row by row in three planes (xx, xy, yy) of
+//     jp doubles (backflow tables that are not identically zero);
+//   f[t]: F_x then F_y of spin t, n x n each, F_a(l, j) at l + j n, then
+//     ln|det|, the singular flag and D2_j (xx, xy, yy of every j);
+//   s[t]: spin t's share of the drift (2N) and of the Laplacian per type (2);
+//   w[t] (a spin above kRealFused orbitals, both spins then): the transposed inverse, Dinv(l, o) at
+//     o ldw + l, and the orbital matrix, row o at o ldw.
+// Largest spin whose inverse and orbital matrix share one CTA's shared memory.
+constexpr int kRealFused = 113;
+struct RealLayout {
+  size_t f[2], s[2], w[2], end;
+  int jp, ldw[2];
+};
+// Offset of (i, j), i <= j, in a Jacobian plane is jac_row(N, i) + j.
+__host__ __device__ inline int jac_row(int N, int i) { return i * N - i * (i + 1) / 2; }
+__host__ __device__ inline RealLayout real_layout(const DevSys &s) {
+  RealLayout r{};
+  r.jp = s.N * (s.N + 1) / 2;
+  size_t o = s.has_bf && !s.bf_zero ? ((size_t)3 * r.jp + 1) & ~size_t(1) : 0;
+  for (int t = 0; t < s.nt; t++) {
+    const size_t n = s.np[t];
+    r.f[t] = o;
+    o += (2 * n * n + 2 + 3 * n + 1) & ~size_t(1);
+    r.s[t] = o;
+    o += 2 * (size_t)s.N + 2;
+    r.ldw[t] = (s.np[t] + 3) & ~3;
+    r.w[t] = o;
+    if (s.nmax > kRealFused && n > 32) o += 2 * n * r.ldw[t];
+  }
+  r.end = o;
+  return r;
+}
+
 // with_inv: the layout of VMC/DMC moves, which may batch their inversion;
 // reptation's kernels never do and lay their blocks out without that region
-// (the same allocation holds them, closer together).
+// (the same allocation holds them, closer together). The real-orbital region
+// (RealLayout) takes the place of both from l.pair on.
 __host__ __device__ inline MoveScratch move_scratch(const DevSys &s, bool with_inv = true) {
   const int N = s.N;
   MoveScratch l;
@@ -309,6 +345,10 @@ __host__ __device__ inline MoveScratch move_scratch(const DevSys &s, bool with_i
     end = (end + 1) & ~size_t(1);
     l.inv = end;
     for (int sp = 0; sp < s.nt; sp++) end += inv_spin_doubles(s.np[sp]);
+  }
+  if (s.real_room && !s.gmat) {
+    const size_t re = (size_t)l.pair + real_layout(s).end;
+    end = re > end ? re : end;
   }
   l.stride = (end + 31) & ~size_t(31);  // 256-byte aligned walker blocks
   return l;
@@ -1338,7 +1378,10 @@ __device__ inline void pair_rhok(const DevSys &S, const EvalSmem &m, int t, int 
 //
 // Pair passes A and B: writes m.{ltf, g, lap, vp, G3, S3, q, Sb, qbd} and
 // zeroes m.{gd, lapd, ph2, ph2d}. With pout (backflow), also the backflow
-// spline values of every pair i < j, laid out as in MoveScratch.
+// spline values of every pair i < j, laid out as in MoveScratch; with kJ
+// (real orbitals, real_det.cuh) pout takes the Jacobian blocks instead
+// (RealLayout) and m.{qbd, Sb} the sums of lap q_j over each type's
+// electrons.
 // NT threads (a multiple of 32) run the passes; the pair rows (layout
 // RowLayout<R>) are read at `rows`, from shared memory when kSh.
 // R is the precision of the u2 and v2 terms: double, or float with the pair
@@ -1350,7 +1393,8 @@ __device__ inline void pair_rhok(const DevSys &S, const EvalSmem &m, int t, int 
 // distance to the nearest node.
 // Sync is the barrier of the NT threads (the CTA, or a named-barrier group
 // of a CTA that runs several walkers); tid is the thread's index among them.
-template <int NT, bool kSh, class R = double, class Sync = CtaSync, int LG = kGroup>
+template <int NT, bool kSh, class R = double, class Sync = CtaSync, int LG = kGroup,
+          bool kJ = false>
 __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long &tph,
                                   double *pout, const R *rows, Sync sync = Sync(),
                                   int tid = threadIdx.x) {
@@ -1373,6 +1417,8 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
     PairSum<double> ltf3, gx3, gy3, lap3;  // the u3 terms' share when R = float
     PairSum<double> Gx, Gy, s3xx, s3xy, s3yy;
     PairSum<double> qx, qy, sbxx, sbxy, sbyy, qbx, qby;
+    PairSum<double> qbx1, qby1;  // kJ: the sums over type 1 (qbx, qby those over type 0)
+    const int jp = N * (N + 1) / 2;  // kJ: a plane of Jacobian blocks
     if (valid) {
       for (int j = lane8; j < N; j += LG) {
         if (j == i) continue;
@@ -1437,9 +1483,25 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
           sbxy.add(c * rxd * ryd);
           sbyy.add(t + c * ryd * ryd);
           double w2 = dt * byrd * 3.0 + ddt;
-          qbx.add(w2 * rxd);
-          qby.add(w2 * ryd);
-          if (pout && i < j) {
+          if constexpr (kJ) {
+            if (tj) {
+              qbx1.add(w2 * rxd);
+              qby1.add(w2 * ryd);
+            } else {
+              qbx.add(w2 * rxd);
+              qby.add(w2 * ryd);
+            }
+            if (pout && i < j) {
+              double *e = pout + jac_row(N, i) + j;
+              e[0] = -(t + c * rxd * rxd);
+              e[jp] = -(c * rxd * ryd);
+              e[2 * jp] = -(t + c * ryd * ryd);
+            }
+          } else {
+            qbx.add(w2 * rxd);
+            qby.add(w2 * ryd);
+          }
+          if (!kJ && pout && i < j) {
             const size_t e = pair_tri(N, i, j);
             pout[e] = t;
             pout[NP + e] = c;
@@ -1480,6 +1542,11 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
       qbx_s = group_sum<LG>(qbx.value());
       qby_s = group_sum<LG>(qby.value());
     }
+    double qbx1_s = 0, qby1_s = 0;
+    if (kJ && S.has_bf && S.nt > 1) {
+      qbx1_s = group_sum<LG>(qbx1.value());
+      qby1_s = group_sum<LG>(qby1.value());
+    }
     if (valid && lane8 == 0) {
       m.ltf[i] = ltf_s;
       m.g[2 * i] = gx_s;
@@ -1495,11 +1562,27 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
       }
       m.q[2 * i] = m.x[2 * i] + qx_s;
       m.q[2 * i + 1] = m.x[2 * i + 1] + qy_s;
-      m.Sb[3 * i] = sbxx_s;
-      m.Sb[3 * i + 1] = sbxy_s;
-      m.Sb[3 * i + 2] = sbyy_s;
-      m.qbd[2 * i] = qbx_s;
-      m.qbd[2 * i + 1] = qby_s;
+      if constexpr (kJ) {
+        // sum over the electrons of type 0 (qbd) and 1 (Sb) of lap q_i: the
+        // partners' terms, and i's own for its type
+        const double ox = qbx_s + qbx1_s, oy = qby_s + qby1_s;
+        m.qbd[2 * i] = qbx_s + (ti ? 0.0 : ox);
+        m.qbd[2 * i + 1] = qby_s + (ti ? 0.0 : oy);
+        m.Sb[2 * i] = qbx1_s + (ti ? ox : 0.0);
+        m.Sb[2 * i + 1] = qby1_s + (ti ? oy : 0.0);
+        if (pout) {
+          double *e = pout + jac_row(N, i) + i;
+          e[0] = 1.0 + sbxx_s;
+          e[jp] = sbxy_s;
+          e[2 * jp] = 1.0 + sbyy_s;
+        }
+      } else {
+        m.Sb[3 * i] = sbxx_s;
+        m.Sb[3 * i + 1] = sbxy_s;
+        m.Sb[3 * i + 2] = sbyy_s;
+        m.qbd[2 * i] = qbx_s;
+        m.qbd[2 * i + 1] = qby_s;
+      }
       m.gd[2 * i] = 0.0;
       m.gd[2 * i + 1] = 0.0;
       m.lapd[i] = 0.0;
@@ -1552,6 +1635,168 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
     sync();
     phase_mark(S, PH_U3, tph, tid == 0);
   }
+}
+
+// The end of an evaluation: -ln psi from the Jastrow sum ltf_j and ln|det|,
+// the kinetic and potential energies and every property from the
+// per-particle sums in m and rho_k; returns status with what it adds.
+__device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double ltf_j,
+                                    double logdet_sum, int status, double *hl, double *props,
+                                    double *sign, long long &tph) {
+  const int tid = threadIdx.x, N = S.N, nt = S.nt;
+  // ---- assemble: -ln psi, kinetic (reptation.f:2729), potential (:3986)
+  double ltf = ltf_j - logdet_sum;
+  bool underflow = false;
+  if (S.has_bf && S.ref_underflow) underflow = exp(-ltf * 2.0) <= 0.0;
+  if (underflow) status |= ST_UNDERFLOW;
+  // determinant terms and the drift cutoff (kinetic, reptation.f:2748-2763),
+  // and on the way the per-type sums: Laplacian, |g|^2, pair potential,
+  // phase gradient^2 (register arrays with compile-time indices only:
+  // nt <= 2), the drift cutoff factors, and the k-space sums of every type
+  // pair (reptation.f:4034-4052), all in one block reduction
+  double sums[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int i = tid; i < N; i += kThreads) {
+    double gx = m.g[2 * i], gy = m.g[2 * i + 1], lp = m.lap[i], ph = 0.0;
+    if (S.has_bf && !underflow) {
+      gx += m.gd[2 * i];
+      gy += m.gd[2 * i + 1];
+      lp += m.lapd[i];
+      ph = m.ph2d[i];
+    }
+    double x2 = gx * gx + gy * gy;
+    const int ti = type_of(S, i);
+    if (S.adrift != 0.0) {
+      double vari = 1.0 / (2.0 * S.hbs2m[ti] * S.delta);
+      double gg = x2 * S.adrift * S.delta * S.delta * vari;
+      gg = (-1.0 + sqrt(1.0 + 2.0 * gg)) / gg;
+      sums[8] += gg;
+      gx *= gg;
+      gy *= gg;
+    }
+    m.g[2 * i] = gx;
+    m.g[2 * i + 1] = gy;
+    m.lap[i] = lp;
+    m.ph2[i] = ph;
+    m.ph2d[i] = x2;  // |g|^2 before the cutoff, for the kinetic energy
+    const bool t1 = ti == 1;
+    const double v = m.vp[i];
+    sums[0] += t1 ? 0.0 : lp;
+    sums[1] += t1 ? 0.0 : x2;
+    sums[2] += t1 ? 0.0 : v;
+    sums[3] += t1 ? 0.0 : ph;
+    sums[4] += t1 ? lp : 0.0;
+    sums[5] += t1 ? x2 : 0.0;
+    sums[6] += t1 ? v : 0.0;
+    sums[7] += t1 ? ph : 0.0;
+  }
+  {
+    // every type pair in one loop, so the four v_k loads of a k are in
+    // flight together (the sums keep their order: k ascending per thread)
+    int nkp[4], nkmax = 0;
+    const double *vkp[4];
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const int it = p >> 1, jt = p & 1;
+      const int iv = (it < nt && jt < nt) ? S.iv2[it][jt] : -1;
+      nkp[p] = iv >= 0 ? S.tab_nkew[iv] : 0;
+      vkp[p] = S.coef + (iv >= 0 ? S.tab_vkoff[iv] : 0);
+      nkmax = max(nkmax, nkp[p]);
+    }
+    for (int k = tid; k < nkmax; k += kThreads) {
+      double vk[4];
+#pragma unroll
+      for (int p = 0; p < 4; p++) vk[p] = k < nkp[p] ? __ldg(vkp[p] + k) : 0.0;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const int it = p >> 1, jt = p & 1;
+        if (k < nkp[p])
+          sums[9 + p] += vk[p] * (m.rhok[2 * (it * S.nk + k)] * m.rhok[2 * (jt * S.nk + k)] +
+                                  m.rhok[2 * (it * S.nk + k) + 1] * m.rhok[2 * (jt * S.nk + k) + 1]);
+      }
+    }
+  }
+  block_sum_n<13>(sums, m.red);
+  double kin0 = 0.0, pot0 = 0.0, efp = 0.0;
+  double kin_t[2] = {0, 0}, un_t[2] = {0, 0}, pot_t[2] = {0, 0};
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    if (t < nt) {
+    double hs = sums[4 * t], g2 = sums[4 * t + 1];
+    if (tid == 0) hl[t] = hs;
+    kin_t[t] = S.hbs2m[t] * (hs - g2);
+    kin0 += kin_t[t];
+    kin_t[t] /= S.np[t];
+    un_t[t] = 1.0 / sqrt(g2);
+    pot_t[t] = sums[4 * t + 2];
+    efp += S.hbs2m[t] * sums[4 * t + 3];
+    }
+  }
+  kin0 /= S.npnorm;
+  // v2 tails (potential, reptation.f:4001-4022)
+#pragma unroll
+  for (int it = 0; it < 2; it++) {
+    if (it >= nt) continue;
+    int i = S.iv2[it][it];
+    if (i >= 0) pot_t[it] += S.np[it] * (S.np[it] - 1) * 0.5 * S.tab_tail[i];
+    if (it == 0 && nt > 1) {
+      i = S.iv2[0][1];
+      if (i >= 0) {
+        double aux = S.np[0] * S.np[1] * S.tab_tail[i];
+        pot_t[0] += 0.5 * aux;
+        pot_t[1] += 0.5 * aux;
+      }
+    }
+  }
+  pot0 = pot_t[0] + pot_t[1];
+  // k space (reptation.f:4034-4052): the type pairs' sums from above
+#pragma unroll
+  for (int it = 0; it < 2; it++)
+#pragma unroll
+    for (int jt = 0; jt < 2; jt++) {
+      if (it >= nt || jt >= nt) continue;
+      int iv = S.iv2[it][jt];
+      if (iv < 0 || S.tab_nkew[iv] == 0) continue;
+      double c = sums[9 + 2 * it + jt] + S.tab_kself[iv] * S.npnorm;
+      pot_t[it] += c;
+      pot0 += c;
+    }
+  pot0 = (pot0 + S.v0) / S.npnorm;
+  efp = S.ntheta != 0 ? efp / S.npnorm : 0.0;
+  if (tid == 0) {
+    const int J7 = 7;
+    props[QMC2D_JLTF] = ltf;
+    props[QMC2D_JACC] = 0.0;
+    props[QMC2D_JPOT0] = pot0;
+    props[QMC2D_JKIN0] = kin0;
+    props[QMC2D_JGG] = S.adrift != 0.0 ? sums[8] / N : 1.0;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      if (t >= nt) continue;
+      props[J7 + t] = pot_t[t] / S.np[t];
+      props[J7 + nt + t] = kin_t[t];
+      props[J7 + 2 * nt + t] = un_t[t];
+    }
+    props[J7 + 3 * nt] = efp;
+    double et = pot0 + kin0 + efp;
+    props[QMC2D_JETOT] = et;
+    props[QMC2D_JE2] = et * et;
+    *sign = 1.0;
+  }
+  // rho_k properties (compute_properties, reptation.f:2672-2683)
+  {
+    int cnt = 0;
+    for (int it = 0; it < nt; it++) {
+      if (S.irhok[it] == 0) continue;
+      for (int e = tid; e < 2 * S.nk; e += kThreads)
+        props[S.jrhok + cnt + e] = (it < S.nrhok) ? m.rhok[2 * it * S.nk + e] : 0.0;
+      cnt += 2 * S.nk;
+    }
+  }
+  // every thread holds the same sums, so the same total energy
+  if (!isfinite(pot0 + kin0 + efp) || !isfinite(ltf)) status |= ST_NONFINITE;
+  __syncthreads();
+  phase_mark(S, PH_ASSEMBLE, tph);
+  return status;
 }
 
 // Everything after the pair passes: determinants (orbitals, inversion,
@@ -2085,159 +2330,7 @@ __device__ inline int eval_det(const DevSys &S, const EvalSmem &m, double *hl, d
     phase_mark(S, PH_RHOK, tph);
   }
 
-  // ---- assemble: -ln psi, kinetic (reptation.f:2729), potential (:3986)
-  double ltf = ltf_j - logdet_sum;
-  bool underflow = false;
-  if (S.has_bf && S.ref_underflow) underflow = exp(-ltf * 2.0) <= 0.0;
-  if (underflow) status |= ST_UNDERFLOW;
-  // determinant terms and the drift cutoff (kinetic, reptation.f:2748-2763),
-  // and on the way the per-type sums: Laplacian, |g|^2, pair potential,
-  // phase gradient^2 (register arrays with compile-time indices only:
-  // nt <= 2), the drift cutoff factors, and the k-space sums of every type
-  // pair (reptation.f:4034-4052), all in one block reduction
-  double sums[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = tid; i < N; i += kThreads) {
-    double gx = m.g[2 * i], gy = m.g[2 * i + 1], lp = m.lap[i], ph = 0.0;
-    if (S.has_bf && !underflow) {
-      gx += m.gd[2 * i];
-      gy += m.gd[2 * i + 1];
-      lp += m.lapd[i];
-      ph = m.ph2d[i];
-    }
-    double x2 = gx * gx + gy * gy;
-    const int ti = type_of(S, i);
-    if (S.adrift != 0.0) {
-      double vari = 1.0 / (2.0 * S.hbs2m[ti] * S.delta);
-      double gg = x2 * S.adrift * S.delta * S.delta * vari;
-      gg = (-1.0 + sqrt(1.0 + 2.0 * gg)) / gg;
-      sums[8] += gg;
-      gx *= gg;
-      gy *= gg;
-    }
-    m.g[2 * i] = gx;
-    m.g[2 * i + 1] = gy;
-    m.lap[i] = lp;
-    m.ph2[i] = ph;
-    m.ph2d[i] = x2;  // |g|^2 before the cutoff, for the kinetic energy
-    const bool t1 = ti == 1;
-    const double v = m.vp[i];
-    sums[0] += t1 ? 0.0 : lp;
-    sums[1] += t1 ? 0.0 : x2;
-    sums[2] += t1 ? 0.0 : v;
-    sums[3] += t1 ? 0.0 : ph;
-    sums[4] += t1 ? lp : 0.0;
-    sums[5] += t1 ? x2 : 0.0;
-    sums[6] += t1 ? v : 0.0;
-    sums[7] += t1 ? ph : 0.0;
-  }
-  {
-    // every type pair in one loop, so the four v_k loads of a k are in
-    // flight together (the sums keep their order: k ascending per thread)
-    int nkp[4], nkmax = 0;
-    const double *vkp[4];
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      const int it = p >> 1, jt = p & 1;
-      const int iv = (it < nt && jt < nt) ? S.iv2[it][jt] : -1;
-      nkp[p] = iv >= 0 ? S.tab_nkew[iv] : 0;
-      vkp[p] = S.coef + (iv >= 0 ? S.tab_vkoff[iv] : 0);
-      nkmax = max(nkmax, nkp[p]);
-    }
-    for (int k = tid; k < nkmax; k += kThreads) {
-      double vk[4];
-#pragma unroll
-      for (int p = 0; p < 4; p++) vk[p] = k < nkp[p] ? __ldg(vkp[p] + k) : 0.0;
-#pragma unroll
-      for (int p = 0; p < 4; p++) {
-        const int it = p >> 1, jt = p & 1;
-        if (k < nkp[p])
-          sums[9 + p] += vk[p] * (m.rhok[2 * (it * S.nk + k)] * m.rhok[2 * (jt * S.nk + k)] +
-                                  m.rhok[2 * (it * S.nk + k) + 1] * m.rhok[2 * (jt * S.nk + k) + 1]);
-      }
-    }
-  }
-  block_sum_n<13>(sums, m.red);
-  double kin0 = 0.0, pot0 = 0.0, efp = 0.0;
-  double kin_t[2] = {0, 0}, un_t[2] = {0, 0}, pot_t[2] = {0, 0};
-#pragma unroll
-  for (int t = 0; t < 2; t++) {
-    if (t < nt) {
-    double hs = sums[4 * t], g2 = sums[4 * t + 1];
-    if (tid == 0) hl[t] = hs;
-    kin_t[t] = S.hbs2m[t] * (hs - g2);
-    kin0 += kin_t[t];
-    kin_t[t] /= S.np[t];
-    un_t[t] = 1.0 / sqrt(g2);
-    pot_t[t] = sums[4 * t + 2];
-    efp += S.hbs2m[t] * sums[4 * t + 3];
-    }
-  }
-  kin0 /= S.npnorm;
-  // v2 tails (potential, reptation.f:4001-4022)
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    if (it >= nt) continue;
-    int i = S.iv2[it][it];
-    if (i >= 0) pot_t[it] += S.np[it] * (S.np[it] - 1) * 0.5 * S.tab_tail[i];
-    if (it == 0 && nt > 1) {
-      i = S.iv2[0][1];
-      if (i >= 0) {
-        double aux = S.np[0] * S.np[1] * S.tab_tail[i];
-        pot_t[0] += 0.5 * aux;
-        pot_t[1] += 0.5 * aux;
-      }
-    }
-  }
-  pot0 = pot_t[0] + pot_t[1];
-  // k space (reptation.f:4034-4052): the type pairs' sums from above
-#pragma unroll
-  for (int it = 0; it < 2; it++)
-#pragma unroll
-    for (int jt = 0; jt < 2; jt++) {
-      if (it >= nt || jt >= nt) continue;
-      int iv = S.iv2[it][jt];
-      if (iv < 0 || S.tab_nkew[iv] == 0) continue;
-      double c = sums[9 + 2 * it + jt] + S.tab_kself[iv] * S.npnorm;
-      pot_t[it] += c;
-      pot0 += c;
-    }
-  pot0 = (pot0 + S.v0) / S.npnorm;
-  efp = S.ntheta != 0 ? efp / S.npnorm : 0.0;
-  if (tid == 0) {
-    const int J7 = 7;
-    props[QMC2D_JLTF] = ltf;
-    props[QMC2D_JACC] = 0.0;
-    props[QMC2D_JPOT0] = pot0;
-    props[QMC2D_JKIN0] = kin0;
-    props[QMC2D_JGG] = S.adrift != 0.0 ? sums[8] / N : 1.0;
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-      if (t >= nt) continue;
-      props[J7 + t] = pot_t[t] / S.np[t];
-      props[J7 + nt + t] = kin_t[t];
-      props[J7 + 2 * nt + t] = un_t[t];
-    }
-    props[J7 + 3 * nt] = efp;
-    double et = pot0 + kin0 + efp;
-    props[QMC2D_JETOT] = et;
-    props[QMC2D_JE2] = et * et;
-    *sign = 1.0;
-  }
-  // rho_k properties (compute_properties, reptation.f:2672-2683)
-  {
-    int cnt = 0;
-    for (int it = 0; it < nt; it++) {
-      if (S.irhok[it] == 0) continue;
-      for (int e = tid; e < 2 * S.nk; e += kThreads)
-        props[S.jrhok + cnt + e] = (it < S.nrhok) ? m.rhok[2 * it * S.nk + e] : 0.0;
-      cnt += 2 * S.nk;
-    }
-  }
-  // every thread holds the same sums, so the same total energy
-  if (!isfinite(pot0 + kin0 + efp) || !isfinite(ltf)) status |= ST_NONFINITE;
-  __syncthreads();
-  phase_mark(S, PH_ASSEMBLE, tph);
-  return status;
+  return eval_assemble(S, m, ltf_j, logdet_sum, status, hl, props, sign, tph);
 }
 
 // The whole evaluation of the configuration in m.x (compute_properties,

@@ -1,0 +1,86 @@
+"""The real-orbital route of moves (Gamma-point determinants of an odd number of
+plane waves as cosines and sines) against the complex kernels on the same
+start: one VMC step with every move forced, on spins at the edges of the
+kernels' tiles and register rows (one to 161 orbitals, equal and unequal
+spins, with and without backflow displacement, mixed precision). Both routes
+compute the same FP64 formulas in another order, so the step agrees as moves
+agree with the oracle elsewhere in the suite (positions 1e-11, the rest 1e-9
+of the largest value). A twist takes the complex kernels and Gamma, set
+again, the real ones."""
+import importlib
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHELLS = [(1, 1), (3, 1), (5, 5), (9, 0), (15, 13), (17, 17), (31, 25), (31, 33), (33, 0),
+          (39, 41), (47, 49), (63, 0), (65, 63), (83, 0), (85, 45), (103, 0), (105, 0), (113, 0),
+          (115, 33), (127, 0), (129, 31), (151, 0), (161, 0)]
+
+
+def _deck(q, tmp_path, nu, nd, **kw):
+    tables = importlib.import_module("2degas_b200.tables")
+    kw = dict(dict(rs=3.0, backflow=(0.2, 3.0, 1.8), nconf=6, seed=11), **kw)
+    d = tables.make_run(os.path.join(tmp_path, "d"), "c", nu, nd, **kw)
+    s = q.System.read(d, "c")
+    return s, s.read_configs(d, ".0", 0, 6)
+
+
+def _step(q, s, x, mode, precision="fp64"):
+    with q.Handle(s, capacity=len(x), seed=77) as h:
+        h.set_precision(precision)
+        h.set_move_inversion(mode)
+        h.population_set(x)
+        h.block_reset()
+        h.vmc(1, 0.05 * 26 / s.N, 0)  # mage = age: every move is forced
+        return h.population_get(), h.block_get()
+
+
+def _same(a, b, tol):
+    # a pair beyond the tables' cut has no drift and an infinite 1 / |g|: the
+    # same entries have to be infinite
+    fin = np.isfinite(b)
+    if not np.array_equal(a[~fin], b[~fin]):
+        return False
+    a, b = a[fin], b[fin]
+    return np.abs(a - b).max() <= tol * max(np.abs(b).max(), 1e-300)
+
+
+@pytest.mark.parametrize("nu,nd", SHELLS)
+@pytest.mark.parametrize("bf", [0.2, 0.0])
+def test_step_equals_the_complex_route(q, tmp_path, nu, nd, bf):
+    s, x = _deck(q, tmp_path, nu, nd, backflow=(bf, 3.0, 1.8), u3=nu == 17)
+    (r, rb), (c, cb) = _step(q, s, x, 1), _step(q, s, x, 0)
+    assert _same(r["x"], c["x"], 1e-11)
+    for k in ("g", "h", "p"):
+        assert _same(r[k], c[k], 1e-9), k
+    assert _same(rb[0], cb[0], 1e-9) and rb[1] == cb[1]
+
+
+def test_mixed_precision_step(q, tmp_path):
+    s, x = _deck(q, tmp_path, 21, 13)
+    (r, _), (c, _) = _step(q, s, x, 1, "mixed"), _step(q, s, x, 0, "mixed")
+    for k in ("g", "h", "p"):
+        assert _same(r[k], c[k], 1e-9), k
+
+
+def test_a_twist_and_gamma_again(q, tmp_path):
+    s, x = _deck(q, tmp_path, 13, 13, twist=True)
+    ref = {}
+    for mode in (1, 0):
+        with q.Handle(s, capacity=len(x), seed=5) as h:
+            h.set_move_inversion(mode)
+            out = []
+            for tw in ((0, 0), (1, 2), (0, 0)):
+                s.set_twist(*tw)
+                h.update_twist()
+                h.population_set(x)
+                h.vmc(1, 0.05, 0)
+                out.append(h.population_get()["p"])
+            ref[mode] = out
+    s.set_twist(0, 0)
+    for a, b in zip(ref[1], ref[0]):
+        assert _same(a, b, 1e-9)
+    assert not _same(ref[1][1], ref[1][0], 1e-3)
