@@ -725,6 +725,14 @@ extern "C" int qmc2d_profile_get(qmc2d_handle *h, int kernel, double *ms, long *
   return QMC2D_OK;
 }
 
+// nw configurations on stream st: through the real-orbital kernels or fused.
+static cudaError_t evaluate(qmc2d_handle *h, int nw, const double *x, double *g, double *hl,
+                            double *props, double *s, cudaStream_t st) {
+  if (st == h->stream && eval_real(h, nw))
+    return q2d::launch_eval_real(h->hs, h->ds, nw, x, g, hl, props, s, h->d_status, h->d_mscr, st);
+  return q2d::launch_eval(h->hs, h->ds, nw, x, g, hl, props, s, h->d_status, st);
+}
+
 extern "C" int qmc2d_compute_properties_dev(qmc2d_handle *h, int nw, const double *x_dev,
                                             double *g_dev, double *hl_dev, double *props_dev,
                                             double *s_dev, void *stream) {
@@ -737,8 +745,7 @@ extern "C" int qmc2d_compute_properties_dev(qmc2d_handle *h, int nw, const doubl
   CK(join_side(h));
   if (nw > 0) CK(cudaMemsetAsync(h->d_status, 0, sizeof(int) * nw, st));
   ProfScope ps(h, QMC2D_KERNEL_EVAL, st);
-  CK(q2d::launch_eval(h->hs, h->ds, nw, x_dev, g_dev, hl_dev, props_dev, s_dev, h->d_status,
-                      st));
+  CK(evaluate(h, nw, x_dev, g_dev, hl_dev, props_dev, s_dev, st));
   return QMC2D_OK;
 }
 
@@ -767,8 +774,7 @@ extern "C" int qmc2d_compute_properties(qmc2d_handle *h, int nw, const double *x
   CK(cudaMemcpyAsync(h->d_x, x, sizeof(double) * N2 * nw, cudaMemcpyHostToDevice, h->stream));
   {
     ProfScope ps(h, QMC2D_KERNEL_EVAL, h->stream);
-    CK(q2d::launch_eval(h->hs, h->ds, nw, h->d_x, h->d_g, h->d_h, h->d_p, h->d_s, h->d_status,
-                        h->stream));
+    CK(evaluate(h, nw, h->d_x, h->d_g, h->d_h, h->d_p, h->d_s, h->stream));
   }
   if (g) CK(cudaMemcpyAsync(g, h->d_g, sizeof(double) * N2 * nw, cudaMemcpyDeviceToHost, h->stream));
   if (hl)
@@ -792,7 +798,7 @@ extern "C" int qmc2d_population_set(qmc2d_handle *h, int nw, const double *x) {
   size_t N2 = 2 * (size_t)h->N;
   CK(cudaMemsetAsync(h->d_status, 0, sizeof(int) * nw, h->stream));
   CK(cudaMemcpyAsync(p.x, x, sizeof(double) * N2 * nw, cudaMemcpyHostToDevice, h->stream));
-  CK(q2d::launch_eval(h->hs, h->ds, nw, p.x, p.g, p.h, p.p, p.s, h->d_status, h->stream));
+  CK(evaluate(h, nw, p.x, p.g, p.h, p.p, p.s, h->stream));
   // read_conf's metropolis_test(1): accepted, p_old(jacc) = 1, age = 0
   std::vector<double> one(nw, 1.0), zero(nw, 0.0);
   CK(cudaMemcpy2DAsync(p.p + QMC2D_JACC, sizeof(double) * h->nprops, one.data(), sizeof(double),

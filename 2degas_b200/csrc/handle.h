@@ -69,6 +69,9 @@ struct qmc2d_handle {
 // of the CTA, gains 4% at 3.5 and 21% at 7.
 constexpr int kOrbInvMinPerSM = 10, kOrbInvMinPerSMSmall = 10, kOrbInvMinPerSMOneSpin = 3;
 
+// Spin matrices from which an evaluation takes the real-orbital kernels.
+constexpr long kEvalRealMin = 0;
+
 // Whether this handle's next move batches its orbitals and inversion.
 inline bool move_orb_inv(const qmc2d_handle *h) {
   if (h->move_inv_mode == 0) return false;
@@ -84,6 +87,14 @@ inline bool move_orb_inv(const qmc2d_handle *h) {
 // inversion mode chosen by the caller keeps the complex kernels.
 inline bool move_real(const qmc2d_handle *h) {
   return h->hs.real_orb && h->hs.tune_inv == 0 && h->move_inv_mode == 1;
+}
+
+// Whether an evaluation of nw configurations on the handle's own stream runs
+// through the move's kernels (launch_eval_real, in the move scratch) instead
+// of the fused kernel. Evaluations on a caller's stream stay fused: they may
+// overlap the handle's moves, whose scratch this is.
+inline bool eval_real(const qmc2d_handle *h, int nw) {
+  return h->hs.real_orb && h->hs.tune_inv == 0 && (long)nw * h->hs.nt >= kEvalRealMin;
 }
 
 // Orders the handle's stream after the side copies of the last

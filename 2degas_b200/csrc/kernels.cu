@@ -155,6 +155,11 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 // reverse move, metropolis_test and the averages, with the walker's state
 // in shared memory.
 //
+// pairs_kernel and the real-orbital kernels take the system by value: its
+// fields are constant-bank operands, where a copy in shared memory costs a
+// load for every use. A captured graph keeps that value (its key holds what
+// can change: the timers' buffer, the precision, the time step).
+//
 // pairs_kernel is persistent: its CTAs walk over the population with G
 // independent groups of kThreads threads each, every group on its own
 // walker and its own named barrier, so one group's latency overlaps the
@@ -174,13 +179,10 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 // (real_det.cuh) instead of the pairs' spline values; xe (kJ only) the
 // configurations to evaluate instead of a proposal.
 template <class R, int G, int LG, bool kJ>
-__global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(const DevSys *sp, DevPop pop,
-                                                                    MoveArgs a, int stage_rows,
-                                                                    const double *xe) {
+__global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(
+    const __grid_constant__ DevSys S, DevPop pop, MoveArgs a, int stage_rows, const double *xe) {
   constexpr int kPairGroups = G, kPairThreads = G * kThreads;
-  __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
   const size_t carve = (pair_carve(S, nullptr, nullptr, kThreads) + 127) & ~size_t(127);
   const int grp = threadIdx.x / kThreads, tid = threadIdx.x - grp * kThreads;
   EvalSmem m;
@@ -583,25 +585,6 @@ __global__ void __launch_bounds__(kThreads, kSeq ? 3 : 2) move_kernel(const DevS
 }
 
 // --------------------------------------------------- real orbitals
-// The pair passes' sums of walker w into shared memory, the determinant sums
-// zeroed (asynchronous 8-byte copies; the caller waits).
-__device__ __forceinline__ void load_real_sums(const DevSys &S, const EvalSmem &m,
-                                               const double *o, const MoveScratch &L) {
-  const int N = S.N, tid = threadIdx.x;
-  for (int j = tid; j < 2 * N; j += kThreads) {
-    cp_async8(m.x + j, o + L.x + j);
-    cp_async8(m.g + j, o + L.g + j);
-  }
-  for (int j = tid; j < N; j += kThreads) {
-    cp_async8(m.lap + j, o + L.lap + j);
-    cp_async8(m.ltf + j, o + L.ltf + j);
-    cp_async8(m.vp + j, o + L.vp + j);
-    m.lapd[j] = 0.0;
-    m.ph2[j] = 0.0;
-    m.ph2d[j] = 0.0;
-  }
-}
-
 // What move_real_kernel keeps beside the evaluation: the old positions and
 // drift, the new properties, -lap per type, the sign.
 struct MoveRealSmem {
@@ -633,12 +616,10 @@ size_t eval_real_smem_bytes(const DevSys &s) {
 // The rest of a move after launch_real_det: the assembly, the reverse move,
 // Metropolis, the averages. Latency-bound (reductions, transcendentals, the
 // records' reads and writes); four CTAs per SM overlap it.
-__global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const DevSys *sp, DevPop pop,
+__global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_constant__ DevSys S, DevPop pop,
                                                                 MoveArgs a, RealArgs ra,
                                                                 MoveScratch L) {
-  __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   MoveRealSmem v;
@@ -719,14 +700,12 @@ __global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const DevSys *sp
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 4) eval_real_kernel(const DevSys *sp, int nw,
+__global__ void __launch_bounds__(kThreads, 4) eval_real_kernel(const __grid_constant__ DevSys S, int nw,
                                                                 RealArgs ra, MoveScratch L,
                                                                 double *g, double *hl,
                                                                 double *props, double *s,
                                                                 int *status) {
-  __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   double *pn = reinterpret_cast<double *>(smem + off);
@@ -1010,7 +989,7 @@ static cudaError_t launch_pairs_t(const DevSys &hs, const DevSys *ds, DevPop pop
   const int need = (a.nw + G - 1) / G;
   const int cap = nsm * (per_sm > 0 ? per_sm : 1);
   const int grid = need < cap ? need : cap;
-  pairs_kernel<R, G, LG, kJ><<<grid, G * kThreads, sm, st>>>(ds, pop, a, stage, xe);
+  pairs_kernel<R, G, LG, kJ><<<grid, G * kThreads, sm, st>>>(hs, pop, a, stage, xe);
   return cudaGetLastError();
 }
 
@@ -1069,7 +1048,7 @@ cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const d
   if ((e = launch_real_det(hs, ds, nw, scr, st)) != cudaSuccess) return e;
   const size_t sm = eval_real_smem_bytes(hs);
   if ((e = set_smem((const void *)eval_real_kernel, sm)) != cudaSuccess) return e;
-  eval_real_kernel<<<nw, kThreads, sm, st>>>(ds, nw, real_args(hs, scr), move_scratch(hs), g, hl,
+  eval_real_kernel<<<nw, kThreads, sm, st>>>(hs, nw, real_args(hs, scr), move_scratch(hs), g, hl,
                                              props, s, status);
   return cudaGetLastError();
 }
@@ -1109,7 +1088,7 @@ cudaError_t launch_move(const DevSys &hs, const DevSys *ds, DevPop pop, const Mo
     const size_t sm = move_real_smem_bytes(hs);
     cudaError_t e = set_smem((const void *)move_real_kernel, sm);
     if (e != cudaSuccess) return e;
-    move_real_kernel<<<a.nw, kThreads, sm, st>>>(ds, pop, a, real_args(hs, a.scr),
+    move_real_kernel<<<a.nw, kThreads, sm, st>>>(hs, pop, a, real_args(hs, a.scr),
                                                  move_scratch(hs));
     return cudaGetLastError();
   }

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "real_det.cuh"
 
@@ -236,208 +237,268 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs
 }
 
 // ------------------------------------------------- spins above 32 orbitals
-// One CTA per (walker, spin), four lanes per row: lane s of a row holds the
-// columns 4 j + s in C registers, rotated by one register every four steps
-// so that the pivot column of step k is register 0 of lane k mod 4. As
-// gj_invert_reg a step is one barrier: before it every warp publishes its
-// best candidate row (key, reciprocal, columns), after it every thread takes
-// the best key's row. The whole matrix stays in registers, so a step moves
-// only the pivot row through shared memory: C / 2 16-byte reads for C FP64
-// instructions. Above 128 orbitals the last CS of a lane's C columns, which
-// the registers of one SM cannot hold, live in shared memory as a ring that
-// the rotation feeds from. When both spins have at most kRealFused orbitals the
+// One CTA per (walker, spin), the whole Gauss-Jordan matrix in registers: kL
+// lanes share kR rows, lane s holding their columns kL j + s in kC registers
+// per row, rotated by one every kL steps so that the pivot column of step k
+// is register 0 of lane k mod kL. As gj_invert_reg a step is
+// one barrier: before it every warp publishes its best candidate row (key,
+// reciprocal, columns), after it every thread takes the best key's row. Bound
+// by shared-memory wavefronts and the step's latency chain: a pivot-row value
+// read once serves kR rows (one row per four lanes, every value used once,
+// kept the shared-memory pipe 61% and the FP64 pipe 15% busy: 0.29 ms for
+// 2048 matrices of 61, 3.5 ms for 768 of 161).
+// Above 128 orbitals the last kS columns of a lane, which the registers of
+// one SM cannot hold, live in shared memory as a ring that the rotation
+// feeds from. When both spins have at most kRealFused orbitals the
 // transposed inverse and the orbitals then share the CTA's memory and F
 // comes from the FP64 tensor cores here; else both go to device memory for
 // real_f_kernel.
-template <int C>
-__host__ __device__ constexpr int gjc_lane_stride() {  // doubles between the lanes' columns
-  return (C + 1) / 2 * 2 + 2;
+// doubles between the lanes' columns in a published row: twice an odd number,
+// so the lanes' 16-byte reads fall on distinct banks
+__host__ __device__ constexpr int gjc_stride(int c) { return ((c + 1) / 2 | 1) * 2; }
+__host__ __device__ constexpr int gjc_slot(int l, int c) { return l * gjc_stride(c) + 2; }
+__host__ __device__ inline int gjc_warps(int n, int l, int rows) {
+  const int r = 32 / l * rows;  // rows per warp
+  return (n + r - 1) / r;
 }
-template <int C>
-__host__ __device__ constexpr int gjc_slot() {  // a published row: four lanes' columns, 1 / pivot, |pivot|
-  return 4 * gjc_lane_stride<C>() + 2;
-}
-template <int C, int NT, int CS>
-constexpr size_t inv_cta_doubles(int n, bool fused) {
-  // candidate rows and ring; fused: the transposed inverse in their place (the
-  // ring is empty there), the orbitals, the scaled wave vectors
-  const size_t gj = (size_t)2 * (NT / 32) * gjc_slot<C>() + (size_t)CS * NT;
+inline size_t inv_cta_doubles(int n, int l, int rows, int c, int ring, bool fused) {
+  // candidate rows and ring; fused: the transposed inverse in their place (there
+  // is no ring), the orbitals, the scaled wave vectors
+  const size_t g = gjc_warps(n, l, rows), gj = 2 * g * gjc_slot(l, c) + (size_t)ring * rows * 32 * g;
   if (!fused) return gj;
   const size_t m = (size_t)(n + 3) * odd4(n);
-  return (gj > m ? gj : m) + m + 2 * (n + 8);
+  return std::max(gj, m) + m + 2 * (n + 8);
 }
 
-template <int C, int NT, int MB, int CS, bool kFused>
-__global__ void __launch_bounds__(NT, MB) real_inv_cta_kernel(RealArgs a, int nw) {
-  constexpr int CR = C - CS, G = NT / 32, LS = gjc_lane_stride<C>(), SL = gjc_slot<C>();
-  static_assert(!kFused || CS == 0, "the ring would share its place");
+template <int kL, int kR, int kC, int kS, int kMaxT, int kMB, bool kFused>
+__global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, int nw) {
+  constexpr int CR = kC - kS, LS = gjc_stride(kC), SL = gjc_slot(kL, kC), RW = 32 / kL * kR;
+  static_assert(!kFused || kS == 0, "the ring would share its place");
+  static_assert(kC > 1, "the next pivot column is register 1 at a rotation");
   __shared__ unsigned keys[2][32];
-  __shared__ double red[G];
-  __shared__ int perm[NT / 4];
+  __shared__ double red[32], rinv[176], dk[176];
+  __shared__ int perm[176], rowl[176];
   __shared__ int singular;
   extern __shared__ __align__(16) char smem[];
   const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0];
   if (w >= nw || n <= 32) return;  // whole CTAs
-  const int t = threadIdx.x, lane = t & 31, wp = t >> 5, r = t >> 2, s = t & 3;
-  double *slots = reinterpret_cast<double *>(smem);  // [2][G][SL]
-  // logical column CR + i of this thread at xs[((hd + i) mod CS) NT]
-  double *xs = slots + (size_t)2 * G * SL + t;
+  const int t = threadIdx.x, nthr = blockDim.x, G = nthr >> 5, lane = t & 31, wp = t >> 5;
+  const int s = lane & (kL - 1), r0 = wp * RW + lane / kL * kR;  // first of its rows
+  double *slots = reinterpret_cast<double *>(smem);                  // [2][G][SL]
+  // logical column CR + i of row q at xs[(((hd + i) mod kS) kR + q) nthr]
+  double *xs = slots + 2 * G * SL + t;
   int hd = 0;
-  auto xcol = [&](int i) -> double & {
-    const int q = hd + i;
-    return xs[(q >= CS ? q - CS : q) * NT];
+  auto xcol = [&](int i, int q) -> double & {
+    const int h = hd + i;
+    return xs[((h >= kS ? h - kS : h) * kR + q) * nthr];
   };
   double *base = real_base(a, w);
   const int ldw = spn ? a.ldw[1] : a.ldw[0], ld = odd4(n);
   double *Wg = base + (spn ? a.w[1] : a.w[0]), *Bg = Wg + n * ldw;  // !kFused
   double *F = base + (spn ? a.f[1] : a.f[0]);
   // kFused: the inverse over the candidate rows, the orbitals behind it
-  const size_t gj = (size_t)2 * G * SL, mat = (size_t)(n + 3) * ld;
-  double *Wt = slots, *Bs = slots + (gj > mat ? gj : mat);
+  const int gj = 2 * G * SL, mat = (n + 3) * ld;
+  double *Wt = slots, *Bs = slots + max(gj, mat);
   double2 *sg = reinterpret_cast<double2 *>(Bs + mat);
   auto bat = [&](int o, int j) -> double & {
     return kFused ? Bs[o * ld + j] : Bg[o * ldw + j];
   };
   if (t == 0) singular = 0;
   if (t < 64) keys[t >> 5][t & 31] = 0u;
-  orbital_rows(a, a.scr + w * a.stride + a.l_q + 2 * (spn ? a.f0[1] : a.f0[0]), n, t, NT, bat);
+  orbital_rows(a, a.scr + w * a.stride + a.l_q + 2 * (spn ? a.f0[1] : a.f0[0]), n, t, nthr, bat);
   if (kFused) {
-    for (int o = t; o < n + 8; o += NT) sg[o] = orbital_g(a.gvec, o, n);
-    for (int e = t; e < 3 * ld; e += NT) Bs[n * ld + e] = 0.0;  // read past the last row
-    for (int e = t; e < n * (ld - n); e += NT) {
+    for (int o = t; o < n + 8; o += nthr) sg[o] = orbital_g(a.gvec, o, n);
+    for (int e = t; e < 3 * ld; e += nthr) Bs[n * ld + e] = 0.0;  // read past the last row
+    for (int e = t; e < n * (ld - n); e += nthr) {
       const int k = e / (ld - n);
       Bs[k * ld + n + e - k * (ld - n)] = 0.0;
     }
   }
   __syncthreads();
-  const bool row = r < n;
-  auto first_col = [&](int j) { return row && 4 * j + s < n ? bat(r, 4 * j + s) : 0.0; };
-  double v[CR];
+  auto first = [&](int q, int j) {
+    return r0 + q < n && kL * j + s < n ? bat(r0 + q, kL * j + s) : 0.0;
+  };
+  double v[kR][CR];
 #pragma unroll
-  for (int j = 0; j < CR; j++) v[j] = first_col(j);
-  for (int i = 0; i < CS; i++) xcol(i) = first_col(CR + i);
-  bool used = !row;
-  double my_inv = 1.0, my_d = 1.0;
-  int my_l = 0;
-  // step k's candidate of this warp: own is the lane that holds column k in x
-  auto publish = [&](int k, unsigned wk, bool own, double x, double rx) {
-    double *sl = slots + (size_t)((k & 1) * G + wp) * SL;
-    if (wk != 0u && r == 255 - (int)(wk & 0xFFu)) {
+  for (int q = 0; q < kR; q++) {
 #pragma unroll
-      for (int j = 0; j < CR; j += 2)
-        *reinterpret_cast<double2 *>(sl + s * LS + j) =
-            make_double2(v[j], j + 1 < CR ? v[j + 1] : 0.0);
-      for (int i = 0; i < CS; i++) sl[s * LS + CR + i] = xcol(i);
-      if (own) *reinterpret_cast<double2 *>(sl + 4 * LS) = make_double2(rx, fabs(x));
+    for (int j = 0; j < CR; j++) v[q][j] = first(q, j);
+#pragma unroll
+    for (int i = 0; i < kS; i++) xcol(i, q) = first(q, CR + i);
+  }
+  unsigned used = 0;
+#pragma unroll
+  for (int q = 0; q < kR; q++) used |= (r0 + q < n ? 0u : 1u) << q;
+  // a column's best candidate among this thread's rows x[q]
+  auto best_key = [&](const double (&x)[kR], bool own) -> unsigned {
+    unsigned b = 0u;
+#pragma unroll
+    for (int q = 0; q < kR; q++)
+      b = max(b, pivot_key(x[q], r0 + q, own && !((used >> q) & 1u)));
+    return b;
+  };
+  auto pick = [&](const double (&x)[kR], int i) -> double {
+    double y = x[0];
+#pragma unroll
+    for (int q = 1; q < kR; q++) y = i == q ? x[q] : y;
+    return y;
+  };
+  // step k's candidate of this warp, whose column k is x in the lanes own
+  auto publish = [&](int k, unsigned wk, bool own, const double (&x)[kR]) {
+    double *sl = slots + ((k & 1) * G + wp) * SL;
+    const int i = 255 - (int)(wk & 0xFFu) - r0;
+    if (wk != 0u && i >= 0 && i < kR) {
+#pragma unroll
+      for (int q = 0; q < kR; q++)
+        if (i == q) {
+#pragma unroll
+          for (int j = 0; j < CR; j += 2)
+            *reinterpret_cast<double2 *>(sl + s * LS + j) =
+                make_double2(v[q][j], j + 1 < CR ? v[q][j + 1] : 0.0);
+        }
+#pragma unroll
+      for (int c = 0; c < kS; c++) sl[s * LS + CR + c] = xcol(c, i);
+      if (own) {
+        const double y = pick(x, i);
+        *reinterpret_cast<double2 *>(sl + kL * LS) = make_double2(rcp_newton(y), fabs(y));
+      }
     }
     if (lane == 0) keys[k & 1][wp] = wk;
   };
-  double f;  // this row's entry of the pivot column
+  double f[kR];  // the rows' entries of the pivot column
   {
+    double x[kR];
+#pragma unroll
+    for (int q = 0; q < kR; q++) x[q] = v[q][0];
     const bool own = s == 0;
-    const unsigned wk = __reduce_max_sync(0xffffffffu, pivot_key(v[0], r, own && !used));
-    publish(0, wk, own, v[0], rcp_newton(v[0]));
-    f = __shfl_sync(0xffffffffu, v[0], 0, 4);
+    publish(0, __reduce_max_sync(0xffffffffu, best_key(x, own)), own, x);
+#pragma unroll
+    for (int q = 0; q < kR; q++) f[q] = __shfl_sync(0xffffffffu, x[q], 0, kL);
   }
-  const int macros = (n + 3) / 4;
-#pragma unroll 1
-  for (int m = 0; m < macros; m++) {
+  // one step; kRot: the last of kL, which rotates the columns
+  auto step = [&](int k, int u, auto rot) {
+    constexpr bool kRot = decltype(rot)::value;
+    __syncthreads();
+    const unsigned best = __reduce_max_sync(0xffffffffu, keys[k & 1][lane]);
+    const int p = 255 - (int)(best & 0xFFu);
+    const double *ps = slots + ((k & 1) * G + p / RW) * SL;
+    const double inv = ps[kL * LS];
+    if (t == 0) {
+      perm[k] = p;
+      rowl[p] = k;
+      rinv[p] = inv;
+      dk[k] = ps[kL * LS + 1];
+      if ((best >> 8) == 0u) singular = 1;
+    }
+    double fac[kR];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int k = 4 * m + u;
-      if (k < n) {
-        __syncthreads();
-        const unsigned best = __reduce_max_sync(0xffffffffu, keys[k & 1][lane]);
-        const int p = 255 - (int)(best & 0xFFu);
-        const double *ps = slots + (size_t)((k & 1) * G + (p >> 3)) * SL;
-        const double inv = ps[4 * LS];
-        if (t == 0) {
-          perm[k] = p;
-          if ((best >> 8) == 0u) singular = 1;
-        }
-        const bool piv = r == p;
-        used = used || piv;
-        if (piv) {
-          my_inv = inv;
-          my_d = ps[4 * LS + 1];
-          my_l = k;
-        }
-        const double fac = piv ? 0.0 : f * inv;
-        const double *pc = ps + s * LS;
-        // the register of column k + 1 first: the next key needs it
-        const int jn = u == 3 ? 1 : 0;  // before the rotation
-        const double xn = fma(-fac, pc[jn], v[jn]);
-        const bool ownn = s == ((u + 1) & 3);
-        const unsigned wk = __reduce_max_sync(0xffffffffu, pivot_key(xn, r, ownn && !used));
-        const double rx = rcp_newton(xn);
-        const double2 *b = reinterpret_cast<const double2 *>(pc);
-        const double done = piv ? 1.0 : -fac;  // the eliminated column
-        if (u < 3) {
+    for (int q = 0; q < kR; q++) fac[q] = r0 + q == p ? 0.0 : f[q] * inv;
+    if (p >= r0 && p < r0 + kR) used |= 1u << (p - r0);
+    const double *pc = ps + s * LS;
+    // the registers of column k + 1 first: the next key needs them
+    constexpr int jn = kRot ? 1 : 0;  // before the rotation
+    const bool ownn = s == (kRot ? 0 : u + 1);
+    double x[kR];
+    {
+      const double b = pc[jn];
 #pragma unroll
-          for (int j = 0; j < CR; j += 2) {
-            const double2 bb = b[j / 2];
-            v[j] = fma(-fac, bb.x, v[j]);
-            if (j + 1 < CR) v[j + 1] = fma(-fac, bb.y, v[j + 1]);
-          }
-#pragma unroll 4
-          for (int i = 0; i < CS; i++) xcol(i) = fma(-fac, pc[CR + i], xcol(i));
-          if (s == u) v[0] = done;
-        } else {
-          const double first = s == u ? done : fma(-fac, pc[0], v[0]);
+      for (int q = 0; q < kR; q++) x[q] = fma(-fac[q], b, v[q][jn < CR ? jn : 0]);
+    }
+    const unsigned wk = __reduce_max_sync(0xffffffffu, best_key(x, ownn));
+    double done[kR];  // the eliminated column
 #pragma unroll
-          for (int j = 0; j < CR; j += 2) {
-            const double2 bb = b[j / 2];
-            if (j) v[j - 1] = fma(-fac, bb.x, v[j]);
-            if (j + 1 < CR) v[j] = fma(-fac, bb.y, v[j + 1]);
-          }
-          if constexpr (CS > 0) {
-            v[CR - 1] = fma(-fac, pc[CR], xcol(0));
-#pragma unroll 4
-            for (int i = 1; i < CS; i++) xcol(i) = fma(-fac, pc[CR + i], xcol(i));
-            xcol(0) = first;
-            hd = hd + 1 == CS ? 0 : hd + 1;
-          } else {
-            v[CR - 1] = first;
-          }
-        }
-        if (k + 1 < n) {
-          publish(k + 1, wk, ownn, xn, rx);
-          f = __shfl_sync(0xffffffffu, v[0], (u + 1) & 3, 4);
-        }
-      } else if (u == 3) {
-        // past the last step: the rotation alone
-        const double first = v[0];
+    for (int q = 0; q < kR; q++) done[q] = r0 + q == p ? 1.0 : -fac[q];
+    const bool own = s == u;
+    if (!kRot) {
 #pragma unroll
-        for (int j = 1; j < CR; j++) v[j - 1] = v[j];
-        if constexpr (CS > 0) {
-          v[CR - 1] = xcol(0);
-          xcol(0) = first;
-          hd = hd + 1 == CS ? 0 : hd + 1;
-        } else {
-          v[CR - 1] = first;
+      for (int j = 0; j < CR; j += 2) {
+        const double2 b = *reinterpret_cast<const double2 *>(pc + j);
+#pragma unroll
+        for (int q = 0; q < kR; q++) {
+          v[q][j] = fma(-fac[q], b.x, v[q][j]);
+          if (j + 1 < CR) v[q][j + 1] = fma(-fac[q], b.y, v[q][j + 1]);
         }
       }
+#pragma unroll
+      for (int c = 0; c < kS; c++) {
+        const double b = pc[CR + c];
+#pragma unroll
+        for (int q = 0; q < kR; q++) xcol(c, q) = fma(-fac[q], b, xcol(c, q));
+      }
+#pragma unroll
+      for (int q = 0; q < kR; q++) v[q][0] = own ? done[q] : v[q][0];
+    } else {
+      double head[kR];
+#pragma unroll
+      for (int j = 0; j < CR; j += 2) {
+        const double2 b = *reinterpret_cast<const double2 *>(pc + j);
+#pragma unroll
+        for (int q = 0; q < kR; q++) {
+          if (j) v[q][j - 1] = fma(-fac[q], b.x, v[q][j]);
+          else head[q] = own ? done[q] : fma(-fac[q], b.x, v[q][0]);
+          if (j + 1 < CR) v[q][j] = fma(-fac[q], b.y, v[q][j + 1]);
+        }
+      }
+      if constexpr (kS > 0) {
+        const double b = pc[CR];
+#pragma unroll
+        for (int q = 0; q < kR; q++) v[q][CR - 1] = fma(-fac[q], b, xcol(0, q));
+#pragma unroll
+        for (int c = 1; c < kS; c++) {
+          const double bc = pc[CR + c];
+#pragma unroll
+          for (int q = 0; q < kR; q++) xcol(c, q) = fma(-fac[q], bc, xcol(c, q));
+        }
+#pragma unroll
+        for (int q = 0; q < kR; q++) xcol(0, q) = head[q];
+        hd = hd + 1 == kS ? 0 : hd + 1;
+      } else {
+#pragma unroll
+        for (int q = 0; q < kR; q++) v[q][CR - 1] = head[q];
+      }
+    }
+    if (k + 1 < n) {
+      publish(k + 1, wk, ownn, x);
+#pragma unroll
+      for (int q = 0; q < kR; q++)
+        f[q] = __shfl_sync(0xffffffffu, v[q][0], kRot ? 0 : u + 1, kL);
+    }
+  };
+  int turns = 0;  // rotations done
+#pragma unroll 1
+  for (int k0 = 0; k0 < n; k0 += kL) {
+    const int m = min(kL - 1, n - k0);
+#pragma unroll 1
+    for (int u = 0; u < m; u++) step(k0 + u, u, std::false_type());
+    if (k0 + kL - 1 < n) {
+      step(k0 + kL - 1, kL - 1, std::true_type());
+      turns++;
     }
   }
-  __syncthreads();  // perm; the last step's candidates are read
+  __syncthreads();  // perm, rowl, rinv, dk; the last step's candidates are read
   // rows normalised by their own pivot, transposed and in orbital order;
-  // register j holds column 4 ((macros + j) mod C) + s
-  auto store = [&](int j, double x) {
-    const int m = macros + j, c = 4 * (m >= C ? m - C : m) + s;
-    if (row && c < n) (kFused ? Wt + perm[c] * ld : Wg + perm[c] * ldw)[my_l] = x * my_inv;
+  // register j holds column kL ((turns + j) mod kC) + s
+  auto store = [&](int j, int q, double x) {
+    const int m = turns + j, c = kL * (m >= kC ? m - kC : m) + s, r = r0 + q;
+    if (r < n && c < n)
+      (kFused ? Wt + perm[c] * ld : Wg + perm[c] * ldw)[rowl[r]] = x * rinv[r];
   };
 #pragma unroll
-  for (int j = 0; j < CR; j++) store(j, v[j]);
-  for (int i = 0; i < CS; i++) store(CR + i, xcol(i));
+  for (int q = 0; q < kR; q++) {
+#pragma unroll
+    for (int j = 0; j < CR; j++) store(j, q, v[q][j]);
+#pragma unroll
+    for (int i = 0; i < kS; i++) store(CR + i, q, xcol(i, q));
+  }
   if (kFused) {
-    for (int e = t; e < 3 * ld; e += NT) Wt[n * ld + e] = 0.0;
-    for (int e = t; e < n * (ld - n); e += NT) {
+    for (int e = t; e < 3 * ld; e += nthr) Wt[n * ld + e] = 0.0;
+    for (int e = t; e < n * (ld - n); e += nthr) {
       const int k = e / (ld - n);
       Wt[k * ld + n + e - k * (ld - n)] = 0.0;
     }
   }
-  double lg = row && s == 0 ? log(my_d) : 0.0;
+  double lg = t < n ? log(dk[t]) : 0.0;
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, q);
   if (lane == 0) red[wp] = lg;
@@ -449,19 +510,27 @@ __global__ void __launch_bounds__(NT, MB) real_inv_cta_kernel(RealArgs a, int nw
     F[2 * n * n + 1] = (double)singular;
   }
   if constexpr (kFused) {
-    if (t < n) {
+    // D2_l = -sum_o Dinv(l, o) g_a g_b D(o, l), eight lanes per electron
+    for (int lb = 0; lb < n; lb += nthr / 8) {
+      const int l = lb + (t >> 3);
       double xx = 0.0, xy = 0.0, yy = 0.0;
-      for (int o = 0; o < n - 1; o++) {
-        const double x = Wt[o * ld + t] * Bs[o * ld + t];
-        const double2 g = sg[o];
-        xx -= x * (g.x * g.x);
-        xy -= x * (g.x * g.y);
-        yy -= x * (g.y * g.y);
+      if (l < n)
+        for (int o = t & 7; o < n - 1; o += 8) {
+          const double x = Wt[o * ld + l] * Bs[o * ld + l];
+          const double2 g = sg[o];
+          xx -= x * (g.x * g.x);
+          xy -= x * (g.x * g.y);
+          yy -= x * (g.y * g.y);
+        }
+      xx = group8_sum(xx);
+      xy = group8_sum(xy);
+      yy = group8_sum(yy);
+      if (l < n && (t & 7) == 0) {
+        double *d2 = F + 2 * n * n + 2 + 3 * l;
+        d2[0] = xx;
+        d2[1] = xy;
+        d2[2] = yy;
       }
-      double *d2 = F + 2 * n * n + 2;
-      d2[3 * t] = xx;
-      d2[3 * t + 1] = xy;
-      d2[3 * t + 2] = yy;
     }
     // items of one row tile and up to four column tiles
     const int T = (n + 7) / 8, TC = (T + 3) / 4;
@@ -710,7 +779,7 @@ inline size_t s_smem_doubles(int n, int cols, bool resident) {
   return head + (resident ? (size_t)3 * n * odd4(cols) : (size_t)2 * 3 * n * s_chunk(n));
 }
 
-constexpr int kSMaxThreads = 640;  // kB = 1
+constexpr int kSMaxThreads = 768;  // kB = 1: at most 80 registers, 24 warps on an SM
 
 template <int kB>
 __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
@@ -785,13 +854,19 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
     __syncthreads();
     mark(PH_DRIFT);
     drift(jac, 0, cols);
-    for (int it = warp; it < pairs; it += NW) {
+    // (tile pair, type) items in whole runs per warp: a tile pair whose types
+    // fall to two warps is contracted by both
+    const int items = pairs * nt, i0 = items * warp / NW, i1 = items * (warp + 1) / NW;
+    for (int it = i0; it < i1;) {
+      const int tp = nt > 1 ? it >> 1 : it;
+      const bool first = nt == 1 || !(it & 1), second = nt > 1 && 2 * tp + 1 < i1;
       int tj, tk;
-      tile_pair(it, &tj, &tk);
+      tile_pair(tp, &tj, &tk);
       double acc[2][1][1][4][2] = {};
-      s_products<1>(acc[0], jac, ld, n, tj, tk, 0, pad0);
-      if (nt > 1) s_products<1>(acc[1], jac, ld, n, tj, tk, pad0, cols);
+      if (first) s_products<1>(acc[0], jac, ld, n, tj, tk, 0, pad0);
+      if (second) s_products<1>(acc[1], jac, ld, n, tj, tk, pad0, cols);
       s_contract<1, 2>(acc, FX, d2, n, tj, tk, lt);
+      it = (nt > 1 ? 2 * tp + 1 : tp) + 1;
     }
   } else {
     const int rounds = (pairs + NW - 1) / NW;
@@ -853,22 +928,13 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   mark(PH_CROSS);
 }
 
-// Warps per CTA of the resident form: whole rounds of tile pairs, and about
-// 20 warps on an SM with the CTAs that its shared memory holds.
-int s_warps(int n, size_t smem) {
-  const int T = (n + 7) / 8, pairs = T * (T + 1) / 2, ctas = std::max<int>(1, 227 * 1024 / (int)(smem + 1024));
-  double best = 0.0;
-  int nw = 1;
-  for (int k = 2; k <= kSMaxThreads / 32; k++) {
-    const double fill = (double)pairs / ((pairs + k - 1) / k * k);
-    const int res = std::min(ctas * k, 64);
-    const double score = fill * std::min(1.0, res / 20.0) - 0.002 * k;
-    if (score > best) {
-      best = score;
-      nw = k;
-    }
-  }
-  return nw;
+// Warps per CTA of the resident form: a multiple of four, so that the four
+// sub-partitions' FP64 pipes get equal shares (five warps at 29 orbitals: the
+// first sub-partition two fifths of the products), about 20 on an SM with the
+// CTAs that its shared memory holds.
+int s_warps(size_t smem) {
+  const int ctas = 227 * 1024 / (int)(smem + 1024);
+  return ctas >= 4 ? 4 : ctas == 3 ? 8 : ctas == 2 ? 12 : 16;
 }
 
 cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int nw,
@@ -885,20 +951,19 @@ cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int 
   cudaError_t e = raise_smem_limit(k, sm);
   if (e != cudaSuccess) return e;
   if (resident)
-    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st>>>(a, ds, nw);
+    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(sm), sm, st>>>(a, ds, nw);
   else
     real_s_kernel<2><<<nw * hs.nt, 512, sm, st>>>(a, ds, nw);
   return cudaGetLastError();
 }
 
-template <int C, int NT, int MB, int CS = 0>
+template <int kL, int kR, int kC, int kS, int kMaxT, int kMB, bool kFused>
 cudaError_t launch_inv_cta(const RealArgs &a, int n, int items, int nw, cudaStream_t st) {
-  constexpr bool fused = CS == 0 && NT <= 480;
-  const size_t sm = sizeof(double) * inv_cta_doubles<C, NT, CS>(n, fused);
-  const void *k = (const void *)real_inv_cta_kernel<C, NT, MB, CS, fused>;
-  cudaError_t e = raise_smem_limit(k, sm);
+  const size_t sm = sizeof(double) * inv_cta_doubles(n, kL, kR, kC, kS, kFused);
+  auto k = real_inv_cta_kernel<kL, kR, kC, kS, kMaxT, kMB, kFused>;
+  cudaError_t e = raise_smem_limit((const void *)k, sm);
   if (e != cudaSuccess) return e;
-  real_inv_cta_kernel<C, NT, MB, CS, fused><<<items, NT, sm, st>>>(a, nw);
+  k<<<items, 32 * gjc_warps(n, kL, kR), sm, st>>>(a, nw);
   return cudaGetLastError();
 }
 
@@ -928,17 +993,18 @@ cudaError_t launch_orbitals_f(const DevSys &hs, const RealArgs &a, int nw, cudaS
     // spins on both sides of 32: the warp kernel takes the smaller one
     if ((e = launch_det_warp<32>(a, items, nw, st)) != cudaSuccess) return e;
   }
-  // columns per lane, threads (four lanes per row, rows <= NT / 4), CTAs per
-  // SM that the registers are kept for, columns in shared memory
-  e = nm <= 40            ? launch_inv_cta<10, 160, 6>(a, nm, items, nw, st)
-      : nm <= 48          ? launch_inv_cta<12, 192, 5>(a, nm, items, nw, st)
-      : nm <= 64          ? launch_inv_cta<16, 256, 3>(a, nm, items, nw, st)
-      : nm <= 84          ? launch_inv_cta<21, 352, 2>(a, nm, items, nw, st)
-      : nm <= 104         ? launch_inv_cta<26, 416, 1>(a, nm, items, nw, st)
-      : nm <= kRealFused  ? launch_inv_cta<29, 480, 1>(a, nm, items, nw, st)
-      : nm <= 128         ? launch_inv_cta<32, 512, 1, 4>(a, nm, items, nw, st)
-      : nm <= 152         ? launch_inv_cta<38, 608, 1, 12>(a, nm, items, nw, st)
-                          : launch_inv_cta<41, 672, 1, 21>(a, nm, items, nw, st);
+  // lanes per group of rows, rows, columns per lane, of them in shared memory,
+  // most threads, CTAs per SM that the registers are kept for
+  e = nm <= 40           ? launch_inv_cta<8, 4, 5, 0, 96, 6, true>(a, nm, items, nw, st)
+      : nm <= 48         ? launch_inv_cta<8, 4, 6, 0, 96, 6, true>(a, nm, items, nw, st)
+      : nm <= 64         ? launch_inv_cta<8, 4, 8, 0, 128, 3, true>(a, nm, items, nw, st)
+      : nm <= 88         ? launch_inv_cta<8, 4, 11, 0, 192, 2, true>(a, nm, items, nw, st)
+      : nm <= 104        ? launch_inv_cta<8, 4, 13, 0, 224, 1, true>(a, nm, items, nw, st)
+      : nm <= kRealFused ? launch_inv_cta<8, 4, 15, 0, 256, 1, true>(a, nm, items, nw, st)
+      : nm <= 128        ? launch_inv_cta<8, 4, 16, 0, 256, 1, false>(a, nm, items, nw, st)
+      : nm <= 144        ? launch_inv_cta<16, 8, 9, 1, 288, 1, false>(a, nm, items, nw, st)
+      : nm <= 160        ? launch_inv_cta<16, 8, 10, 2, 320, 1, false>(a, nm, items, nw, st)
+                         : launch_inv_cta<16, 8, 11, 3, 352, 1, false>(a, nm, items, nw, st);
   if (e != cudaSuccess || nm <= kRealFused) return e;
   const int blocks = (nm + 31) / 32;
   const size_t sm = sizeof(double) * real_f_doubles(nm, (nm + 3) & ~3);

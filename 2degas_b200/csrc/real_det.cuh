@@ -107,6 +107,25 @@ __host__ __device__ inline size_t real_carve(const DevSys &s, char *base, EvalSm
 cudaError_t launch_real_det(const DevSys &hs, const DevSys *ds, int nw, double *scr,
                             cudaStream_t st);
 
+// The pair passes' sums of walker w into shared memory, the determinant sums
+// zeroed (asynchronous 8-byte copies; the caller waits).
+__device__ __forceinline__ void load_real_sums(const DevSys &S, const EvalSmem &m,
+                                               const double *o, const MoveScratch &L) {
+  const int N = S.N, tid = threadIdx.x;
+  for (int j = tid; j < 2 * N; j += kThreads) {
+    cp_async8(m.x + j, o + L.x + j);
+    cp_async8(m.g + j, o + L.g + j);
+  }
+  for (int j = tid; j < N; j += kThreads) {
+    cp_async8(m.lap + j, o + L.lap + j);
+    cp_async8(m.ltf + j, o + L.ltf + j);
+    cp_async8(m.vp + j, o + L.vp + j);
+    m.lapd[j] = 0.0;
+    m.ph2[j] = 0.0;
+    m.ph2d[j] = 0.0;
+  }
+}
+
 // The end of an evaluation after launch_real_det, as eval_det: m holds x, g,
 // lap, ltf, vp of the pair passes (their asynchronous copies may be in
 // flight) and zeroed lapd, ph2, ph2d; o is the walker's scratch block, base its

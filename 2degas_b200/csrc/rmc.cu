@@ -10,6 +10,7 @@
 #include "../../include/qmc2d.h"
 #include "common.h"
 #include "kernels.cuh"
+#include "real_det.cuh"
 #include "rmc.cuh"
 #include "walker_eval.cuh"
 
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_move_kernel(const DevSys *sp,
 // and, after the reptile's last growth of the move, the path tail. A move
 // of mdelta > 1 takes mdelta launch pairs; a reptile whose move has fewer
 // growths skips the later ones.
-template <class R, int G, int LG>
+template <class R, int G, int LG, bool kJ>
 __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(const DevSys *sp,
                                                                         RmcArgs a, double *scr,
                                                                         int idelta,
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(const De
   const int N = S.N, N2 = 2 * N, nb = a.nbuf;
   const uint32_t t = a.step0;
   const double pi = 3.141592653589793;
-  const MoveScratch L = move_scratch(S, false);
+  const MoveScratch L = move_scratch(S, kJ);
   for (int r = blockIdx.x * G + grp; r < a.nrep; r += gridDim.x * G) {
     int idir, ndelta;
     rmc_dir(a, r, t, idir, ndelta);
@@ -583,12 +584,14 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(const De
     const double lng = block_sum_t<kThreads>(wg, m.red, sync, tid);
     phase_mark(S, PH_PROPOSE, tph, tid == 0);
     double *o = scr + (size_t)r * L.stride;
-    double *pout = (S.has_bf && !S.bf_zero) ? o + L.pair : nullptr;
+    double *pout = !S.has_bf || S.bf_zero ? nullptr
+                   : kJ && S.gmat         ? S.gmat_base + (size_t)r * S.gmat_stride
+                                          : o + L.pair;
     if (stage_rows)
-      eval_pairs<kThreads, true, R, GroupSync, LG>(S, m, tph, pout, (const R *)rows_s, sync,
-                                                   tid);
+      eval_pairs<kThreads, true, R, GroupSync, LG, kJ>(S, m, tph, pout, (const R *)rows_s, sync,
+                                                       tid);
     else
-      eval_pairs<kThreads, false, R, GroupSync, LG>(S, m, tph, pout, rows_g, sync, tid);
+      eval_pairs<kThreads, false, R, GroupSync, LG, kJ>(S, m, tph, pout, rows_g, sync, tid);
     pair_rhok<LG>(S, m, tid, kThreads, sync);
     sync();
     for (int e = tid; e < 4 * S.nk; e += kThreads) o[L.rhok + e] = m.rhok[e];
@@ -613,62 +616,17 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(const De
   }
 }
 
-template <bool kGmat>
-__global__ void __launch_bounds__(kThreads, 2) rmc_det_kernel(const DevSys *sp, RmcArgs a,
-                                                              const double *scr, int idelta) {
-  __shared__ DevSys S;
-  extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
-  EvalSmem m;
-  size_t off = eval_carve<kGmat>(S, smem, &m, kGmat ? gmat_block(S, blockIdx.x) : nullptr);
-  double *pn = reinterpret_cast<double *>(smem + off);
-  double *pp = pn + S.nprops;
-  double *ppo = pp + S.nprops;
-  double *blk = ppo + S.nprops;
-  double *psum = blk + S.nprops;
-  double *hn = psum + S.nprops;
-  double *sc = hn + 2;
-  const int r = blockIdx.x, tid = threadIdx.x;
-  if (r >= a.nrep) return;
-  const uint32_t t = a.step0;
-  int idir, ndelta;
-  rmc_dir(a, r, t, idir, ndelta);
-  if (idelta > ndelta) return;  // the whole CTA
-  const int N = S.N, N2 = 2 * N, nb = a.nbuf;
-  const MoveScratch L = move_scratch(S, false);
-  const double *o = scr + (size_t)r * L.stride;
-  const bool pairs_stored = S.has_bf && !S.bf_zero;
-  if (pairs_stored) {
-    // bring the stored pair values back into L2 before the Jacobian build
-    const size_t bytes = (sizeof(double) * 3 * pair_count(N)) & ~size_t(15);
-    const char *base = reinterpret_cast<const char *>(o + L.pair);
-    for (size_t b0 = (size_t)tid * 32768; b0 < bytes; b0 += (size_t)kThreads * 32768) {
-      const unsigned sz = (unsigned)(bytes - b0 < 32768 ? bytes - b0 : 32768);
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + b0), "r"(sz)
-                   : "memory");
-    }
-  }
-  for (int e = tid; e < N2; e += kThreads) {
-    m.x[e] = o[L.x + e];
-    m.g[e] = o[L.g + e];
-    m.q[e] = o[L.q + e];
-    m.qbd[e] = o[L.qbd + e];
-    m.gd[e] = 0.0;
-  }
-  for (int e = tid; e < 3 * N; e += kThreads) m.Sb[e] = o[L.sb + e];
-  for (int e = tid; e < N; e += kThreads) {
-    m.lap[e] = o[L.lap + e];
-    m.ltf[e] = o[L.ltf + e];
-    m.vp[e] = o[L.vp + e];
-    m.lapd[e] = 0.0;
-    m.ph2[e] = 0.0;
-    m.ph2d[e] = 0.0;
-  }
+// A split bead growth after its evaluation: the bead's tail and, after the
+// reptile's last growth of the move, the path tail. pn: the proposal's
+// properties, then four arrays of nprops for the path's sums.
+__device__ void rmc_finish(const DevSys &S, const RmcArgs &a, const EvalSmem &m, int r, uint32_t t,
+                           int idir, int ndelta, int idelta, const double *o,
+                           const MoveScratch &L, int status, double *pn, double *hn, double *sc,
+                           long long &tph) {
+  const int tid = threadIdx.x, nb = a.nbuf;
   const double wold = o[L.wold], dold = o[L.dold], lng = o[L.lng];
-  __syncthreads();
-  long long tph = clock64();
-  const int status = eval_det<kGmat>(S, m, hn, pn, sc, tph, pairs_stored ? o + L.pair : nullptr,
-                                     o + L.rhok);
+  double *pp = pn + S.nprops, *ppo = pp + S.nprops, *blk = ppo + S.nprops,
+         *psum = blk + S.nprops;
   const int jstart = idir == 1 ? a.ends[2 * r + 1] : a.ends[2 * r];
   const int j = (jstart + idir * (idelta - 1) + nb) % nb;
   const int jn = (jstart + idir * idelta + nb) % nb;
@@ -700,6 +658,83 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_det_kernel(const DevSys *sp, 
     a.cnt[4 * r + 1] += 1.0;
   }
   phase_mark(S, PH_PATH, tpp);
+}
+
+template <bool kGmat>
+__global__ void __launch_bounds__(kThreads, 2) rmc_det_kernel(const DevSys *sp, RmcArgs a,
+                                                              const double *scr, int idelta) {
+  __shared__ DevSys S;
+  extern __shared__ __align__(16) char smem[];
+  load_sys(S, sp);
+  EvalSmem m;
+  size_t off = eval_carve<kGmat>(S, smem, &m, kGmat ? gmat_block(S, blockIdx.x) : nullptr);
+  double *pn = reinterpret_cast<double *>(smem + off);
+  double *hn = pn + 5 * S.nprops, *sc = hn + 2;
+  const int r = blockIdx.x, tid = threadIdx.x;
+  if (r >= a.nrep) return;
+  const uint32_t t = a.step0;
+  int idir, ndelta;
+  rmc_dir(a, r, t, idir, ndelta);
+  if (idelta > ndelta) return;  // the whole CTA
+  const int N = S.N, N2 = 2 * N;
+  const MoveScratch L = move_scratch(S, false);
+  const double *o = scr + (size_t)r * L.stride;
+  const bool pairs_stored = S.has_bf && !S.bf_zero;
+  if (pairs_stored) {
+    // bring the stored pair values back into L2 before the Jacobian build
+    const size_t bytes = (sizeof(double) * 3 * pair_count(N)) & ~size_t(15);
+    const char *base = reinterpret_cast<const char *>(o + L.pair);
+    for (size_t b0 = (size_t)tid * 32768; b0 < bytes; b0 += (size_t)kThreads * 32768) {
+      const unsigned sz = (unsigned)(bytes - b0 < 32768 ? bytes - b0 : 32768);
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + b0), "r"(sz)
+                   : "memory");
+    }
+  }
+  for (int e = tid; e < N2; e += kThreads) {
+    m.x[e] = o[L.x + e];
+    m.g[e] = o[L.g + e];
+    m.q[e] = o[L.q + e];
+    m.qbd[e] = o[L.qbd + e];
+    m.gd[e] = 0.0;
+  }
+  for (int e = tid; e < 3 * N; e += kThreads) m.Sb[e] = o[L.sb + e];
+  for (int e = tid; e < N; e += kThreads) {
+    m.lap[e] = o[L.lap + e];
+    m.ltf[e] = o[L.ltf + e];
+    m.vp[e] = o[L.vp + e];
+    m.lapd[e] = 0.0;
+    m.ph2[e] = 0.0;
+    m.ph2d[e] = 0.0;
+  }
+  __syncthreads();
+  long long tph = clock64();
+  const int status = eval_det<kGmat>(S, m, hn, pn, sc, tph, pairs_stored ? o + L.pair : nullptr,
+                                     o + L.rhok);
+  rmc_finish(S, a, m, r, t, idir, ndelta, idelta, o, L, status, pn, hn, sc, tph);
+}
+
+// The same with real orbitals, after launch_real_det.
+__global__ void __launch_bounds__(kThreads, 3) rmc_real_kernel(const DevSys *sp, RmcArgs a,
+                                                              RealArgs ra, MoveScratch L,
+                                                              int idelta) {
+  __shared__ DevSys S;
+  extern __shared__ __align__(16) char smem[];
+  load_sys(S, sp);
+  EvalSmem m;
+  const size_t off = real_carve(S, smem, &m);
+  double *pn = reinterpret_cast<double *>(smem + off);
+  double *hn = pn + 5 * S.nprops, *sc = hn + 2;
+  const int r = blockIdx.x;
+  if (r >= a.nrep) return;
+  const uint32_t t = a.step0;
+  int idir, ndelta;
+  rmc_dir(a, r, t, idir, ndelta);
+  if (idelta > ndelta) return;  // the whole CTA
+  const double *o = ra.scr + (size_t)r * L.stride;
+  load_real_sums(S, m, o, L);
+  long long tph = clock64();
+  const int status = eval_det_real(S, m, hn, pn, sc, tph, o, L, ra, real_base(ra, r));
+  rmc_finish(S, a, m, r, t, idir, ndelta, idelta, o, L, status, pn, hn, sc, tph);
 }
 
 // The path estimators of path_props (reptation.f:1578-1737) of reptile r's
@@ -970,7 +1005,7 @@ extern "C" int qmc2d_rmc_init(qmc2d_handle *h, int nrep, const qmc2d_rmc_params 
   return q2d_sync_status(h, nrep);
 }
 
-template <int G, int LG>
+template <int G, int LG, bool kJ>
 static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *ds,
                                       const q2d::RmcArgs &a, double *scr, int idelta,
                                       cudaStream_t st) {
@@ -982,7 +1017,7 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *
   if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
       cudaSuccess)
     return e;
-  const void *k = (const void *)q2d::rmc_pairs_kernel<double, G, LG>;
+  const void *k = (const void *)q2d::rmc_pairs_kernel<double, G, LG, kJ>;
   const size_t carve =
       G * ((q2d::pair_carve(hs, nullptr, nullptr, q2d::kThreads) + 127) & ~size_t(127));
   const size_t rows = sizeof(double) * q2d::RowLayout<double>::sstride * (size_t)hs.cmb_nblk *
@@ -996,21 +1031,31 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *
                                                                    sm)) != cudaSuccess)
     return e;
   const int need = (a.nrep + G - 1) / G, cap = nsm * (per_sm > 0 ? per_sm : 1);
-  q2d::rmc_pairs_kernel<double, G, LG>
+  q2d::rmc_pairs_kernel<double, G, LG, kJ>
       <<<need < cap ? need : cap, G * q2d::kThreads, sm, st>>>(ds, a, scr, idelta, stage);
   return cudaGetLastError();
 }
 
 // the lanes per particle in force (DevSys::tune_lanes, as the DMC pair kernel)
-template <int G>
-static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs, const q2d::DevSys *ds,
+template <int G, bool kJ>
+static cudaError_t launch_rmc_pairs_g(const q2d::DevSys &hs, const q2d::DevSys *ds,
                                     const q2d::RmcArgs &a, double *scr, int idelta,
                                     cudaStream_t st) {
   switch (hs.tune_lanes) {
-    case 4: return launch_rmc_pairs_t<G, 4>(hs, ds, a, scr, idelta, st);
-    case 16: return launch_rmc_pairs_t<G, 16>(hs, ds, a, scr, idelta, st);
-    default: return launch_rmc_pairs_t<G, 8>(hs, ds, a, scr, idelta, st);
+    case 4: return launch_rmc_pairs_t<G, 4, kJ>(hs, ds, a, scr, idelta, st);
+    case 16: return launch_rmc_pairs_t<G, 16, kJ>(hs, ds, a, scr, idelta, st);
+    default: return launch_rmc_pairs_t<G, 8, kJ>(hs, ds, a, scr, idelta, st);
   }
+}
+
+static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs, const q2d::DevSys *ds,
+                                    const q2d::RmcArgs &a, double *scr, int idelta, bool real,
+                                    cudaStream_t st) {
+  if (hs.tune_groups == 1)
+    return real ? launch_rmc_pairs_g<1, true>(hs, ds, a, scr, idelta, st)
+                : launch_rmc_pairs_g<1, false>(hs, ds, a, scr, idelta, st);
+  return real ? launch_rmc_pairs_g<2, true>(hs, ds, a, scr, idelta, st)
+              : launch_rmc_pairs_g<2, false>(hs, ds, a, scr, idelta, st);
 }
 
 extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
@@ -1039,15 +1084,31 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
     // per move and bead growth: the pair passes, then the rest
     const void *kd = h->hs.gmat ? (const void *)q2d::rmc_det_kernel<true>
                                 : (const void *)q2d::rmc_det_kernel<false>;
-    RCK(q2d::raise_smem_limit(kd, sm));
+    // real orbitals as VMC and DMC moves take them
+    const bool real = move_real(h);
+    const size_t smr = q2d::real_carve(h->hs, nullptr, nullptr) +
+                       sizeof(double) * (5 * (size_t)h->hs.nprops + 16);
+    if (real)
+      RCK(q2d::raise_smem_limit((const void *)q2d::rmc_real_kernel, smr));
+    else
+      RCK(q2d::raise_smem_limit(kd, sm));
     for (int istp = 0; istp < nstp; istp++) {
       a.step0 = h->rmc.step + (uint32_t)istp;
       for (int idelta = 1; idelta <= h->rmc.mdelta; idelta++) {
         {
           ProfScope ps(h, QMC2D_KERNEL_PAIRS, h->stream);
-          RCK(h->hs.tune_groups == 1
-                  ? launch_rmc_pairs<1>(h->hs, h->ds, a, h->d_mscr, idelta, h->stream)
-                  : launch_rmc_pairs<2>(h->hs, h->ds, a, h->d_mscr, idelta, h->stream));
+          RCK(launch_rmc_pairs(h->hs, h->ds, a, h->d_mscr, idelta, real, h->stream));
+        }
+        if (real) {
+          {
+            ProfScope ps(h, QMC2D_KERNEL_ORB_INV, h->stream);
+            RCK(q2d::launch_real_det(h->hs, h->ds, h->rmc.nrep, h->d_mscr, h->stream));
+          }
+          ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
+          q2d::rmc_real_kernel<<<h->rmc.nrep, q2d::kThreads, smr, h->stream>>>(
+              h->ds, a, q2d::real_args(h->hs, h->d_mscr), q2d::move_scratch(h->hs), idelta);
+          RCK(cudaGetLastError());
+          continue;
         }
         ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
         if (h->hs.gmat)

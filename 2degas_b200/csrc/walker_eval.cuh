@@ -322,7 +322,7 @@ __host__ __device__ inline RealLayout real_layout(const DevSys &s) {
 // with_inv: the layout of VMC/DMC moves, which may batch their inversion;
 // reptation's kernels never do and lay their blocks out without that region
 // (the same allocation holds them, closer together). The real-orbital region
-// (RealLayout) takes the place of both from l.pair on.
+// (RealLayout, in reptation too) takes the place of both from l.pair on.
 __host__ __device__ inline MoveScratch move_scratch(const DevSys &s, bool with_inv = true) {
   const int N = s.N;
   MoveScratch l;
@@ -346,7 +346,7 @@ __host__ __device__ inline MoveScratch move_scratch(const DevSys &s, bool with_i
     l.inv = end;
     for (int sp = 0; sp < s.nt; sp++) end += inv_spin_doubles(s.np[sp]);
   }
-  if (s.real_room && !s.gmat) {
+  if (with_inv && s.real_room && !s.gmat) {
     const size_t re = (size_t)l.pair + real_layout(s).end;
     end = re > end ? re : end;
   }
