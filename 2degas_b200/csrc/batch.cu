@@ -100,7 +100,7 @@ cudaError_t enqueue(qmc2d_batch *b, int k, int g0, int ngen, int dmc, double del
     a.cnt = h->d_cnt;
     a.wate = dmc ? h->d_wate : nullptr;
     a.status = h->d_status;
-    a.real = move_real(h) ? 1 : 0;
+    a.real = move_real(h, h->nw) ? 1 : 0;
     a.orb_inv = !a.real && move_orb_inv(h) ? 1 : 0;
     a.ctr = ctr;
     if ((e = q2d::launch_pairs(h->hs, h->ds, h->pop[cur], a, st)) != cudaSuccess) return e;
@@ -215,7 +215,10 @@ int run(qmc2d_batch *b, int n, int dmc, const double *delta, const double *etria
       key.push_back((double)b->h[k]->cur);
       key.push_back((double)(intptr_t)b->h[k]);
       key.push_back(b->h[k]->dmc_ecut);
-      key.push_back(move_real(b->h[k]) ? 1.0 : 0.0);  // a twist may have changed it
+      key.push_back(move_real(b->h[k], b->h[k]->nw) ? 1.0 : 0.0);  // a twist may have changed it
+      // kernels take the system by value: the timers' buffer and the precision
+      key.push_back((double)(intptr_t)b->h[k]->hs.phase);
+      key.push_back((double)b->h[k]->hs.pair_f32);
     }
     if (!b->exec || key != b->key) {
       if (b->exec) {

@@ -510,7 +510,7 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   CK(join_side(h));
   q2d::MoveArgs a{};
   a.nw = h->nw;
-  a.real = move_real(h) ? 1 : 0;
+  a.real = move_real(h, h->nw) ? 1 : 0;
   a.scr = h->d_mscr;
   a.delta = h->hs.delta > 0.0 ? h->hs.delta : 0.01;
   a.seed = h->seed;
@@ -952,7 +952,7 @@ static int run_moves(qmc2d_handle *h, int nstp, int dmc, double delta, double et
   a.cnt = h->d_cnt;
   a.wate = dmc ? h->d_wate : nullptr;
   a.status = h->d_status;
-  a.real = move_real(h) ? 1 : 0;
+  a.real = move_real(h, h->nw) ? 1 : 0;
   a.orb_inv = !a.real && move_orb_inv(h) ? 1 : 0;
   if (h->hs.delta != delta && h->hs.adrift != 0.0) {
     h->hs.delta = delta;

@@ -69,9 +69,6 @@ struct qmc2d_handle {
 // of the CTA, gains 4% at 3.5 and 21% at 7.
 constexpr int kOrbInvMinPerSM = 10, kOrbInvMinPerSMSmall = 10, kOrbInvMinPerSMOneSpin = 3;
 
-// Spin matrices from which an evaluation takes the real-orbital kernels.
-constexpr long kEvalRealMin = 0;
-
 // Whether this handle's next move batches its orbitals and inversion.
 inline bool move_orb_inv(const qmc2d_handle *h) {
   if (h->move_inv_mode == 0) return false;
@@ -82,11 +79,24 @@ inline bool move_orb_inv(const qmc2d_handle *h) {
   return q2d::orb_inv_pays(h->hs, h->nw, h->nsm, need);
 }
 
-// Whether this handle's moves take the real-orbital route (real_det.cuh): at
-// every population size it is the faster one; an inversion layout or a move
-// inversion mode chosen by the caller keeps the complex kernels.
-inline bool move_real(const qmc2d_handle *h) {
-  return h->hs.real_orb && h->hs.tune_inv == 0 && h->move_inv_mode == 1;
+// Small work for which the fused or complex kernels, with fewer launches, are
+// the faster ones: at most `walkers` configurations of small spins. Measured
+// against them: evaluations of 13 + 13 lose 12% at 64 configurations, 5% at
+// 256 and gain 22% at 512 (25 polarised: -13%, -10%, +32%; 21 + 21: +7%, +41%,
+// +42%).
+inline bool small_work(const qmc2d_handle *h, int nw, int walkers) {
+  return nw <= walkers && h->hs.nmax <= (h->hs.nt == 1 ? 29 : 16);
+}
+
+// Whether this handle's moves (nw walkers or reptiles) take the real-orbital
+// route (real_det.cuh); an inversion layout or a move inversion mode chosen
+// by the caller keeps the complex kernels, and so do up to 128 walkers of one
+// small spin, whose in-kernel inversion spreads one matrix over eight warps
+// (25 polarised: real orbitals lose 4% at 64 walkers, gain 6% at 256; 13 + 13
+// gain 12% at 64).
+inline bool move_real(const qmc2d_handle *h, int nw) {
+  return h->hs.real_orb && h->hs.tune_inv == 0 && h->move_inv_mode == 1 &&
+         !(h->hs.nt == 1 && small_work(h, nw, 128));
 }
 
 // Whether an evaluation of nw configurations on the handle's own stream runs
@@ -94,7 +104,7 @@ inline bool move_real(const qmc2d_handle *h) {
 // of the fused kernel. Evaluations on a caller's stream stay fused: they may
 // overlap the handle's moves, whose scratch this is.
 inline bool eval_real(const qmc2d_handle *h, int nw) {
-  return h->hs.real_orb && h->hs.tune_inv == 0 && (long)nw * h->hs.nt >= kEvalRealMin;
+  return h->hs.real_orb && h->hs.tune_inv == 0 && !small_work(h, nw, 2 * h->nsm);
 }
 
 // Orders the handle's stream after the side copies of the last

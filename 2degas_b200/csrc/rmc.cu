@@ -527,14 +527,10 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_move_kernel(const DevSys *sp,
 // of mdelta > 1 takes mdelta launch pairs; a reptile whose move has fewer
 // growths skips the later ones.
 template <class R, int G, int LG, bool kJ>
-__global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(const DevSys *sp,
-                                                                        RmcArgs a, double *scr,
-                                                                        int idelta,
-                                                                        int stage_rows) {
+__global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
+    const __grid_constant__ DevSys S, RmcArgs a, double *scr, int idelta, int stage_rows) {
   constexpr int kPairThreads = G * kThreads;
-  __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
   const size_t carve = (pair_carve(S, nullptr, nullptr, kThreads) + 127) & ~size_t(127);
   const int grp = threadIdx.x / kThreads, tid = threadIdx.x - grp * kThreads;
   EvalSmem m;
@@ -714,12 +710,9 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_det_kernel(const DevSys *sp, 
 }
 
 // The same with real orbitals, after launch_real_det.
-__global__ void __launch_bounds__(kThreads, 3) rmc_real_kernel(const DevSys *sp, RmcArgs a,
-                                                              RealArgs ra, MoveScratch L,
-                                                              int idelta) {
-  __shared__ DevSys S;
+__global__ void __launch_bounds__(kThreads, 3) rmc_real_kernel(
+    const __grid_constant__ DevSys S, RmcArgs a, RealArgs ra, MoveScratch L, int idelta) {
   extern __shared__ __align__(16) char smem[];
-  load_sys(S, sp);
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   double *pn = reinterpret_cast<double *>(smem + off);
@@ -1032,7 +1025,7 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *
     return e;
   const int need = (a.nrep + G - 1) / G, cap = nsm * (per_sm > 0 ? per_sm : 1);
   q2d::rmc_pairs_kernel<double, G, LG, kJ>
-      <<<need < cap ? need : cap, G * q2d::kThreads, sm, st>>>(ds, a, scr, idelta, stage);
+      <<<need < cap ? need : cap, G * q2d::kThreads, sm, st>>>(hs, a, scr, idelta, stage);
   return cudaGetLastError();
 }
 
@@ -1085,7 +1078,7 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
     const void *kd = h->hs.gmat ? (const void *)q2d::rmc_det_kernel<true>
                                 : (const void *)q2d::rmc_det_kernel<false>;
     // real orbitals as VMC and DMC moves take them
-    const bool real = move_real(h);
+    const bool real = move_real(h, h->rmc.nrep);
     const size_t smr = q2d::real_carve(h->hs, nullptr, nullptr) +
                        sizeof(double) * (5 * (size_t)h->hs.nprops + 16);
     if (real)
@@ -1106,7 +1099,7 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
           }
           ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
           q2d::rmc_real_kernel<<<h->rmc.nrep, q2d::kThreads, smr, h->stream>>>(
-              h->ds, a, q2d::real_args(h->hs, h->d_mscr), q2d::move_scratch(h->hs), idelta);
+              h->hs, a, q2d::real_args(h->hs, h->d_mscr), q2d::move_scratch(h->hs), idelta);
           RCK(cudaGetLastError());
           continue;
         }

@@ -22,10 +22,11 @@ SHELLS = [(1, 1), (3, 1), (5, 5), (9, 0), (15, 13), (17, 17), (31, 25), (31, 33)
 
 def _deck(q, tmp_path, nu, nd, **kw):
     tables = importlib.import_module("2degas_b200.tables")
-    kw = dict(dict(rs=3.0, backflow=(0.2, 3.0, 1.8), nconf=6, seed=11), **kw)
+    n = 130 if nd == 0 and nu <= 29 else 6  # small populations of one small spin stay complex
+    kw = dict(dict(rs=3.0, backflow=(0.2, 3.0, 1.8), nconf=n, seed=11), **kw)
     d = tables.make_run(os.path.join(tmp_path, "d"), "c", nu, nd, **kw)
     s = q.System.read(d, "c")
-    return s, s.read_configs(d, ".0", 0, 6)
+    return s, s.read_configs(d, ".0", 0, kw["nconf"])
 
 
 def _step(q, s, x, mode, precision="fp64"):
@@ -64,6 +65,45 @@ def test_mixed_precision_step(q, tmp_path):
     (r, _), (c, _) = _step(q, s, x, 1, "mixed"), _step(q, s, x, 0, "mixed")
     for k in ("g", "h", "p"):
         assert _same(r[k], c[k], 1e-9), k
+
+
+@pytest.mark.parametrize("nu,nd", [(13, 13), (25, 0), (37, 33), (61, 61)])
+def test_evaluation_equals_the_fused_kernel(q, tmp_path, nu, nd):
+    """Evaluations on the handle's stream (through the move's kernels where the
+    configurations are enough) and on a caller's (always the fused kernel)."""
+    import torch
+
+    n = 320 if nu < 30 else 5
+    s, x = _deck(q, tmp_path, nu, nd, nconf=n)
+    st = torch.cuda.Stream()
+    with q.Handle(s, capacity=n, seed=1) as h:
+        a = h.compute_properties(x)
+        with torch.cuda.stream(st):
+            xd = torch.from_numpy(x).cuda()
+            o = [torch.zeros(n, k, dtype=torch.float64, device="cuda")
+                 for k in (2 * s.N, s.ntypes, s.nprops, 1)]
+        h.compute_properties_dev(n, xd.data_ptr(), *(t.data_ptr() for t in o),
+                                 stream=st.cuda_stream)
+        h.compute_properties_dev_status(n, st.cuda_stream)
+    for u, v in zip(a, o):
+        assert _same(u.reshape(n, -1), v.cpu().numpy(), 1e-9)
+
+
+def test_reptation_equals_the_complex_route(q, tmp_path):
+    s, x = _deck(q, tmp_path, 37, 29, u3=True)
+    rng = np.random.default_rng(3)
+    walk = np.cumsum(rng.normal(0.0, 0.02, size=(6, 12, x.shape[1])), axis=1)
+    paths = (x[:, None, :] + walk).reshape(72, -1)
+    out = []
+    for mode in (1, 0):
+        with q.Handle(s, capacity=6, seed=9) as h:
+            h.set_move_inversion(mode)
+            h.rmc_init(6, paths, 12, 1, 2, 0.002, -0.4, 10 ** 9, 0)  # every move forced
+            h.block_reset()
+            h.rmc(2)
+            out.append((h.block_get()[0],) + h.rmc_get_path(5, 12))
+    for u, v in zip(*out):
+        assert _same(u, v, 1e-9)
 
 
 def test_a_twist_and_gamma_again(q, tmp_path):
