@@ -615,8 +615,10 @@ size_t eval_real_smem_bytes(const DevSys &s) {
 
 // The rest of a move after launch_real_det: the assembly, the reverse move,
 // Metropolis, the averages. Latency-bound (reductions, transcendentals, the
-// records' reads and writes); four CTAs per SM overlap it.
-__global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_constant__ DevSys S, DevPop pop,
+// records' reads and writes) and by instructions every thread repeats (the
+// scalar end of the assembly): 128 threads, eight CTAs per SM.
+constexpr int kEndThreads = 128;
+__global__ void __launch_bounds__(kEndThreads, 8) move_real_kernel(const __grid_constant__ DevSys S, DevPop pop,
                                                                 MoveArgs a, RealArgs ra,
                                                                 MoveScratch L) {
   extern __shared__ __align__(16) char smem[];
@@ -628,8 +630,8 @@ __global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_con
   if (w >= a.nw) return;
   const int N2 = 2 * S.N, np = S.nprops, nt = S.nt;
   const double *o = a.scr + (size_t)w * L.stride;
-  load_real_sums(S, m, o, L);
-  for (int j = tid; j < N2; j += kThreads) {
+  load_real_sums<kEndThreads>(S, m, o, L);
+  for (int j = tid; j < N2; j += kEndThreads) {
     cp_async8(v.xo + j, pop.x + (size_t)w * N2 + j);
     cp_async8(v.go + j, pop.g + (size_t)w * N2 + j);
   }
@@ -639,21 +641,21 @@ __global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_con
   const double age0 = pop.age[w];
   double wate = (a.dmc && !a.first) ? a.wate[w] : 1.0;
   long long tph = clock64();
-  const int status = eval_det_real(S, m, v.hn, v.pn, &v.sc[0], tph, o, L, ra,
+  const int status = eval_det_real<kEndThreads>(S, m, v.hn, v.pn, &v.sc[0], tph, o, L, ra,
                                    real_base(ra, w));
   // reverse move (reptation.f:4660-4674)
-  double wn = 0.0;
-  for (int j = tid; j < N2; j += kThreads) {
+  double wn[1] = {0.0};
+  for (int j = tid; j < N2; j += kEndThreads) {
     int ti = type_of(S, j >> 1);
     double var = 2.0 * S.hbs2m[ti] * a.delta, vari = 1.0 / var;
     double chi = v.xo[j] - m.x[j] - (-var * m.g[j]);
-    wn -= chi * chi * vari;
+    wn[0] -= chi * chi * vari;
   }
-  const double wnew = block_sum(wn, m.red);
+  block_sum_n<1, kEndThreads>(wn, m.red);
   const bool forced = age0 == a.mage;
   double p = 1.0;
   if (!forced) {
-    p = (po_ltf - v.pn[QMC2D_JLTF]) * 2.0 + 0.5 * (wnew - wold);
+    p = (po_ltf - v.pn[QMC2D_JLTF]) * 2.0 + 0.5 * (wn[0] - wold);
     p = exp(fmin(0.0, fmax(-50.0, p)));
   }
   // metropolis_test (reptation.f:2622-2659)
@@ -673,13 +675,13 @@ __global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_con
   }
   phase_mark(S, PH_ACCEPT, tph);
   if (acc)
-    for (int j = tid; j < N2; j += kThreads) {
+    for (int j = tid; j < N2; j += kEndThreads) {
       pop.x[(size_t)w * N2 + j] = m.x[j];
       pop.g[(size_t)w * N2 + j] = m.g[j];
     }
   // the walker's properties, the new ones if accepted, with the acceptance
   // probability; the block sums
-  for (int j = tid; j < np; j += kThreads) {
+  for (int j = tid; j < np; j += kEndThreads) {
     const size_t i = (size_t)w * np + j;
     double val = acc ? v.pn[j] : pop.p[i];
     if (j == QMC2D_JACC) val = p;
@@ -700,7 +702,7 @@ __global__ void __launch_bounds__(kThreads, 4) move_real_kernel(const __grid_con
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 4) eval_real_kernel(const __grid_constant__ DevSys S, int nw,
+__global__ void __launch_bounds__(kEndThreads, 8) eval_real_kernel(const __grid_constant__ DevSys S, int nw,
                                                                 RealArgs ra, MoveScratch L,
                                                                 double *g, double *hl,
                                                                 double *props, double *s,
@@ -713,11 +715,11 @@ __global__ void __launch_bounds__(kThreads, 4) eval_real_kernel(const __grid_con
   const int w = blockIdx.x;
   if (w >= nw) return;
   const double *o = ra.scr + (size_t)w * L.stride;
-  load_real_sums(S, m, o, L);
+  load_real_sums<kEndThreads>(S, m, o, L);
   long long tph = clock64();
-  const int st = eval_det_real(S, m, hn, pn, sn, tph, o, L, ra, real_base(ra, w));
-  for (int j = threadIdx.x; j < 2 * S.N; j += kThreads) g[(size_t)w * 2 * S.N + j] = m.g[j];
-  for (int j = threadIdx.x; j < S.nprops; j += kThreads) props[(size_t)w * S.nprops + j] = pn[j];
+  const int st = eval_det_real<kEndThreads>(S, m, hn, pn, sn, tph, o, L, ra, real_base(ra, w));
+  for (int j = threadIdx.x; j < 2 * S.N; j += kEndThreads) g[(size_t)w * 2 * S.N + j] = m.g[j];
+  for (int j = threadIdx.x; j < S.nprops; j += kEndThreads) props[(size_t)w * S.nprops + j] = pn[j];
   if (threadIdx.x < S.nt) hl[(size_t)w * S.nt + threadIdx.x] = hn[threadIdx.x];
   if (threadIdx.x == 0) {
     s[w] = *sn;
@@ -968,17 +970,62 @@ cudaError_t launch_eval(const DevSys &hs, const DevSys *ds, int nw, const double
   return cudaGetLastError();
 }
 
+// Shared memory of the pair kernels: per group, and for the staged rows.
+static size_t pair_group_bytes(const DevSys &hs) {
+  return (pair_carve(hs, nullptr, nullptr, kThreads) + 127) & ~size_t(127);
+}
+static size_t pair_rows_bytes(const DevSys &hs) {
+  const size_t row = hs.pair_f32 ? sizeof(float) * RowLayout<float>::sstride
+                                 : sizeof(double) * RowLayout<double>::sstride;
+  return row * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
+}
+
+// Groups, staging and lanes compute the same pair terms; groups and staging
+// leave every bit, the lanes the order of a particle's partial sums.
+//   groups and staging (FP64, us per launch, 148 SMs): one group per CTA
+//   when two and the rows do not fit a CTA's shared memory (N = 122, 1024
+//   walkers: 321 against 344; N = 161, 148: 95 against 173) and when every SM
+//   has at most one walker (N = 58, 148: 25 against 29); rows of small
+//   systems stay in global memory up to seven walkers per SM, where copying
+//   them costs more than it saves (N = 26: 17.0 against 19.4 at 64 walkers, 29.5
+//   against 31.4 at 512, equal at 1024); else two groups with staged rows
+//   (N = 58, 4096: 312 against 355).
+//   lanes: the fewest sweeps, ceil(N / particles per round) rounds of
+//   ceil(N / lanes) partners and the round's reductions (N = 58: four lanes 273,
+//   eight 312; N = 122: 344 against 360; N = 74: eight 209, four 230). Eight in
+//   mixed precision, whose FP32 sums follow the order.
+PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin) {
+  PairLaunch p{hs.tune_groups, hs.tune_stage != 1, hs.tune_lanes};
+  const size_t grp = pair_group_bytes(hs), rows = pair_rows_bytes(hs), lim = (size_t)optin - 1024;
+  if (p.groups == 0) {
+    if (2 * grp + rows > lim || nw <= nsm) {
+      p.groups = 1;
+      if (hs.N <= 32) p.stage = 0;
+    } else if (hs.N <= 32 && nw < 7 * nsm) {
+      p.groups = 1;
+      p.stage = 0;
+    } else {
+      p.groups = 2;
+    }
+  }
+  if (p.groups * grp + rows > lim) p.stage = 0;
+  if (p.lanes == 0) {
+    p.lanes = 8;
+    if (!hs.pair_f32) {
+      const int per4 = kThreads / 4, per8 = kThreads / 8;
+      const double c4 = (hs.N + per4 - 1) / per4 * ((hs.N + 3) / 4 + 1.4);
+      const double c8 = (hs.N + per8 - 1) / per8 * ((hs.N + 7) / 8 + 2.1);
+      if (c4 < c8) p.lanes = 4;
+    }
+  }
+  return p;
+}
+
 template <class R, int G, int LG, bool kJ>
-static cudaError_t launch_pairs_t(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
-                                  const double *xe) {
+static cudaError_t launch_pairs_t(const DevSys &hs, DevPop pop, const MoveArgs &a,
+                                  cudaStream_t st, int nsm, int stage, const double *xe) {
   const void *k = (const void *)pairs_kernel<R, G, LG, kJ>;
-  const size_t carve = G * ((pair_carve(hs, nullptr, nullptr, kThreads) + 127) & ~size_t(127));
-  const size_t rows =
-      sizeof(R) * RowLayout<R>::sstride * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
-  const int stage =
-      hs.tune_stage != 1 && carve + rows + sizeof(DevSys) <= (size_t)optin ? 1 : 0;
-  const size_t sm = carve + (stage ? rows : 0);
+  const size_t sm = G * pair_group_bytes(hs) + (stage ? pair_rows_bytes(hs) : 0);
   cudaError_t e;
   if ((e = set_smem(k, sm)) != cudaSuccess) return e;
   int per_sm = 1;
@@ -994,26 +1041,26 @@ static cudaError_t launch_pairs_t(const DevSys &hs, const DevSys *ds, DevPop pop
 }
 
 template <class R, int LG, bool kJ>
-static cudaError_t launch_pairs_g(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
+static cudaError_t launch_pairs_g(const DevSys &hs, DevPop pop, const MoveArgs &a,
+                                  cudaStream_t st, int nsm, const PairLaunch &p,
                                   const double *xe) {
-  return hs.tune_groups == 1 ? launch_pairs_t<R, 1, LG, kJ>(hs, ds, pop, a, st, nsm, optin, xe)
-                             : launch_pairs_t<R, 2, LG, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
+  return p.groups == 1 ? launch_pairs_t<R, 1, LG, kJ>(hs, pop, a, st, nsm, p.stage, xe)
+                       : launch_pairs_t<R, 2, LG, kJ>(hs, pop, a, st, nsm, p.stage, xe);
 }
 
 template <class R, bool kJ>
-static cudaError_t launch_pairs_r(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, int nsm, int optin,
-                                  const double *xe) {
-  switch (hs.tune_lanes) {
-    case 4: return launch_pairs_g<R, 4, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
-    case 16: return launch_pairs_g<R, 16, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
-    default: return launch_pairs_g<R, 8, kJ>(hs, ds, pop, a, st, nsm, optin, xe);
+static cudaError_t launch_pairs_r(const DevSys &hs, DevPop pop, const MoveArgs &a,
+                                  cudaStream_t st, int nsm, int optin, const double *xe) {
+  const PairLaunch p = pair_launch(hs, a.nw, nsm, optin);
+  switch (p.lanes) {
+    case 4: return launch_pairs_g<R, 4, kJ>(hs, pop, a, st, nsm, p, xe);
+    case 16: return launch_pairs_g<R, 16, kJ>(hs, pop, a, st, nsm, p, xe);
+    default: return launch_pairs_g<R, 8, kJ>(hs, pop, a, st, nsm, p, xe);
   }
 }
 
-static cudaError_t launch_pairs_x(const DevSys &hs, const DevSys *ds, DevPop pop,
-                                  const MoveArgs &a, cudaStream_t st, const double *xe) {
+static cudaError_t launch_pairs_x(const DevSys &hs, DevPop pop, const MoveArgs &a,
+                                  cudaStream_t st, const double *xe) {
   if (a.nw <= 0) return cudaSuccess;
   int dev = 0, nsm = 0, optin = 0;
   cudaError_t e;
@@ -1024,15 +1071,16 @@ static cudaError_t launch_pairs_x(const DevSys &hs, const DevSys *ds, DevPop pop
       cudaSuccess)
     return e;
   if (a.real)
-    return hs.pair_f32 ? launch_pairs_r<float, true>(hs, ds, pop, a, st, nsm, optin, xe)
-                       : launch_pairs_r<double, true>(hs, ds, pop, a, st, nsm, optin, xe);
-  return hs.pair_f32 ? launch_pairs_r<float, false>(hs, ds, pop, a, st, nsm, optin, nullptr)
-                     : launch_pairs_r<double, false>(hs, ds, pop, a, st, nsm, optin, nullptr);
+    return hs.pair_f32 ? launch_pairs_r<float, true>(hs, pop, a, st, nsm, optin, xe)
+                       : launch_pairs_r<double, true>(hs, pop, a, st, nsm, optin, xe);
+  return hs.pair_f32 ? launch_pairs_r<float, false>(hs, pop, a, st, nsm, optin, nullptr)
+                     : launch_pairs_r<double, false>(hs, pop, a, st, nsm, optin, nullptr);
 }
 
 cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
                          cudaStream_t st) {
-  return launch_pairs_x(hs, ds, pop, a, st, nullptr);
+  (void)ds;
+  return launch_pairs_x(hs, pop, a, st, nullptr);
 }
 
 cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const double *x,
@@ -1044,11 +1092,11 @@ cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const d
   a.real = 1;
   a.scr = scr;
   cudaError_t e;
-  if ((e = launch_pairs_x(hs, ds, DevPop{}, a, st, x)) != cudaSuccess) return e;
+  if ((e = launch_pairs_x(hs, DevPop{}, a, st, x)) != cudaSuccess) return e;
   if ((e = launch_real_det(hs, ds, nw, scr, st)) != cudaSuccess) return e;
   const size_t sm = eval_real_smem_bytes(hs);
   if ((e = set_smem((const void *)eval_real_kernel, sm)) != cudaSuccess) return e;
-  eval_real_kernel<<<nw, kThreads, sm, st>>>(hs, nw, real_args(hs, scr), move_scratch(hs), g, hl,
+  eval_real_kernel<<<nw, kEndThreads, sm, st>>>(hs, nw, real_args(hs, scr), move_scratch(hs), g, hl,
                                              props, s, status);
   return cudaGetLastError();
 }
@@ -1088,7 +1136,7 @@ cudaError_t launch_move(const DevSys &hs, const DevSys *ds, DevPop pop, const Mo
     const size_t sm = move_real_smem_bytes(hs);
     cudaError_t e = set_smem((const void *)move_real_kernel, sm);
     if (e != cudaSuccess) return e;
-    move_real_kernel<<<a.nw, kThreads, sm, st>>>(hs, pop, a, real_args(hs, a.scr),
+    move_real_kernel<<<a.nw, kEndThreads, sm, st>>>(hs, pop, a, real_args(hs, a.scr),
                                                  move_scratch(hs));
     return cudaGetLastError();
   }

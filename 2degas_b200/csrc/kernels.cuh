@@ -34,6 +34,12 @@ struct MoveArgs {
   const uint32_t *ctr;
 };
 
+// The pair kernels' launch when the caller has not chosen one (DevSys::tune_*).
+struct PairLaunch {
+  int groups, stage, lanes;
+};
+PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin);
+
 // Raise (never lower) kernel fn's dynamic shared-memory limit on the current
 // device to bytes; safe to call from several host threads.
 cudaError_t raise_smem_limit(const void *fn, size_t bytes);

@@ -928,13 +928,13 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   mark(PH_CROSS);
 }
 
-// Warps per CTA of the resident form: a multiple of four, so that the four
-// sub-partitions' FP64 pipes get equal shares (five warps at 29 orbitals: the
-// first sub-partition two fifths of the products), about 20 on an SM with the
-// CTAs that its shared memory holds.
-int s_warps(size_t smem) {
+// Warps per CTA of the resident form, by the CTAs an SM's shared memory holds
+// (us with the orbital kernel, one B200: 13 + 13, 4096 walkers: 3 warps 109, 4
+// 117; 29 + 29: 4 443, 5 421, 6 413, 8 441; 37 + 37, 1001: 6 253, 8 244, 12 264;
+// 45 + 45, 1024: 8 374, 10 364, 12 384; 61 + 61: 12 768, 16 780, 20 749).
+int s_warps(int n, size_t smem) {
   const int ctas = 227 * 1024 / (int)(smem + 1024);
-  return ctas >= 4 ? 4 : ctas == 3 ? 8 : ctas == 2 ? 12 : 16;
+  return ctas >= 8 ? 3 : ctas >= 5 ? 4 : ctas == 4 ? 6 : ctas == 3 || n <= 40 ? 8 : ctas == 2 ? 10 : 20;
 }
 
 cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int nw,
@@ -951,7 +951,7 @@ cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int 
   cudaError_t e = raise_smem_limit(k, sm);
   if (e != cudaSuccess) return e;
   if (resident)
-    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(sm), sm, st>>>(a, ds, nw);
+    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st>>>(a, ds, nw);
   else
     real_s_kernel<2><<<nw * hs.nt, 512, sm, st>>>(a, ds, nw);
   return cudaGetLastError();

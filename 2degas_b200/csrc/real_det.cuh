@@ -109,14 +109,15 @@ cudaError_t launch_real_det(const DevSys &hs, const DevSys *ds, int nw, double *
 
 // The pair passes' sums of walker w into shared memory, the determinant sums
 // zeroed (asynchronous 8-byte copies; the caller waits).
+template <int NT>
 __device__ __forceinline__ void load_real_sums(const DevSys &S, const EvalSmem &m,
                                                const double *o, const MoveScratch &L) {
   const int N = S.N, tid = threadIdx.x;
-  for (int j = tid; j < 2 * N; j += kThreads) {
+  for (int j = tid; j < 2 * N; j += NT) {
     cp_async8(m.x + j, o + L.x + j);
     cp_async8(m.g + j, o + L.g + j);
   }
-  for (int j = tid; j < N; j += kThreads) {
+  for (int j = tid; j < N; j += NT) {
     cp_async8(m.lap + j, o + L.lap + j);
     cp_async8(m.ltf + j, o + L.ltf + j);
     cp_async8(m.vp + j, o + L.vp + j);
@@ -130,12 +131,13 @@ __device__ __forceinline__ void load_real_sums(const DevSys &S, const EvalSmem &
 // lap, ltf, vp of the pair passes (their asynchronous copies may be in
 // flight) and zeroed lapd, ph2, ph2d; o is the walker's scratch block, base its
 // real region.
+template <int NT>
 __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *hl, double *props,
                                     double *sign, long long &tph, const double *o,
                                     const MoveScratch &L, const RealArgs &R,
                                     const double *base) {
   const int tid = threadIdx.x, N = S.N, nt = S.nt;
-  for (int e = tid; e < 4 * S.nk; e += kThreads) cp_async8(m.rhok + e, o + L.rhok + e);
+  for (int e = tid; e < 4 * S.nk; e += NT) cp_async8(m.rhok + e, o + L.rhok + e);
   int status = ST_OK;
   double logdet_sum = 0.0, l0 = 0.0, l1 = 0.0;
   if (S.bf_zero) {
@@ -147,21 +149,21 @@ __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *
       if (t >= nt) continue;
       const int n = S.np[t];
       const double *FX = base + R.f[t], *FY = FX + n * n;
-      for (int j = tid; j < 2 * n; j += kThreads)
+      for (int j = tid; j < 2 * n; j += NT)
         m.gd[2 * S.ipfrst[t] + j] = -__ldg((j & 1 ? FY : FX) + (j >> 1) * (n + 1));
-      for (int e = tid; e < n * n; e += kThreads) {
+      for (int e = tid; e < n * n; e += NT) {
         const int j = e / n, k = e - j * n;
         if (k > j)
           s[t] -= 2.0 * (__ldg(FX + k + j * n) * __ldg(FX + j + k * n) +
                          __ldg(FY + k + j * n) * __ldg(FY + j + k * n));
       }
     }
-    block_sum_n<2>(s, m.red);
+    block_sum_n<2, NT>(s, m.red);
     l0 = s[0];
     l1 = s[1];
   } else {
     // the determinants' drift: every spin's share
-    for (int j = tid; j < 2 * N; j += kThreads) {
+    for (int j = tid; j < 2 * N; j += NT) {
       double g = __ldg(base + R.s[0] + j);
       if (nt > 1) g += __ldg(base + R.s[1] + j);
       m.gd[j] = g;
@@ -183,11 +185,11 @@ __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *
   // the assembly sums lapd per type
   if (tid == 0) m.lapd[0] = l0;
   if (tid == 1 && nt > 1) m.lapd[S.ipfrst[1]] = l1;
-  double ltf_j = 0.0;
-  for (int j = tid; j < N; j += kThreads) ltf_j += m.ltf[j];
-  ltf_j = block_sum(ltf_j, m.red);  // its barriers cover lapd too
+  double ltf_j[1] = {0.0};
+  for (int j = tid; j < N; j += NT) ltf_j[0] += m.ltf[j];
+  block_sum_n<1, NT>(ltf_j, m.red);  // its barriers cover lapd too
   phase_mark(S, PH_ORBITALS, tph);
-  return eval_assemble(S, m, ltf_j, logdet_sum, status, hl, props, sign, tph);
+  return eval_assemble<NT>(S, m, ltf_j[0], logdet_sum, status, hl, props, sign, tph);
 }
 
 }  // namespace q2d

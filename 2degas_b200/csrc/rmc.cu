@@ -724,9 +724,9 @@ __global__ void __launch_bounds__(kThreads, 3) rmc_real_kernel(
   rmc_dir(a, r, t, idir, ndelta);
   if (idelta > ndelta) return;  // the whole CTA
   const double *o = ra.scr + (size_t)r * L.stride;
-  load_real_sums(S, m, o, L);
+  load_real_sums<kThreads>(S, m, o, L);
   long long tph = clock64();
-  const int status = eval_det_real(S, m, hn, pn, sc, tph, o, L, ra, real_base(ra, r));
+  const int status = eval_det_real<kThreads>(S, m, hn, pn, sc, tph, o, L, ra, real_base(ra, r));
   rmc_finish(S, a, m, r, t, idir, ndelta, idelta, o, L, status, pn, hn, sc, tph);
 }
 
@@ -999,24 +999,14 @@ extern "C" int qmc2d_rmc_init(qmc2d_handle *h, int nrep, const qmc2d_rmc_params 
 }
 
 template <int G, int LG, bool kJ>
-static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *ds,
-                                      const q2d::RmcArgs &a, double *scr, int idelta,
-                                      cudaStream_t st) {
-  int dev = 0, nsm = 0, optin = 0;
+static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::RmcArgs &a, double *scr,
+                                      int idelta, int nsm, int stage, cudaStream_t st) {
   cudaError_t e;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-    return e;
-  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
-      cudaSuccess)
-    return e;
   const void *k = (const void *)q2d::rmc_pairs_kernel<double, G, LG, kJ>;
   const size_t carve =
       G * ((q2d::pair_carve(hs, nullptr, nullptr, q2d::kThreads) + 127) & ~size_t(127));
   const size_t rows = sizeof(double) * q2d::RowLayout<double>::sstride * (size_t)hs.cmb_nblk *
                       (hs.cmb_ng + 1);
-  const int stage =
-      hs.tune_stage != 1 && carve + rows + sizeof(q2d::DevSys) <= (size_t)optin ? 1 : 0;
   const size_t sm = carve + (stage ? rows : 0);
   if ((e = q2d::raise_smem_limit(k, sm)) != cudaSuccess) return e;
   int per_sm = 1;
@@ -1029,26 +1019,36 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::DevSys *
   return cudaGetLastError();
 }
 
-// the lanes per particle in force (DevSys::tune_lanes, as the DMC pair kernel)
 template <int G, bool kJ>
-static cudaError_t launch_rmc_pairs_g(const q2d::DevSys &hs, const q2d::DevSys *ds,
-                                    const q2d::RmcArgs &a, double *scr, int idelta,
-                                    cudaStream_t st) {
-  switch (hs.tune_lanes) {
-    case 4: return launch_rmc_pairs_t<G, 4, kJ>(hs, ds, a, scr, idelta, st);
-    case 16: return launch_rmc_pairs_t<G, 16, kJ>(hs, ds, a, scr, idelta, st);
-    default: return launch_rmc_pairs_t<G, 8, kJ>(hs, ds, a, scr, idelta, st);
+static cudaError_t launch_rmc_pairs_g(const q2d::DevSys &hs, const q2d::RmcArgs &a, double *scr,
+                                      int idelta, int nsm, const q2d::PairLaunch &p,
+                                      cudaStream_t st) {
+  switch (p.lanes) {
+    case 4: return launch_rmc_pairs_t<G, 4, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
+    case 16: return launch_rmc_pairs_t<G, 16, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
+    default: return launch_rmc_pairs_t<G, 8, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
   }
 }
 
-static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs, const q2d::DevSys *ds,
-                                    const q2d::RmcArgs &a, double *scr, int idelta, bool real,
-                                    cudaStream_t st) {
-  if (hs.tune_groups == 1)
-    return real ? launch_rmc_pairs_g<1, true>(hs, ds, a, scr, idelta, st)
-                : launch_rmc_pairs_g<1, false>(hs, ds, a, scr, idelta, st);
-  return real ? launch_rmc_pairs_g<2, true>(hs, ds, a, scr, idelta, st)
-              : launch_rmc_pairs_g<2, false>(hs, ds, a, scr, idelta, st);
+// The launch of the DMC pair kernel (pair_launch); reptation's pair terms are FP64.
+static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs0, const q2d::RmcArgs &a, double *scr,
+                                    int idelta, bool real, cudaStream_t st) {
+  q2d::DevSys hs = hs0;
+  hs.pair_f32 = 0;
+  int dev = 0, nsm = 0, optin = 0;
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    return e;
+  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
+      cudaSuccess)
+    return e;
+  const q2d::PairLaunch p = q2d::pair_launch(hs, a.nrep, nsm, optin);
+  if (p.groups == 1)
+    return real ? launch_rmc_pairs_g<1, true>(hs, a, scr, idelta, nsm, p, st)
+                : launch_rmc_pairs_g<1, false>(hs, a, scr, idelta, nsm, p, st);
+  return real ? launch_rmc_pairs_g<2, true>(hs, a, scr, idelta, nsm, p, st)
+              : launch_rmc_pairs_g<2, false>(hs, a, scr, idelta, nsm, p, st);
 }
 
 extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
@@ -1090,7 +1090,7 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
       for (int idelta = 1; idelta <= h->rmc.mdelta; idelta++) {
         {
           ProfScope ps(h, QMC2D_KERNEL_PAIRS, h->stream);
-          RCK(launch_rmc_pairs(h->hs, h->ds, a, h->d_mscr, idelta, real, h->stream));
+          RCK(launch_rmc_pairs(h->hs, a, h->d_mscr, idelta, real, h->stream));
         }
         if (real) {
           {

@@ -424,6 +424,17 @@ __device__ __forceinline__ double spline0(const DevSys &S, const double *part, i
   return f;
 }
 
+// r and 1/r from r^2: one reciprocal square root (1 ulp, as a correctly
+// rounded root and its reciprocal are together) and a Newton correction of
+// r = r^2 / sqrt(r^2), in place of a square root and a division (about 45
+// FP64 instructions and their slow-path branches per pair).
+__device__ __forceinline__ void pair_dist(double r2, double &r, double &byr) {
+  byr = rsqrt(r2);
+  const double r0 = r2 * byr;
+  r = fma(0.5 * byr, fma(-r0, r0, r2), r0);
+  if (r2 == 0.0) r = 0.0;  // two electrons at one point: 1/r is infinite, r is not NaN
+}
+
 // Minimum-image pair geometry (distances, reptation.f:4136-4160).
 __device__ __forceinline__ void pair_geom(const DevSys &S, const double *x, int i, int j,
                                           double &rx, double &ry, double &r, double &byr,
@@ -432,10 +443,9 @@ __device__ __forceinline__ void pair_geom(const DevSys &S, const double *x, int 
   ry = x[2 * i + 1] - x[2 * j + 1];
   rx = rx - S.el[0] * round(S.eli[0] * rx);
   ry = ry - S.el[1] * round(S.eli[1] * ry);
-  r = sqrt(rx * rx + ry * ry);
+  pair_dist(rx * rx + ry * ry, r, byr);
   ind = (int)(r * S.drti);
   rem = r - ind * S.drt;
-  byr = 1.0 / r;
 }
 
 // ---- the pair passes in either precision R of the two-body Jastrow and
@@ -510,7 +520,8 @@ __device__ __forceinline__ R spline0(const Knots<R> &K, const R *part, int iexp,
   const auto u = row_part<kSh>(part);
   const R rm = rem * K.drti;
   R f = u.x + rm * (u.y + rm * (u.z + rm * u.w));
-  for (int k = 0; k < iexp; k++) f *= byr;
+  if (iexp > 0) f *= byr;
+  for (int k = 1; k < iexp; k++) f *= byr;
   return f;
 }
 
@@ -525,10 +536,9 @@ __device__ __forceinline__ void pair_geom(const DevSys &S, const Knots<double> &
   ry = x[2 * i + 1] - x[2 * j + 1];
   rx = rx - S.el[0] * round(S.eli[0] * rx);
   ry = ry - S.el[1] * round(S.eli[1] * ry);
-  r = sqrt(rx * rx + ry * ry);
+  pair_dist(rx * rx + ry * ry, r, byr);
   ind = (int)(r * K.drti);
   rem = r - ind * K.drt;
-  byr = 1.0 / r;
 }
 __device__ __forceinline__ void pair_geom(const DevSys &S, const Knots<float> &K,
                                           const double *x, int i, int j, float &rx, float &ry,
@@ -608,7 +618,7 @@ __device__ __forceinline__ double group8_sum(double v) { return group_sum<8>(v);
 
 // Deterministic block sum of K values at once; results valid in every
 // thread. Uses red[0 .. K*8).
-template <int K>
+template <int K, int NT = kThreads>
 __device__ __forceinline__ void block_sum_n(double (&v)[K], double *red) {
 #pragma unroll
   for (int k = 0; k < K; k++)
@@ -622,7 +632,7 @@ __device__ __forceinline__ void block_sum_n(double (&v)[K], double *red) {
 #pragma unroll
   for (int k = 0; k < K; k++) {
     double t = 0.0;
-    for (int ww = 0; ww < kThreads / 32; ww++) t += red[k * 8 + ww];
+    for (int ww = 0; ww < NT / 32; ww++) t += red[k * 8 + ww];
     v[k] = t;
   }
   __syncthreads();
@@ -1419,6 +1429,11 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
     PairSum<double> qx, qy, sbxx, sbxy, sbyy, qbx, qby;
     PairSum<double> qbx1, qby1;  // kJ: the sums over type 1 (qbx, qby those over type 0)
     const int jp = N * (N + 1) / 2;  // kJ: a plane of Jacobian blocks
+    double *const jrow = kJ && pout ? pout + jac_row(N, i) : nullptr;
+    const R *const rows0 = rows + (size_t)S.cmb_blk[ti][0] * (S.cmb_ng + 1) * RS;
+    const R *const rows1 = rows + (size_t)S.cmb_blk[ti][1] * (S.cmb_ng + 1) * RS;
+    const int iexp0 = S.has_v2 ? S.tab_iexp[S.iv2[ti][0]] : 0;
+    const int iexp1 = S.has_v2 && S.nt > 1 ? S.tab_iexp[S.iv2[ti][1]] : 0;
     if (valid) {
       for (int j = lane8; j < N; j += LG) {
         if (j == i) continue;
@@ -1436,7 +1451,8 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
         } else {
           pair_geom(S, K, m.x, i, j, rx, ry, r, byr, ind, rem);
         }
-        const R *row = pair_row<RS>(S, rows, ti, tj, ind);
+        // as pair_row: the knot getf clamps to
+        const R *row = (tj ? rows1 : rows0) + max(0, min(S.cmb_ng, ind)) * RS;
         if (S.has_u2) {
           R t, dt, ddt;
           spline3<kSh>(K, row + Lay::u2, rem, t, dt, ddt);
@@ -1491,8 +1507,8 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
               qbx.add(w2 * rxd);
               qby.add(w2 * ryd);
             }
-            if (pout && i < j) {
-              double *e = pout + jac_row(N, i) + j;
+            if (jrow && i < j) {
+              double *e = jrow + j;
               e[0] = -(t + c * rxd * rxd);
               e[jp] = -(c * rxd * ryd);
               e[2 * jp] = -(t + c * ryd * ryd);
@@ -1509,7 +1525,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
           }
         }
         if (S.has_v2)
-          vp.add((R)0.5 * spline0<kSh>(K, row + Lay::v2, S.tab_iexp[S.iv2[ti][tj]], rem, byr));
+          vp.add((R)0.5 * spline0<kSh>(K, row + Lay::v2, tj ? iexp1 : iexp0, rem, byr));
       }
     }
     double ltf_v = ltf.value(), gx_v = gx.value(), gy_v = gy.value(), lap_v = lap.value();
@@ -1640,6 +1656,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
 // The end of an evaluation: -ln psi from the Jastrow sum ltf_j and ln|det|,
 // the kinetic and potential energies and every property from the
 // per-particle sums in m and rho_k; returns status with what it adds.
+template <int NT = kThreads>
 __device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double ltf_j,
                                     double logdet_sum, int status, double *hl, double *props,
                                     double *sign, long long &tph) {
@@ -1655,7 +1672,7 @@ __device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double l
   // nt <= 2), the drift cutoff factors, and the k-space sums of every type
   // pair (reptation.f:4034-4052), all in one block reduction
   double sums[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = tid; i < N; i += kThreads) {
+  for (int i = tid; i < N; i += NT) {
     double gx = m.g[2 * i], gy = m.g[2 * i + 1], lp = m.lap[i], ph = 0.0;
     if (S.has_bf && !underflow) {
       gx += m.gd[2 * i];
@@ -1702,7 +1719,7 @@ __device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double l
       vkp[p] = S.coef + (iv >= 0 ? S.tab_vkoff[iv] : 0);
       nkmax = max(nkmax, nkp[p]);
     }
-    for (int k = tid; k < nkmax; k += kThreads) {
+    for (int k = tid; k < nkmax; k += NT) {
       double vk[4];
 #pragma unroll
       for (int p = 0; p < 4; p++) vk[p] = k < nkp[p] ? __ldg(vkp[p] + k) : 0.0;
@@ -1715,7 +1732,7 @@ __device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double l
       }
     }
   }
-  block_sum_n<13>(sums, m.red);
+  block_sum_n<13, NT>(sums, m.red);
   double kin0 = 0.0, pot0 = 0.0, efp = 0.0;
   double kin_t[2] = {0, 0}, un_t[2] = {0, 0}, pot_t[2] = {0, 0};
 #pragma unroll
@@ -1787,7 +1804,7 @@ __device__ inline int eval_assemble(const DevSys &S, const EvalSmem &m, double l
     int cnt = 0;
     for (int it = 0; it < nt; it++) {
       if (S.irhok[it] == 0) continue;
-      for (int e = tid; e < 2 * S.nk; e += kThreads)
+      for (int e = tid; e < 2 * S.nk; e += NT)
         props[S.jrhok + cnt + e] = (it < S.nrhok) ? m.rhok[2 * it * S.nk + e] : 0.0;
       cnt += 2 * S.nk;
     }
