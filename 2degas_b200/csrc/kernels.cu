@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(
     }
     cp_async_wait_all();
   }
+  pdl_wait();  // the rows above are tables, written when the handle was made
   __syncthreads();
   const GroupSync sync{1 + grp, kThreads};
   const int N = S.N, N2 = 2 * N;
@@ -622,6 +623,7 @@ __global__ void __launch_bounds__(kEndThreads, 8) move_real_kernel(const __grid_
                                                                 MoveArgs a, RealArgs ra,
                                                                 MoveScratch L) {
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   MoveRealSmem v;
@@ -708,6 +710,7 @@ __global__ void __launch_bounds__(kEndThreads, 8) eval_real_kernel(const __grid_
                                                                 double *props, double *s,
                                                                 int *status) {
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   double *pn = reinterpret_cast<double *>(smem + off);
@@ -767,7 +770,16 @@ constexpr int kBranchThreads = 1024;
 __global__ void __launch_bounds__(kBranchThreads) branch_kernel(int nw, double *wate,
                                                                 uint64_t seed, uint32_t gen0,
                                                                 const uint32_t *ctr,
-                                                                BranchScratch b) {
+                                                                BranchScratch b, int in_smem) {
+  extern __shared__ __align__(16) char smem[];
+  pdl_wait();
+  if (in_smem) {  // the per-walker arrays but the result and the counter
+    b.delt = reinterpret_cast<double *>(smem);
+    b.csum = b.delt + nw;
+    b.mult = reinterpret_cast<int *>(b.csum + nw);
+    b.ecum = b.mult + nw;
+    b.zrank = b.ecum + nw;
+  }
   const uint32_t gen = gen0 + (ctr ? ctr[1] : 0u);
   __shared__ double dws[33];
   __shared__ int iws[33];
@@ -872,6 +884,7 @@ __global__ void __launch_bounds__(kBranchThreads) branch_kernel(int nw, double *
 }
 
 __global__ void gather_kernel(DevPop from, DevPop to, const int *src, int N2, int nt, int np) {
+  pdl_wait();
   const int j = blockIdx.x, i = src[j];
   for (int e = threadIdx.x; e < N2; e += blockDim.x) {
     to.x[(size_t)j * N2 + e] = from.x[(size_t)i * N2 + e];
@@ -1036,8 +1049,7 @@ static cudaError_t launch_pairs_t(const DevSys &hs, DevPop pop, const MoveArgs &
   const int need = (a.nw + G - 1) / G;
   const int cap = nsm * (per_sm > 0 ? per_sm : 1);
   const int grid = need < cap ? need : cap;
-  pairs_kernel<R, G, LG, kJ><<<grid, G * kThreads, sm, st>>>(hs, pop, a, stage, xe);
-  return cudaGetLastError();
+  return launch_pdl(pairs_kernel<R, G, LG, kJ>, grid, G * kThreads, sm, st, hs, pop, a, stage, xe);
 }
 
 template <class R, int LG, bool kJ>
@@ -1096,9 +1108,8 @@ cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const d
   if ((e = launch_real_det(hs, ds, nw, scr, st)) != cudaSuccess) return e;
   const size_t sm = eval_real_smem_bytes(hs);
   if ((e = set_smem((const void *)eval_real_kernel, sm)) != cudaSuccess) return e;
-  eval_real_kernel<<<nw, kEndThreads, sm, st>>>(hs, nw, real_args(hs, scr), move_scratch(hs), g, hl,
-                                             props, s, status);
-  return cudaGetLastError();
+  return launch_pdl(eval_real_kernel, nw, kEndThreads, sm, st, hs, nw, real_args(hs, scr),
+                    move_scratch(hs), g, hl, props, s, status);
 }
 
 bool orb_inv_applies(const DevSys &hs) { return hs.split_inv && orb_inv_fits(hs); }
@@ -1136,9 +1147,8 @@ cudaError_t launch_move(const DevSys &hs, const DevSys *ds, DevPop pop, const Mo
     const size_t sm = move_real_smem_bytes(hs);
     cudaError_t e = set_smem((const void *)move_real_kernel, sm);
     if (e != cudaSuccess) return e;
-    move_real_kernel<<<a.nw, kEndThreads, sm, st>>>(hs, pop, a, real_args(hs, a.scr),
-                                                 move_scratch(hs));
-    return cudaGetLastError();
+    return launch_pdl(move_real_kernel, a.nw, kEndThreads, sm, st, hs, pop, a,
+                      real_args(hs, a.scr), move_scratch(hs));
   }
   const bool seq = !hs.gmat && a.orb_inv && orb_inv_applies(hs) && props_buf_fits(hs);
   size_t sm = seq ? move_smem_bytes_seq(hs) : move_smem_bytes(hs);
@@ -1160,15 +1170,20 @@ cudaError_t launch_block_reduce(const double *blk, const double *norm, int n, in
 cudaError_t launch_branch(int nw, double *wate, uint64_t seed, uint32_t gen, BranchScratch b,
                           cudaStream_t st, const uint32_t *ctr) {
   if (nw <= 0) return cudaSuccess;
-  branch_kernel<<<1, kBranchThreads, 0, st>>>(nw, wate, seed, gen, ctr, b);
-  return cudaGetLastError();
+  // 28 bytes per walker in shared memory while they fit (25 us per 4096
+  // walkers from global memory: chains of loads at L2 latency)
+  const size_t sm = 28 * (size_t)nw;
+  const int in_smem = sm <= 200 * 1024;
+  cudaError_t e;
+  if (in_smem && (e = set_smem((const void *)branch_kernel, sm)) != cudaSuccess) return e;
+  return launch_pdl(branch_kernel, 1, kBranchThreads, in_smem ? sm : 0, st, nw, wate, seed, gen,
+                    ctr, b, in_smem);
 }
 
 cudaError_t launch_gather(const DevSys &hs, DevPop from, DevPop to, const int *src, int nw,
                           cudaStream_t st) {
   if (nw <= 0) return cudaSuccess;
-  gather_kernel<<<nw, 128, 0, st>>>(from, to, src, 2 * hs.N, hs.nt, hs.nprops);
-  return cudaGetLastError();
+  return launch_pdl(gather_kernel, nw, 128, 0, st, from, to, src, 2 * hs.N, hs.nt, hs.nprops);
 }
 
 __global__ void counters_add_kernel(uint32_t *ctr, uint32_t steps, uint32_t gens) {

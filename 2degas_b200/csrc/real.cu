@@ -128,6 +128,7 @@ template <int NM>
 __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs a, int nw) {
   static_assert(NM <= 32, "one lane per row");
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   constexpr int LD = real_ld(NM), TT = (NM + 7) / 8;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int item = blockIdx.x * kRealWarps + wl;
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, in
   __shared__ int perm[176], rowl[176];
   __shared__ int singular;
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0];
   if (w >= nw || n <= 32) return;  // whole CTAs
@@ -557,6 +559,7 @@ inline size_t real_f_doubles(int n, int ldw) {
 
 __global__ void __launch_bounds__(kFThreads, 1) real_f_kernel(RealArgs a, int nw, int blocks) {
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   const int bj = blockIdx.x % blocks, item = blockIdx.x / blocks;
   const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0], j0 = 32 * bj;
@@ -785,6 +788,7 @@ template <int kB>
 __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
     real_s_kernel(RealArgs a, const DevSys *ds, int nw) {
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
   if (w >= nw) return;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x, NW = nthr >> 5;
@@ -950,11 +954,9 @@ cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int 
   const void *k = resident ? (const void *)real_s_kernel<1> : (const void *)real_s_kernel<2>;
   cudaError_t e = raise_smem_limit(k, sm);
   if (e != cudaSuccess) return e;
-  if (resident)
-    real_s_kernel<1><<<nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st>>>(a, ds, nw);
-  else
-    real_s_kernel<2><<<nw * hs.nt, 512, sm, st>>>(a, ds, nw);
-  return cudaGetLastError();
+  return resident ? launch_pdl(real_s_kernel<1>, nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st, a,
+                               ds, nw)
+                  : launch_pdl(real_s_kernel<2>, nw * hs.nt, 512, sm, st, a, ds, nw);
 }
 
 template <int kL, int kR, int kC, int kS, int kMaxT, int kMB, bool kFused>
@@ -963,8 +965,7 @@ cudaError_t launch_inv_cta(const RealArgs &a, int n, int items, int nw, cudaStre
   auto k = real_inv_cta_kernel<kL, kR, kC, kS, kMaxT, kMB, kFused>;
   cudaError_t e = raise_smem_limit((const void *)k, sm);
   if (e != cudaSuccess) return e;
-  k<<<items, 32 * gjc_warps(n, kL, kR), sm, st>>>(a, nw);
-  return cudaGetLastError();
+  return launch_pdl(k, items, 32 * gjc_warps(n, kL, kR), sm, st, a, nw);
 }
 
 template <int NM>
@@ -973,9 +974,8 @@ cudaError_t launch_det_warp(const RealArgs &a, int items, int nw, cudaStream_t s
   const void *k = (const void *)real_det_warp_kernel<NM>;
   cudaError_t e = raise_smem_limit(k, sm);
   if (e != cudaSuccess) return e;
-  real_det_warp_kernel<NM>
-      <<<(items + kRealWarps - 1) / kRealWarps, 32 * kRealWarps, sm, st>>>(a, nw);
-  return cudaGetLastError();
+  return launch_pdl(real_det_warp_kernel<NM>, (items + kRealWarps - 1) / kRealWarps,
+                    32 * kRealWarps, sm, st, a, nw);
 }
 
 cudaError_t launch_orbitals_f(const DevSys &hs, const RealArgs &a, int nw, cudaStream_t st) {
@@ -1009,8 +1009,7 @@ cudaError_t launch_orbitals_f(const DevSys &hs, const RealArgs &a, int nw, cudaS
   const int blocks = (nm + 31) / 32;
   const size_t sm = sizeof(double) * real_f_doubles(nm, (nm + 3) & ~3);
   if ((e = raise_smem_limit((const void *)real_f_kernel, sm)) != cudaSuccess) return e;
-  real_f_kernel<<<items * blocks, kFThreads, sm, st>>>(a, nw, blocks);
-  return cudaGetLastError();
+  return launch_pdl(real_f_kernel, items * blocks, kFThreads, sm, st, a, nw, blocks);
 }
 
 }  // namespace

@@ -548,6 +548,7 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
           __ldg(src + (size_t)rr * VG + q);
     }
   }
+  pdl_wait();  // the rows above are tables, written when the handle was made
   __syncthreads();
   const GroupSync sync{1 + grp, kThreads};
   const int N = S.N, N2 = 2 * N, nb = a.nbuf;
@@ -713,6 +714,7 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_det_kernel(const DevSys *sp, 
 __global__ void __launch_bounds__(kThreads, 3) rmc_real_kernel(
     const __grid_constant__ DevSys S, RmcArgs a, RealArgs ra, MoveScratch L, int idelta) {
   extern __shared__ __align__(16) char smem[];
+  pdl_wait();
   EvalSmem m;
   const size_t off = real_carve(S, smem, &m);
   double *pn = reinterpret_cast<double *>(smem + off);
@@ -1014,9 +1016,8 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::RmcArgs 
                                                                    sm)) != cudaSuccess)
     return e;
   const int need = (a.nrep + G - 1) / G, cap = nsm * (per_sm > 0 ? per_sm : 1);
-  q2d::rmc_pairs_kernel<double, G, LG, kJ>
-      <<<need < cap ? need : cap, G * q2d::kThreads, sm, st>>>(hs, a, scr, idelta, stage);
-  return cudaGetLastError();
+  return q2d::launch_pdl(q2d::rmc_pairs_kernel<double, G, LG, kJ>, need < cap ? need : cap,
+                         G * q2d::kThreads, sm, st, hs, a, scr, idelta, stage);
 }
 
 template <int G, bool kJ>
@@ -1098,9 +1099,8 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
             RCK(q2d::launch_real_det(h->hs, h->ds, h->rmc.nrep, h->d_mscr, h->stream));
           }
           ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
-          q2d::rmc_real_kernel<<<h->rmc.nrep, q2d::kThreads, smr, h->stream>>>(
-              h->hs, a, q2d::real_args(h->hs, h->d_mscr), q2d::move_scratch(h->hs), idelta);
-          RCK(cudaGetLastError());
+          RCK(q2d::launch_pdl(q2d::rmc_real_kernel, h->rmc.nrep, q2d::kThreads, smr, h->stream, h->hs, a,
+                              q2d::real_args(h->hs, h->d_mscr), q2d::move_scratch(h->hs), idelta));
           continue;
         }
         ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
