@@ -56,6 +56,7 @@ struct EvalSmem {
   // lattice power tables of rho_k in the pair kernels (DevSys::rk_lat):
   // exp(2 pi i p x_i / Lx) at [p N + i], p <= rk_p1, then exp(2 pi i p y_i / Ly)
   double2 *rkt = nullptr;
+  double *rks = nullptr;  // their products summed over a type's particles
 };
 
 __host__ __device__ inline size_t align16(size_t b) { return (b + 15) & ~size_t(15); }
@@ -247,6 +248,9 @@ __host__ __device__ inline size_t pair_carve(const DevSys &s, char *base, EvalSm
   t.rhok = (double *)take(sizeof(double) * 2 * (s.nk > 0 ? s.nk : 1) * 2);
   t.red = (double *)take(sizeof(double) * nthreads);
   t.rkt = s.rk_lat ? (double2 *)take(sizeof(double2) * (s.rk_p1 + s.rk_p2 + 2) * N) : nullptr;
+  t.rks = s.rk_lat ? (double *)take(sizeof(double) * 4 * s.nt * 64 * ((s.rk_p1 + 8) >> 3) *
+                                    ((s.rk_p2 + 8) >> 3))
+                   : nullptr;
   if (m) *m = t;
   return off;
 }
@@ -1319,59 +1323,67 @@ __device__ inline void compute_rhok(const DevSys &S, const EvalSmem &m, int t, i
 // (DevSys::rk_lat): with k = 2 pi (n1 / Lx, n2 / Ly), exp(i k.x) =
 // X_{n1}(x) Y_{n2}(y), X_p(x) = exp(2 pi i p x / Lx), and each particle's
 // X_0 .. X_{rk_p1}, Y_0 .. Y_{rk_p2} are built once by repeated complex
-// multiplication (conjugates for negative indices), so a (k, particle) term
-// is one complex product instead of a sincos. Items, lanes and the shuffle
-// tree as compute_rhok; each term agrees with its sincos to a few ulp.
-// Threads t .. t+nthr-1 of the group whose barrier is sync.
-template <int LG, class Sync>
+// multiplication. The sums over a type's particles of the four real products
+// of X_p and Y_q, p and q >= 0, are small matrix products over the particles
+// (FP64 tensor cores, mma.m8n8k4: 64 for two types of 29 electrons), from which
+// rho at any signs follows: RR - II + i (RI + IR) at (p, q), conjugated factors
+// at negative indices. A complex product per (k, particle) took 30% of the
+// pair kernel's time at N = 58 and 60 k vectors.
+// Threads t .. t+nthr-1 (whole warps) of the group whose barrier is sync.
+template <class Sync>
 __device__ inline void compute_rhok_lattice(const DevSys &S, const EvalSmem &m, int t, int nthr,
                                             Sync sync) {
   const int N = S.N, P1 = S.rk_p1, P2 = S.rk_p2;
   double2 *X = m.rkt, *Y = m.rkt + (size_t)(P1 + 1) * N;
-  for (int i = t; i < N; i += nthr) {
-    double sx, cx, sy, cy;
-    sincospi(2.0 * (m.x[2 * i] * S.eli[0]), &sx, &cx);
-    sincospi(2.0 * (m.x[2 * i + 1] * S.eli[1]), &sy, &cy);
-    const double2 bx = make_double2(cx, sx), by = make_double2(cy, sy);
-    double2 px = make_double2(1.0, 0.0), py = px;
-    X[i] = px;
-    Y[i] = py;
-    for (int p = 1; p <= P1; p++) {
-      px = cmul(px, bx);
-      X[(size_t)p * N + i] = px;
+  for (int e = t; e < 2 * N; e += nthr) {
+    const int ax = e >= N ? 1 : 0, i = e - ax * N, P = ax ? P2 : P1;
+    double2 *T = (ax ? Y : X) + i;
+    double sb, cb;
+    sincospi(2.0 * (m.x[2 * i + ax] * S.eli[ax]), &sb, &cb);
+    const double2 b = make_double2(cb, sb);
+    double2 p = make_double2(1.0, 0.0);
+    T[0] = p;
+    for (int k = 1; k <= P; k++) {
+      p = cmul(p, b);
+      T[(size_t)k * N] = p;
     }
-    for (int p = 1; p <= P2; p++) {
-      py = cmul(py, by);
-      Y[(size_t)p * N + i] = py;
+  }
+  sync();
+  const int T1 = (P1 + 8) >> 3, T2 = (P2 + 8) >> 3, ldt = 8 * T2, tab = 8 * T1 * ldt;
+  double *R = m.rks;  // [type][RR, II, RI, IR][p][q]
+  {
+    const int warp = t >> 5, lane = t & 31, lg = lane >> 2, lt = lane & 3;
+    const double *xd = reinterpret_cast<const double *>(X), *yd = reinterpret_cast<const double *>(Y);
+    for (int it = warp; it < 4 * T1 * T2 * S.nt; it += nthr >> 5) {
+      const int pr = it & 3, tile = (it >> 2) % (T1 * T2), ty = (it >> 2) / (T1 * T2);
+      const int p0 = 8 * (tile / T2), q0 = 8 * (tile % T2);
+      const int f0 = S.ipfrst[ty], n = S.np[ty];
+      // RR, II, RI, IR: component of X, component of Y
+      const double *xa = xd + 2 * ((size_t)min(p0 + lg, P1) * N + f0) + (pr == 1 || pr == 3);
+      const double *ya = yd + 2 * ((size_t)min(q0 + lg, P2) * N + f0) + (pr == 1 || pr == 2);
+      double acc[2] = {0.0, 0.0};
+      for (int k0 = 0; k0 < n; k0 += 4) {
+        const int k = k0 + lt;
+        dmma_m8n8k4(acc, k < n ? xa[2 * k] : 0.0, k < n ? ya[2 * k] : 0.0);
+      }
+      double *o = R + (ty * 4 + pr) * tab + (p0 + lg) * ldt + q0 + 2 * lt;
+      o[0] = acc[0];
+      o[1] = acc[1];
     }
   }
   sync();
   const double c1 = S.el[0] * 0.15915494309189535, c2 = S.el[1] * 0.15915494309189535;
-  const int total = S.nt * S.nk, per_round = nthr / LG, l8 = t & (LG - 1);
-  for (int e0 = 0; e0 < total; e0 += per_round) {
-    const int e = e0 + t / LG;
-    const int ty = e < total ? e / S.nk : 0, k = e - ty * S.nk;
-    const bool on = e < total && S.irhok[ty] != 0;
-    double c = 0.0, sn = 0.0;
-    if (on) {
-      const int n1 = __double2int_rn(__ldg(S.kvec + 2 * k) * c1);
-      const int n2 = __double2int_rn(__ldg(S.kvec + 2 * k + 1) * c2);
-      const double2 *xp = X + (size_t)abs(n1) * N, *yp = Y + (size_t)abs(n2) * N;
-      for (int i = S.ipfrst[ty] + l8; i < S.ipfrst[ty] + S.np[ty]; i += LG) {
-        double2 xv = xp[i], yv = yp[i];
-        if (n1 < 0) xv.y = -xv.y;
-        if (n2 < 0) yv.y = -yv.y;
-        c += xv.x * yv.x - xv.y * yv.y;
-        sn += xv.x * yv.y + xv.y * yv.x;
-      }
-    }
-    c = group_sum<LG>(c);
-    sn = group_sum<LG>(sn);
-    if (on && l8 == 0) {
-      const int slot = S.irhok[ty] - 1;
-      m.rhok[2 * (slot * S.nk + k)] = c;
-      m.rhok[2 * (slot * S.nk + k) + 1] = sn;
-    }
+  for (int e = t; e < S.nt * S.nk; e += nthr) {
+    const int ty = e / S.nk, k = e - ty * S.nk;
+    if (S.irhok[ty] == 0) continue;
+    const int n1 = __double2int_rn(__ldg(S.kvec + 2 * k) * c1);
+    const int n2 = __double2int_rn(__ldg(S.kvec + 2 * k + 1) * c2);
+    const double *r = R + ty * 4 * tab + abs(n1) * ldt + abs(n2);
+    // factors conjugated at negative indices: the imaginary part's sign
+    const double s1 = n1 < 0 ? -1.0 : 1.0, s2 = n2 < 0 ? -1.0 : 1.0;
+    const int slot = S.irhok[ty] - 1;
+    m.rhok[2 * (slot * S.nk + k)] = r[0] - s1 * s2 * r[tab];
+    m.rhok[2 * (slot * S.nk + k) + 1] = s2 * r[2 * tab] + s1 * r[3 * tab];
   }
 }
 
@@ -1380,7 +1392,7 @@ __device__ inline void compute_rhok_lattice(const DevSys &S, const EvalSmem &m, 
 template <int LG, class Sync>
 __device__ inline void pair_rhok(const DevSys &S, const EvalSmem &m, int t, int nthr, Sync sync) {
   if (m.rkt)
-    compute_rhok_lattice<LG>(S, m, t, nthr, sync);
+    compute_rhok_lattice(S, m, t, nthr, sync);
   else
     compute_rhok<LG>(S, m, t, nthr);
 }
