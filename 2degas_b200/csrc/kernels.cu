@@ -177,8 +177,11 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 // the lanes per particle of the pair passes (4, 8 or 16: a launch choice,
 // DevSys::tune_lanes). kJ: the Jacobian blocks of the real-orbital route
 // (real_det.cuh) instead of the pairs' spline values; xe (kJ only) the
-// configurations to evaluate instead of a proposal.
-template <class R, int G, int LG, bool kJ>
+// configurations to evaluate instead of a proposal. kU3 = 0 (kJ, FP64): no
+// u3, whose rows are then not staged: 112 bytes a knot instead of 144, so two
+// groups fit beside them up to N = 162 (N = 122, 1024 walkers: 303 -> 217 us; N
+// = 58, 4096: 224 -> 218).
+template <class R, int G, int LG, bool kJ, int kU3 = -1>
 __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(
     const __grid_constant__ DevSys S, DevPop pop, MoveArgs a, int stage_rows, const double *xe) {
   constexpr int kPairGroups = G, kPairThreads = G * kThreads;
@@ -189,15 +192,16 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(
   pair_carve(S, smem + grp * carve, &m, kThreads);
   const R *rows_g = pair_rows<R>(S);
   R *rows_s = reinterpret_cast<R *>(smem + kPairGroups * carve);
-  if (stage_rows) {  // the first copy16 16-byte parts of each global row
-    using Lay = RowLayout<R>;
-    constexpr int V = Lay::copy16, VG = Lay::gstride * (int)sizeof(R) / 16;
+  if (stage_rows) {  // 16-byte parts of each global row: the first copy16, or those but u3's
+    constexpr bool kNoU3 = sizeof(R) == 8 && kU3 == 0;
+    using Lay = std::conditional_t<kNoU3, RowLayoutNoU3, RowLayout<R>>;
+    constexpr int V = Lay::copy16, VG = RowLayout<R>::gstride * (int)sizeof(R) / 16;
     const int nrow = S.cmb_nblk * (S.cmb_ng + 1);
     const float4 *src = reinterpret_cast<const float4 *>(rows_g);
     for (int e = threadIdx.x; e < nrow * V; e += kPairThreads) {
       const int r = e / V, q = e - r * V;
       cp_async16(reinterpret_cast<float4 *>(rows_s + (size_t)r * Lay::sstride) + q,
-                 src + (size_t)r * VG + q);
+                 src + (size_t)r * VG + (kNoU3 && q > 1 ? q + 2 : q));
     }
     cp_async_wait_all();
   }
@@ -232,10 +236,10 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) pairs_kernel(
                    : S.gmat    ? S.gmat_base + (size_t)w * S.gmat_stride
                                : o + L.pair;  // as real_base()
     if (stage_rows)
-      eval_pairs<kThreads, true, R, GroupSync, LG, kJ>(S, m, tph, pout, (const R *)rows_s, sync,
+      eval_pairs<kThreads, true, R, GroupSync, LG, kJ, kU3>(S, m, tph, pout, (const R *)rows_s, sync,
                                                        tid);
     else
-      eval_pairs<kThreads, false, R, GroupSync, LG, kJ>(S, m, tph, pout, rows_g, sync, tid);
+      eval_pairs<kThreads, false, R, GroupSync, LG, kJ, kU3>(S, m, tph, pout, rows_g, sync, tid);
     pair_rhok<LG>(S, m, tid, kThreads, sync);
     sync();
     for (int j = tid; j < 4 * S.nk; j += kThreads) o[L.rhok + j] = m.rhok[j];
@@ -987,8 +991,8 @@ cudaError_t launch_eval(const DevSys &hs, const DevSys *ds, int nw, const double
 static size_t pair_group_bytes(const DevSys &hs) {
   return (pair_carve(hs, nullptr, nullptr, kThreads) + 127) & ~size_t(127);
 }
-static size_t pair_rows_bytes(const DevSys &hs) {
-  const size_t row = hs.pair_f32 ? sizeof(float) * RowLayout<float>::sstride
+static size_t pair_rows_bytes(const DevSys &hs, bool no_u3 = false) {
+  const size_t row = no_u3 && !hs.pair_f32 ? sizeof(double) * RowLayoutNoU3::sstride : hs.pair_f32 ? sizeof(float) * RowLayout<float>::sstride
                                  : sizeof(double) * RowLayout<double>::sstride;
   return row * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
 }
@@ -996,8 +1000,8 @@ static size_t pair_rows_bytes(const DevSys &hs) {
 // Groups, staging and lanes compute the same pair terms; groups and staging
 // leave every bit, the lanes the order of a particle's partial sums.
 //   groups and staging (FP64, us per launch, 148 SMs): one group per CTA
-//   when two and the rows do not fit a CTA's shared memory (N = 122, 1024
-//   walkers: 321 against 344; N = 161, 148: 95 against 173) and when every SM
+//   when two and the rows do not fit a CTA's shared memory (N = 122 with 144-byte
+//   rows, 1024 walkers: 321 against 344; N = 161, 148: 95 against 173) and when every SM
 //   has at most one walker (N = 58, 148: 25 against 29); rows of small
 //   systems stay in global memory up to seven walkers per SM, where copying
 //   them costs more than it saves (N = 26: 17.0 against 19.4 at 64 walkers, 29.5
@@ -1007,9 +1011,10 @@ static size_t pair_rows_bytes(const DevSys &hs) {
 //   ceil(N / lanes) partners and the round's reductions (N = 58: four lanes 273,
 //   eight 312; N = 122: 344 against 360; N = 74: eight 209, four 230). Eight in
 //   mixed precision, whose FP32 sums follow the order.
-PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin) {
+PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3) {
   PairLaunch p{hs.tune_groups, hs.tune_stage != 1, hs.tune_lanes};
-  const size_t grp = pair_group_bytes(hs), rows = pair_rows_bytes(hs), lim = (size_t)optin - 1024;
+  const size_t grp = pair_group_bytes(hs), rows = pair_rows_bytes(hs, no_u3),
+               lim = (size_t)optin - 1024;
   if (p.groups == 0) {
     if (2 * grp + rows > lim || nw <= nsm) {
       p.groups = 1;
@@ -1034,11 +1039,11 @@ PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin) {
   return p;
 }
 
-template <class R, int G, int LG, bool kJ>
+template <class R, int G, int LG, bool kJ, int kU3 = -1>
 static cudaError_t launch_pairs_t(const DevSys &hs, DevPop pop, const MoveArgs &a,
                                   cudaStream_t st, int nsm, int stage, const double *xe) {
-  const void *k = (const void *)pairs_kernel<R, G, LG, kJ>;
-  const size_t sm = G * pair_group_bytes(hs) + (stage ? pair_rows_bytes(hs) : 0);
+  const void *k = (const void *)pairs_kernel<R, G, LG, kJ, kU3>;
+  const size_t sm = G * pair_group_bytes(hs) + (stage ? pair_rows_bytes(hs, kU3 == 0) : 0);
   cudaError_t e;
   if ((e = set_smem(k, sm)) != cudaSuccess) return e;
   int per_sm = 1;
@@ -1049,13 +1054,18 @@ static cudaError_t launch_pairs_t(const DevSys &hs, DevPop pop, const MoveArgs &
   const int need = (a.nw + G - 1) / G;
   const int cap = nsm * (per_sm > 0 ? per_sm : 1);
   const int grid = need < cap ? need : cap;
-  return launch_pdl(pairs_kernel<R, G, LG, kJ>, grid, G * kThreads, sm, st, hs, pop, a, stage, xe);
+  return launch_pdl(pairs_kernel<R, G, LG, kJ, kU3>, grid, G * kThreads, sm, st, hs, pop, a, stage, xe);
 }
 
 template <class R, int LG, bool kJ>
 static cudaError_t launch_pairs_g(const DevSys &hs, DevPop pop, const MoveArgs &a,
                                   cudaStream_t st, int nsm, const PairLaunch &p,
                                   const double *xe) {
+  if constexpr (kJ && sizeof(R) == 8)
+    if (!hs.has_u3)
+      return p.groups == 1
+                 ? launch_pairs_t<R, 1, LG, kJ, 0>(hs, pop, a, st, nsm, p.stage, xe)
+                 : launch_pairs_t<R, 2, LG, kJ, 0>(hs, pop, a, st, nsm, p.stage, xe);
   return p.groups == 1 ? launch_pairs_t<R, 1, LG, kJ>(hs, pop, a, st, nsm, p.stage, xe)
                        : launch_pairs_t<R, 2, LG, kJ>(hs, pop, a, st, nsm, p.stage, xe);
 }
@@ -1063,7 +1073,7 @@ static cudaError_t launch_pairs_g(const DevSys &hs, DevPop pop, const MoveArgs &
 template <class R, bool kJ>
 static cudaError_t launch_pairs_r(const DevSys &hs, DevPop pop, const MoveArgs &a,
                                   cudaStream_t st, int nsm, int optin, const double *xe) {
-  const PairLaunch p = pair_launch(hs, a.nw, nsm, optin);
+  const PairLaunch p = pair_launch(hs, a.nw, nsm, optin, kJ && sizeof(R) == 8 && !hs.has_u3);
   switch (p.lanes) {
     case 4: return launch_pairs_g<R, 4, kJ>(hs, pop, a, st, nsm, p, xe);
     case 16: return launch_pairs_g<R, 16, kJ>(hs, pop, a, st, nsm, p, xe);

@@ -60,7 +60,8 @@ cudaError_t launch_pdl(void (*k)(P...), int grid, int block, size_t smem, cudaSt
 struct PairLaunch {
   int groups, stage, lanes;
 };
-PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin);
+// no_u3: the kernel for systems without u3 (its staged rows are smaller).
+PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3);
 
 // Raise (never lower) kernel fn's dynamic shared-memory limit on the current
 // device to bytes; safe to call from several host threads.

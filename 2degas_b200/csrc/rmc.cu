@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 2) rmc_move_kernel(const DevSys *sp,
 // and, after the reptile's last growth of the move, the path tail. A move
 // of mdelta > 1 takes mdelta launch pairs; a reptile whose move has fewer
 // growths skips the later ones.
-template <class R, int G, int LG, bool kJ>
+template <class R, int G, int LG, bool kJ, int kU3>
 __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
     const __grid_constant__ DevSys S, RmcArgs a, double *scr, int idelta, int stage_rows) {
   constexpr int kPairThreads = G * kThreads;
@@ -537,16 +537,18 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
   pair_carve(S, smem + grp * carve, &m, kThreads);
   const R *rows_g = pair_rows<R>(S);
   R *rows_s = reinterpret_cast<R *>(smem + G * carve);
-  if (stage_rows) {  // the first copy16 16-byte parts of each global row
-    using Lay = RowLayout<R>;
-    constexpr int V = Lay::copy16, VG = Lay::gstride * (int)sizeof(R) / 16;
+  if (stage_rows) {  // as pairs_kernel
+    constexpr bool kNoU3 = kU3 == 0;
+    using Lay = std::conditional_t<kNoU3, RowLayoutNoU3, RowLayout<R>>;
+    constexpr int V = Lay::copy16, VG = RowLayout<R>::gstride * (int)sizeof(R) / 16;
     const int nrow = S.cmb_nblk * (S.cmb_ng + 1);
     const float4 *src = reinterpret_cast<const float4 *>(rows_g);
     for (int e = threadIdx.x; e < nrow * V; e += kPairThreads) {
       const int rr = e / V, q = e - rr * V;
-      reinterpret_cast<float4 *>(rows_s + (size_t)rr * Lay::sstride)[q] =
-          __ldg(src + (size_t)rr * VG + q);
+      cp_async16(reinterpret_cast<float4 *>(rows_s + (size_t)rr * Lay::sstride) + q,
+                 src + (size_t)rr * VG + (kNoU3 && q > 1 ? q + 2 : q));
     }
+    cp_async_wait_all();
   }
   pdl_wait();  // the rows above are tables, written when the handle was made
   __syncthreads();
@@ -585,10 +587,10 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
                    : kJ && S.gmat         ? S.gmat_base + (size_t)r * S.gmat_stride
                                           : o + L.pair;
     if (stage_rows)
-      eval_pairs<kThreads, true, R, GroupSync, LG, kJ>(S, m, tph, pout, (const R *)rows_s, sync,
+      eval_pairs<kThreads, true, R, GroupSync, LG, kJ, kU3>(S, m, tph, pout, (const R *)rows_s, sync,
                                                        tid);
     else
-      eval_pairs<kThreads, false, R, GroupSync, LG, kJ>(S, m, tph, pout, rows_g, sync, tid);
+      eval_pairs<kThreads, false, R, GroupSync, LG, kJ, kU3>(S, m, tph, pout, rows_g, sync, tid);
     pair_rhok<LG>(S, m, tid, kThreads, sync);
     sync();
     for (int e = tid; e < 4 * S.nk; e += kThreads) o[L.rhok + e] = m.rhok[e];
@@ -1000,15 +1002,16 @@ extern "C" int qmc2d_rmc_init(qmc2d_handle *h, int nrep, const qmc2d_rmc_params 
   return q2d_sync_status(h, nrep);
 }
 
-template <int G, int LG, bool kJ>
+template <int G, int LG, bool kJ, int kU3>
 static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::RmcArgs &a, double *scr,
                                       int idelta, int nsm, int stage, cudaStream_t st) {
   cudaError_t e;
-  const void *k = (const void *)q2d::rmc_pairs_kernel<double, G, LG, kJ>;
+  const void *k = (const void *)q2d::rmc_pairs_kernel<double, G, LG, kJ, kU3>;
   const size_t carve =
       G * ((q2d::pair_carve(hs, nullptr, nullptr, q2d::kThreads) + 127) & ~size_t(127));
-  const size_t rows = sizeof(double) * q2d::RowLayout<double>::sstride * (size_t)hs.cmb_nblk *
-                      (hs.cmb_ng + 1);
+  constexpr int stride =
+      kU3 == 0 ? q2d::RowLayoutNoU3::sstride : q2d::RowLayout<double>::sstride;
+  const size_t rows = sizeof(double) * stride * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
   const size_t sm = carve + (stage ? rows : 0);
   if ((e = q2d::raise_smem_limit(k, sm)) != cudaSuccess) return e;
   int per_sm = 1;
@@ -1016,18 +1019,18 @@ static cudaError_t launch_rmc_pairs_t(const q2d::DevSys &hs, const q2d::RmcArgs 
                                                                    sm)) != cudaSuccess)
     return e;
   const int need = (a.nrep + G - 1) / G, cap = nsm * (per_sm > 0 ? per_sm : 1);
-  return q2d::launch_pdl(q2d::rmc_pairs_kernel<double, G, LG, kJ>, need < cap ? need : cap,
+  return q2d::launch_pdl(q2d::rmc_pairs_kernel<double, G, LG, kJ, kU3>, need < cap ? need : cap,
                          G * q2d::kThreads, sm, st, hs, a, scr, idelta, stage);
 }
 
-template <int G, bool kJ>
+template <int G, bool kJ, int kU3>
 static cudaError_t launch_rmc_pairs_g(const q2d::DevSys &hs, const q2d::RmcArgs &a, double *scr,
                                       int idelta, int nsm, const q2d::PairLaunch &p,
                                       cudaStream_t st) {
   switch (p.lanes) {
-    case 4: return launch_rmc_pairs_t<G, 4, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
-    case 16: return launch_rmc_pairs_t<G, 16, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
-    default: return launch_rmc_pairs_t<G, 8, kJ>(hs, a, scr, idelta, nsm, p.stage, st);
+    case 4: return launch_rmc_pairs_t<G, 4, kJ, kU3>(hs, a, scr, idelta, nsm, p.stage, st);
+    case 16: return launch_rmc_pairs_t<G, 16, kJ, kU3>(hs, a, scr, idelta, nsm, p.stage, st);
+    default: return launch_rmc_pairs_t<G, 8, kJ, kU3>(hs, a, scr, idelta, nsm, p.stage, st);
   }
 }
 
@@ -1044,12 +1047,16 @@ static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs0, const q2d::RmcArgs &
   if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
       cudaSuccess)
     return e;
-  const q2d::PairLaunch p = q2d::pair_launch(hs, a.nrep, nsm, optin);
+  const bool no_u3 = real && !hs.has_u3;
+  const q2d::PairLaunch p = q2d::pair_launch(hs, a.nrep, nsm, optin, no_u3);
+  if (no_u3)
+    return p.groups == 1 ? launch_rmc_pairs_g<1, true, 0>(hs, a, scr, idelta, nsm, p, st)
+                         : launch_rmc_pairs_g<2, true, 0>(hs, a, scr, idelta, nsm, p, st);
   if (p.groups == 1)
-    return real ? launch_rmc_pairs_g<1, true>(hs, a, scr, idelta, nsm, p, st)
-                : launch_rmc_pairs_g<1, false>(hs, a, scr, idelta, nsm, p, st);
-  return real ? launch_rmc_pairs_g<2, true>(hs, a, scr, idelta, nsm, p, st)
-              : launch_rmc_pairs_g<2, false>(hs, a, scr, idelta, nsm, p, st);
+    return real ? launch_rmc_pairs_g<1, true, -1>(hs, a, scr, idelta, nsm, p, st)
+                : launch_rmc_pairs_g<1, false, -1>(hs, a, scr, idelta, nsm, p, st);
+  return real ? launch_rmc_pairs_g<2, true, -1>(hs, a, scr, idelta, nsm, p, st)
+              : launch_rmc_pairs_g<2, false, -1>(hs, a, scr, idelta, nsm, p, st);
 }
 
 extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {

@@ -28,6 +28,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "devsys.h"
 
 namespace q2d {
@@ -470,6 +472,12 @@ template <>
 struct RowLayout<double> {
   static constexpr int u2 = 0, u3 = 4, bf = 8, v2 = 12;
   static constexpr int gstride = 16, sstride = kPairRowSh, copy16 = 8;
+};
+// FP64 rows staged without u3 (systems that have none): u2 | backflow | v2, 96
+// bytes, 112 apart.
+struct RowLayoutNoU3 {
+  static constexpr int u2 = 0, bf = 4, u3 = 0, v2 = 8;
+  static constexpr int sstride = 14, copy16 = 6;
 };
 template <>
 struct RowLayout<float> {
@@ -1422,17 +1430,19 @@ __device__ inline void pair_rhok(const DevSys &S, const EvalSmem &m, int t, int 
 // Sync is the barrier of the NT threads (the CTA, or a named-barrier group
 // of a CTA that runs several walkers); tid is the thread's index among them.
 template <int NT, bool kSh, class R = double, class Sync = CtaSync, int LG = kGroup,
-          bool kJ = false>
+          bool kJ = false, int kU3 = -1>
 __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long &tph,
                                   double *pout, const R *rows, Sync sync = Sync(),
                                   int tid = threadIdx.x) {
-  using Lay = RowLayout<R>;
+  constexpr bool kF64 = sizeof(R) == 8;
+  using Lay = std::conditional_t<kF64 && kSh && kU3 == 0, RowLayoutNoU3, RowLayout<R>>;
   const int N = S.N;
   const int lane8 = tid & (LG - 1);
   const int per_round = NT / LG;
   const size_t NP = pair_count(N);
-  constexpr int RS = kSh ? Lay::sstride : Lay::gstride;
-  constexpr bool kF64 = sizeof(R) == 8;
+  constexpr int RS = kSh ? Lay::sstride : RowLayout<R>::gstride;
+  // kU3: u3 present (1) or absent (0) at compile time, or as the system says
+  const bool has_u3 = kU3 < 0 ? S.has_u3 != 0 : kU3 != 0;
   const Knots<R> K(S);
 
   // ---- pass A: pair sums of u2, the pair part of u3, u3 G vectors and S,
@@ -1459,7 +1469,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
         R rx, ry, r, byr, rem;
         double rxd = 0, ryd = 0, rd = 0, byrd = 0, remd = 0;
         int ind;
-        if (kF64 || S.has_bf || S.has_u3) {  // FP64 geometry (the u3 and backflow terms)
+        if (kF64 || S.has_bf || has_u3) {  // FP64 geometry (the u3 and backflow terms)
           pair_geom(S, Knots<double>(S), m.x, i, j, rxd, ryd, rd, byrd, ind, remd);
           rx = (R)rxd;
           ry = (R)ryd;
@@ -1480,7 +1490,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
           gy.add(dtr * ry);
           lap.add(ddt + dtr);
         }
-        if (S.has_u3) {
+        if (has_u3) {
           double t, dt, ddt;
           spline3<kSh>(Knots<double>(S), reinterpret_cast<const double *>(row + Lay::u3), remd, t,
                        dt, ddt);
@@ -1547,7 +1557,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
       }
     }
     double ltf_v = ltf.value(), gx_v = gx.value(), gy_v = gy.value(), lap_v = lap.value();
-    if (!kF64 && S.has_u3) {
+    if (!kF64 && has_u3) {
       ltf_v += ltf3.value();
       gx_v += gx3.value();
       gy_v += gy3.value();
@@ -1559,7 +1569,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
     const double lap_s = group_sum<LG>(lap_v);
     const double vp_s = group_sum<LG>(vp.value());
     double Gx_s = 0, Gy_s = 0, s3xx_s = 0, s3xy_s = 0, s3yy_s = 0;
-    if (S.has_u3) {
+    if (has_u3) {
       Gx_s = group_sum<LG>(Gx.value());
       Gy_s = group_sum<LG>(Gy.value());
       s3xx_s = group_sum<LG>(s3xx.value());
@@ -1587,7 +1597,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
       m.g[2 * i + 1] = gy_s;
       m.lap[i] = lap_s;
       m.vp[i] = vp_s;
-      if (S.has_u3) {
+      if (has_u3) {
         m.G3[2 * i] = Gx_s;
         m.G3[2 * i + 1] = Gy_s;
         m.S3[3 * i] = s3xx_s;
@@ -1628,7 +1638,7 @@ __device__ inline void eval_pairs(const DevSys &S, const EvalSmem &m, long long 
   phase_mark(S, PH_PAIRS, tph, tid == 0);
 
   // ---- pass B: u3 gradient and Laplacian from the G vectors (FP64).
-  if (S.has_u3) {
+  if (has_u3) {
     for (int base = 0; base < N; base += per_round) {
       int k = base + tid / LG;
       bool valid = k < N;
