@@ -113,8 +113,8 @@ __device__ __forceinline__ void f_store(const double (&acc)[kR][kT][2][2], doubl
 // and the step loop stays rolled; the pivot row reaches the other lanes
 // through shared memory. The inverse then goes to shared memory and F comes
 // from the FP64 tensor cores: 450 instructions per matrix of 29 where lanes
-// holding a row of the inverse and 8 columns of F took 3200 (0.177 ms per
-// 4096 walkers at 29 + 29). Both matrices have rows of LD doubles, columns
+// holding a row of the inverse and 8 columns of F took 3200. 0.15 ms per 4096
+// walkers at 29 + 29, bound by the chains of 12 warps per SM. Both matrices have rows of LD doubles, columns
 // XOR-swizzled by 4 (row mod 4): the fragments' half-warp reads (four rows,
 // four columns) and the lanes' column writes fall on distinct banks.
 constexpr int kRealWarps = 4;
@@ -245,9 +245,9 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs
 // one barrier: before it every warp publishes its best candidate row (key,
 // reciprocal, columns), after it every thread takes the best key's row. Bound
 // by shared-memory wavefronts and the step's latency chain: a pivot-row value
-// read once serves kR rows (one row per four lanes, every value used once,
-// kept the shared-memory pipe 61% and the FP64 pipe 15% busy: 0.29 ms for
-// 2048 matrices of 61, 3.5 ms for 768 of 161).
+// read once serves kR rows: 2.19 ms for 768 matrices of 161, 0.73 for 1024 of
+// 113, where one row per four lanes with every value used once (shared-memory
+// pipe 61%, FP64 pipe 15% busy) took 3.53 and 1.94.
 // Above 128 orbitals the last kS columns of a lane, which the registers of
 // one SM cannot hold, live in shared memory as a ring that the rotation
 // feeds from. When both spins have at most kRealFused orbitals the
@@ -647,58 +647,86 @@ __global__ void __launch_bounds__(kFThreads, 1) real_f_kernel(RealArgs a, int nw
 // F_a(k,j) F_c(j,k) (and D2_j on the diagonal) and the CTA sums them. Bound by
 // the FP64 pipe (one product of 256 FMAs per 16 cycles and sub-partition).
 //
-// kB: tiles per side of a warp's item. kB = 1 keeps every column resident
-// (spins of at most 61 orbitals) and takes both types of a tile pair in one
-// item; kB = 2 streams chunks of columns through two buffers, one type after
-// the other.
+// kB: tiles per side of a warp's item. kB = 1 keeps its columns resident: those
+// of both types, a tile pair's two types in one item, or (launch_s) those of
+// one type per CTA, up to about 96 orbitals; kB = 2 streams chunks of columns
+// through two buffers, one type after the other.
+// Measured on one B200: 29 + 29, 4096 walkers 0.25 ms (0.60 as 3 x 3 register
+// tiles of FMAs in the move's end); 161 polarised, 768 walkers 1.95 ms, 2.48
+// before the staging visited only the triangle rows of its chunk and the last
+// round's items were shared by several warps.
 __host__ __device__ inline int s_chunk(int n) {  // columns per chunk: two buffers in 176 KB
   const int c = (int)(88 * 1024 / (sizeof(double) * 3 * n)) / 4;
   return (c & 1 ? c : c - 1) * 4;
 }
 
-// Jacobian columns c0 .. c1-1 (padded numbering) of the n electrons j from
-// f0 on into dst[p][j][c - c0] (asynchronous 8-byte copies, zeros in the
-// padding): from row j of the triangle for i >= j (lanes on consecutive i),
-// from row i for i < j (lanes on consecutive j).
+// The three planes' entries at e of the triangle into shared address d
+// (asynchronous 8-byte copies).
+__device__ __forceinline__ void copy_entry(unsigned d, unsigned pl, const double *e, int jp) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(e) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + pl), "l"(e + jp) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + 2 * pl), "l"(e + 2 * jp) : "memory");
+}
+
+// The columns of one type (from column c0 of dst's first on, padded
+// numbering) of spin spn's electrons j into dst[p][j][c], zeros in the padding.
+// One pass over the triangle's rows r that hold them, lanes on consecutive
+// entries (r, c): of the spin's own type each goes to (j, i) = (r, c) and
+// (c, r); between the types to (r, c) or, for type 1's electrons, (c, r).
+__device__ inline void stage_type(const RealArgs &a, double *dst, int ld, const double *jg, int spn,
+                                  int type) {
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nw = blockDim.x >> 5;
+  const int n0 = a.np[0], N = a.N, n = spn ? a.np[1] : n0, f0 = spn ? n0 : 0;
+  const int i0 = type ? n0 : 0, ni = type ? a.np[1] : n0;
+  const bool own = spn == type;
+  const int rb = own ? f0 : 0, re = own ? f0 + n : n0, ce = own ? re : N;
+  const unsigned pl = 8 * n * ld, d = (unsigned)__cvta_generic_to_shared(dst);
+  for (int r = rb + warp; r < re; r += nw) {
+    const double *src = jg + jac_row(N, r);
+    const unsigned row = d + 8 * ((r - f0) * ld - i0), col = d + 8 * (r - i0 - f0 * ld);
+    for (int c = (own ? r : n0) + lane; c < ce; c += 32) {
+      if (own || !spn) copy_entry(row + 8 * c, pl, src + c, a.jp);
+      if (own ? c > r : spn) copy_entry(col + 8 * c * ld, pl, src + c, a.jp);
+    }
+  }
+  const int np = -ni & 3;
+  for (int e = t; e < n * np; e += blockDim.x) {
+    double *z = dst + e / np * ld + ni + e % np;
+    z[0] = z[n * ld] = z[2 * n * ld] = 0.0;
+  }
+}
+
+// Columns c0 .. c1-1 of one type: from row j of the triangle for i >= j (lanes
+// on consecutive i), from row i for i < j (lanes on consecutive j).
 __device__ inline void stage_cols(const RealArgs &a, double *dst, int ld, const double *jg, int f0,
                                   int n, int c0, int c1) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int n0 = a.np[0], n1 = a.np[1], pad0 = a.pad0, jp = a.jp, pl = n * ld;
-  for (int jl = warp; jl < n; jl += nw) {
-    const int j = f0 + jl;
+  const int n0 = a.np[0], shift = a.pad0 - n0, t1 = c0 >= a.pad0;
+  // electrons i0 .. i1-1; columns from i1 on are padding
+  const int i0 = t1 ? c0 - shift : c0, i1 = min(t1 ? c1 - shift : c1, t1 ? a.N : n0);
+  const unsigned pl = 8 * n * ld, d = (unsigned)__cvta_generic_to_shared(dst);
+  for (int j = f0 + warp; j < min(f0 + n, i1); j += nw) {
     const double *src = jg + jac_row(a.N, j);
-    double *d = dst + jl * ld - c0;
-    for (int c = c0 + lane; c < c1; c += 32) {
-      const int x = c < pad0 ? c : c - pad0, i = c < pad0 ? c : n0 + x;
-      if (x >= (c < pad0 ? n0 : n1)) {
-        d[c] = d[c + pl] = d[c + 2 * pl] = 0.0;
-      } else if (i >= j) {
-        const double *e = src + i;
-        cp_async8(d + c, e);
-        cp_async8(d + c + pl, e + jp);
-        cp_async8(d + c + 2 * pl, e + 2 * jp);
-      }
-    }
+    for (int i = max(j, i0) + lane; i < i1; i += 32)
+      copy_entry(d + 8 * ((j - f0) * ld + i - i0), pl, src + i, a.jp);
   }
-  for (int c = c0 + warp; c < c1; c += nw) {
-    const int x = c < pad0 ? c : c - pad0, i = c < pad0 ? c : n0 + x;
-    if (x >= (c < pad0 ? n0 : n1)) continue;
-    const double *src = jg + jac_row(a.N, i) + f0;
-    double *d = dst + (c - c0);
-    for (int jl = max(0, i + 1 - f0) + lane; jl < n; jl += 32) {
-      const double *e = src + jl;
-      double *q = d + jl * ld;
-      cp_async8(q, e);
-      cp_async8(q + pl, e + jp);
-      cp_async8(q + 2 * pl, e + 2 * jp);
-    }
+  for (int i = i0 + warp; i < i1; i += nw) {
+    const double *src = jg + jac_row(a.N, i);
+    const unsigned col = d + 8 * (i - i0);
+    for (int j = max(f0, i + 1) + lane; j < f0 + n; j += 32)
+      copy_entry(col + 8 * ((j - f0) * ld), pl, src + j, a.jp);
+  }
+  const int np = c1 - c0 - (i1 - i0);
+  for (int e = threadIdx.x; e < n * np; e += blockDim.x) {
+    double *z = dst + e / np * ld + (i1 - i0) + e % np;
+    z[0] = z[n * ld] = z[2 * n * ld] = 0.0;
   }
 }
 
 // Products of kB x kB tile pairs over the columns [k0, k1) of a buffer.
 template <int kB>
 __device__ __forceinline__ void s_products(double (&acc)[kB][kB][4][2], const double *buf, int ld,
-                                           int n, int tj, int tk, int k0, int k1) {
+                                           int n, int tj, int tk, int k0, int k1, int step = 4) {
   const int lane = threadIdx.x & 31, lg = lane >> 2, lt = lane & 3;
   const int pl = n * ld;
   const double *pj[kB], *pk[kB];
@@ -708,7 +736,7 @@ __device__ __forceinline__ void s_products(double (&acc)[kB][kB][4][2], const do
     pk[a] = buf + min(8 * (kB * tk + a) + lg, n - 1) * ld + lt;
   }
 #pragma unroll 2
-  for (int c = k0; c < k1; c += 4) {
+  for (int c = k0; c < k1; c += step) {
     double j[kB][3], k[kB][3];
 #pragma unroll
     for (int a = 0; a < kB; a++)
@@ -786,10 +814,12 @@ constexpr int kSMaxThreads = 768;  // kB = 1: at most 80 registers, 24 warps on 
 
 template <int kB>
 __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
-    real_s_kernel(RealArgs a, const DevSys *ds, int nw) {
+    real_s_kernel(RealArgs a, const DevSys *ds, int nw, int split) {
   extern __shared__ __align__(16) char smem[];
   pdl_wait();
-  const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
+  // split (kB = 1, two types): one CTA per type of the columns
+  const int item = blockIdx.x >> split, type = split ? blockIdx.x & 1 : 0;
+  const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
   if (w >= nw) return;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x, NW = nthr >> 5;
   const int nt = a.nt, n = spn ? a.np[1] : a.np[0], f0 = spn ? a.f0[1] : a.f0[0];
@@ -803,7 +833,10 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   auto mark = [&](int k) {
     if (timed) phase_mark(*ds, k, tph, t == 0);
   };
-  const int pad0 = a.pad0, cols = a.cols, n0 = a.np[0];
+  const int n0 = a.np[0];
+  // split: the type's columns in buffer numbering 0 .. cols-1
+  const int pad0 = type ? 0 : a.pad0;
+  const int cols = split ? (type ? a.cols - a.pad0 : a.pad0) : a.cols;
   const int ic = kB == 1 ? cols : s_chunk(n), ld = kB == 1 ? odd4(cols) : ic;
   const size_t bufd = (size_t)3 * n * ld;
   // kB = 2: chunks never span both types
@@ -824,7 +857,10 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   auto stage = [&](int ch, int buf) {
     int c0, c1;
     chunk(ch, &c0, &c1);
-    stage_cols(a, jac + buf * bufd, ld, base, f0, n, c0, c1);
+    if (kB == 1) {
+      stage_type(a, jac, ld, base, spn, type);
+      if (nt > 1 && !split) stage_type(a, jac + a.pad0, ld, base, spn, 1);
+    } else stage_cols(a, jac + buf * bufd, ld, base, f0, n, c0, c1);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   stage(0, 0);
@@ -860,23 +896,32 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
     drift(jac, 0, cols);
     // (tile pair, type) items in whole runs per warp: a tile pair whose types
     // fall to two warps is contracted by both
-    const int items = pairs * nt, i0 = items * warp / NW, i1 = items * (warp + 1) / NW;
+    const bool one = nt == 1 || split;
+    const int items = one ? pairs : 2 * pairs;
+    const int i0 = items * warp / NW, i1 = items * (warp + 1) / NW;
     for (int it = i0; it < i1;) {
-      const int tp = nt > 1 ? it >> 1 : it;
-      const bool first = nt == 1 || !(it & 1), second = nt > 1 && 2 * tp + 1 < i1;
+      const int tp = one ? it : it >> 1;
+      const bool first = one || !(it & 1), second = !one && 2 * tp + 1 < i1;
       int tj, tk;
       tile_pair(tp, &tj, &tk);
       double acc[2][1][1][4][2] = {};
-      if (first) s_products<1>(acc[0], jac, ld, n, tj, tk, 0, pad0);
+      if (first) s_products<1>(acc[0], jac, ld, n, tj, tk, 0, one ? cols : pad0);
       if (second) s_products<1>(acc[1], jac, ld, n, tj, tk, pad0, cols);
       s_contract<1, 2>(acc, FX, d2, n, tj, tk, lt);
-      it = (nt > 1 ? 2 * tp + 1 : tp) + 1;
+      it = (one ? tp : 2 * tp + 1) + 1;
+    }
+    if (type) {  // the sums are type 1's
+      lt[1] = lt[0];
+      lt[0] = 0.0;
     }
   } else {
     const int rounds = (pairs + NW - 1) / NW;
     for (int round = 0; round < rounds; round++) {
-      const int it = round * NW + warp;
-      const bool on = it < pairs;
+      // the last round's items are shared by ks warps each, which take every
+      // ks-th product step of a chunk (the contraction is linear in the sums)
+      const int left = min(pairs - round * NW, NW), ks = NW / left;
+      const int it = round * NW + warp % left, kq = warp / left;
+      const bool on = kq < ks;
       int tj = 0, tk = 0;
       if (on) tile_pair(it, &tj, &tk);
       double acc[1][kB][kB][4][2];
@@ -897,7 +942,7 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
         chunk(ch, &c0, &c1);
         const double *buf = jac + (seq & 1) * bufd;
         if (round == 0) drift(buf, c0, c1);
-        if (on) s_products<kB>(acc[0], buf, ld, n, tj, tk, 0, c1 - c0);
+        if (on) s_products<kB>(acc[0], buf, ld, n, tj, tk, 4 * kq, c1 - c0, 4 * ks);
         if (on && (ch + 1 == nch0 || ch + 1 == nch)) {
           double s = 0.0;
           s_contract<kB, 1>(acc, FX, d2, n, tj, tk, &s);
@@ -911,8 +956,8 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   // - sum_j f_j . L_j
   const double *o = a.scr + w * a.stride;
   for (int e = t; e < 2 * n; e += nthr) {
-    lt[0] -= fd[e] * __ldg(o + a.l_qbd + 2 * f0 + e);
-    if (nt > 1) lt[1] -= fd[e] * __ldg(o + a.l_sb + 2 * f0 + e);
+    if (!type) lt[0] -= fd[e] * __ldg(o + a.l_qbd + 2 * f0 + e);
+    if (split ? type : nt > 1) lt[1] -= fd[e] * __ldg(o + a.l_sb + 2 * f0 + e);
   }
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) {
@@ -924,7 +969,7 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
     red[2 * warp + 1] = lt[1];
   }
   __syncthreads();
-  if (t < 2) {
+  if (t < 2 && (!split || t == type)) {
     double s = 0.0;
     for (int q = 0; q < NW; q++) s += red[2 * q + t];
     out[2 * a.N + t] = s;
@@ -935,28 +980,36 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
 // Warps per CTA of the resident form, by the CTAs an SM's shared memory holds
 // (us with the orbital kernel, one B200: 13 + 13, 4096 walkers: 3 warps 109, 4
 // 117; 29 + 29: 4 443, 5 421, 6 413, 8 441; 37 + 37, 1001: 6 253, 8 244, 12 264;
-// 45 + 45, 1024: 8 374, 10 364, 12 384; 61 + 61: 12 768, 16 780, 20 749).
+// 45 + 45, 1024: 8 374, 10 364, 12 384; 61 + 61, a type per CTA: 8 749, 10 710, 12 698).
 int s_warps(int n, size_t smem) {
   const int ctas = 227 * 1024 / (int)(smem + 1024);
-  return ctas >= 8 ? 3 : ctas >= 5 ? 4 : ctas == 4 ? 6 : ctas == 3 || n <= 40 ? 8 : ctas == 2 ? 10 : 20;
+  return ctas >= 8 ? 3 : ctas >= 5 ? 4 : ctas == 4 ? 6 : ctas == 3 || n <= 40 ? 8 : ctas == 2 ? n <= 45 ? 10 : 12 : 20;
 }
 
 cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int nw,
                      cudaStream_t st) {
-  size_t d = 0;
-  for (int t = 0; t < hs.nt; t++) d = std::max(d, s_smem_doubles(hs.np[t], a.cols, true));
-  const bool resident = sizeof(double) * d <= 226 * 1024;
-  if (!resident) {
-    d = 0;
-    for (int t = 0; t < hs.nt; t++) d = std::max(d, s_smem_doubles(hs.np[t], a.cols, false));
-  }
-  const size_t sm = sizeof(double) * d;
+  auto doubles = [&](int cols, bool resident) {
+    size_t d = 0;
+    for (int t = 0; t < hs.nt; t++) d = std::max(d, s_smem_doubles(hs.np[t], cols, resident));
+    return sizeof(double) * d;
+  };
+  size_t sm = doubles(a.cols, true);
+  // One CTA per type of the columns where an SM would hold one CTA with both
+  // (or none): two or three then overlap staging and products (us with the
+  // orbital kernel, 1024 walkers: 49 + 49: 549 -> 483, 61 + 61: 742 -> 698, 81 + 45:
+  // 1757 -> 1387, 81 + 81: 2630 -> 2014, streamed before). Where two or more fit,
+  // F read twice costs more: 29 + 29: 403 -> 420, 37 + 37: 240 -> 246, 45 + 45:
+  // 359 -> 364.
+  const int split = hs.nt > 1 && 2 * (sm + 1024) > 227 * 1024;
+  if (split) sm = doubles(std::max(a.pad0, a.cols - a.pad0), true);
+  const bool resident = sm <= 226 * 1024;
+  if (!resident) sm = doubles(a.cols, false);
   const void *k = resident ? (const void *)real_s_kernel<1> : (const void *)real_s_kernel<2>;
   cudaError_t e = raise_smem_limit(k, sm);
   if (e != cudaSuccess) return e;
-  return resident ? launch_pdl(real_s_kernel<1>, nw * hs.nt, 32 * s_warps(hs.nmax, sm), sm, st, a,
-                               ds, nw)
-                  : launch_pdl(real_s_kernel<2>, nw * hs.nt, 512, sm, st, a, ds, nw);
+  return resident ? launch_pdl(real_s_kernel<1>, nw * hs.nt << split, 32 * s_warps(hs.nmax, sm),
+                               sm, st, a, ds, nw, split)
+                  : launch_pdl(real_s_kernel<2>, nw * hs.nt, 512, sm, st, a, ds, nw, 0);
 }
 
 template <int kL, int kR, int kC, int kS, int kMaxT, int kMB, bool kFused>

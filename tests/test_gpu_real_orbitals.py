@@ -67,6 +67,17 @@ def test_mixed_precision_step(q, tmp_path):
         assert _same(r[k], c[k], 1e-9), k
 
 
+@pytest.mark.parametrize("nu,nd", [(45, 45), (45, 47), (49, 31), (93, 69), (95, 67)])
+def test_columns_of_one_type_per_cta(q, tmp_path, nu, nd):
+    """Both sides of the sizes at which a Laplacian CTA takes one type's
+    columns, and at which they no longer fit and are streamed."""
+    s, x = _deck(q, tmp_path, nu, nd, backflow=(0.2, 3.0, 1.8))
+    (r, _), (c, _) = _step(q, s, x, 1), _step(q, s, x, 0)
+    assert _same(r["x"], c["x"], 1e-11)
+    for k in ("g", "h", "p"):
+        assert _same(r[k], c[k], 1e-9), k
+
+
 @pytest.mark.parametrize("nu,nd", [(13, 13), (25, 0), (37, 33), (61, 61)])
 def test_evaluation_equals_the_fused_kernel(q, tmp_path, nu, nd):
     """Evaluations on the handle's stream (through the move's kernels where the
