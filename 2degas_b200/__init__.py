@@ -311,23 +311,25 @@ class Handle:
         self._chk(self.lib.qmc2d_set_dmc_ecut(self.h, ecut))
 
     def set_launch(self, groups=0, stage=0):
-        """Pair-kernel launch choice: walker groups per CTA (1, 2; 0 default)
+        """Pair-kernel launch choice: walker groups per CTA (1, 2; 0 by size)
         and pair-row staging (0 when it fits, 1 never)."""
         self._chk(self.lib.qmc2d_set_launch(self.h, groups, stage))
 
     def set_inversion(self, layout):
-        """0: register-resident Gauss-Jordan over every warp (default); 1: one
-        warp per spin in shared memory; 2: panel-blocked."""
+        """0 (default): real orbitals where the deck allows them, else the
+        register-resident Gauss-Jordan over every warp; 1: one warp per spin
+        in shared memory; 2: panel-blocked."""
         self._chk(self.lib.qmc2d_set_inversion(self.h, layout))
 
     def set_pair_lanes(self, lanes):
-        """Lanes per particle of the pair passes: 4, 8 or 16 (0: the default, 8)."""
+        """Lanes per particle of the pair passes: 4, 8 or 16 (0: the default, by N)."""
         self._chk(self.lib.qmc2d_set_pair_lanes(self.h, lanes))
 
     def set_move_inversion(self, mode):
-        """Orbitals and inversion of a move in their own kernel before the move
-        kernel: 1 when the population is large enough (default), 2 whenever it
-        fits, 0 never (inside the move kernel)."""
+        """1 (default): real orbitals where the deck allows them, else orbitals
+        and inversion of a move in their own kernel when the population is
+        large enough; 2: complex orbitals, in their own kernel whenever they
+        fit; 0: complex, inside the move kernel."""
         self._chk(self.lib.qmc2d_set_move_inversion(self.h, mode))
 
     def set_autotune_scope(self, mask):

@@ -478,7 +478,8 @@ extern "C" int qmc2d_set_pair_lanes(qmc2d_handle *h, int lanes) {
 
 extern "C" int qmc2d_get_pair_lanes(qmc2d_handle *h, int *lanes) {
   if (!h || !lanes) return QMC2D_ERR_ARG;
-  *lanes = h->hs.tune_lanes == 4 || h->hs.tune_lanes == 16 ? h->hs.tune_lanes : 8;
+  // (the lanes do not depend on the shared memory, the population or the route)
+  *lanes = q2d::pair_launch(h->hs, std::max(1, h->nw), h->nsm, 232448, false).lanes;
   return QMC2D_OK;
 }
 

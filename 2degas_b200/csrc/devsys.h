@@ -51,11 +51,11 @@ struct DevSys {
   // and v2 pair terms in FP32 with compensated sums read out in FP64.
   int pair_f32;
   // Launch choices of the pair kernel (host side, qmc2d_autotune): walker
-  // groups per CTA (0: the default, 2) and the staging of the pair rows in
-  // shared memory (0: when they fit, 1: never).
+  // groups per CTA (0: by the population and N, pair_launch) and the staging
+  // of the pair rows in shared memory (0: when they fit, 1: never).
   int tune_groups, tune_stage;
   // Lanes per particle in the pair kernel's two passes (qmc2d_set_pair_lanes,
-  // also timed by qmc2d_autotune): 4, 8 or 16 (0: the default, 8).
+  // also timed by qmc2d_autotune): 4, 8 or 16 (0: by N, pair_launch).
   int tune_lanes;
   // Inversion layout of the determinant section (qmc2d_set_inversion):
   // 0 the register-resident Gauss-Jordan over every warp (4 warps per

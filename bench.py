@@ -10,8 +10,9 @@ half-space k vectors), FP64. Synthetic: tables written by
 Philox stream, then equilibrated by VMC.
 
 One step = one DMC generation over the whole population (4096
-walker-moves: pairs_kernel, move_kernel, branch, gather). `value` times the device work with CUDA events on the
-library's stream (inputs resident in HBM, L2 flushed between steps);
+walker-moves: pairs_kernel, real_det_warp_kernel, real_s_kernel,
+move_real_kernel, branch, gather). `value` times the device work with CUDA
+events on the library's stream (inputs resident in HBM, L2 flushed between steps);
 `e2e` times the same steps through the public C-ABI with the walker records
 copied from and to pinned host memory every step (qmc2d_population_load_async:
 the records other than x and g arrive while the pair kernel runs).
@@ -47,28 +48,27 @@ import numpy as np  # noqa: E402
 CONFIG = "dmc_bf_n58_rs5"
 METRIC = "walker-moves/sec (DMC with backflow, N=58 r_s=5, 4096 walkers)"
 UNIT = "walker-moves/s"
-# DRAM bytes read per walker by one pairs_kernel + orb_inv_kernel +
-# move_kernel generation, from the ncu capture summarised in
-# profiles/move_kernels_dmc_bf_n58_444w.md (444 walkers, one wave of the
-# move kernel; scaled linearly: the walker records and the move scratch,
-# read cold in ncu's replays), plus the move scratch block the pair and
-# orbital kernels write, which reaches DRAM at 4096 walkers (the blocks
-# exceed L2) though not in the 444-walker capture.
-MOVE_DRAM_READ_PER_WALKER = (1.114624e6 + 0.526080e6 + 49.427200e6) / 444
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum of pairs_kernel + orb_inv_kernel + move_kernel "
-                  "(444 walkers) x walkers/444, + the move scratch written per walker")
+# DRAM bytes read per walker by one generation's pairs_kernel,
+# real_det_warp_kernel, real_s_kernel and move_real_kernel, from the ncu
+# capture summarised in profiles/real_orbital_kernels_dmc_bf_n58_1184w.md (1184
+# walkers; scaled linearly: the walker records and the move scratch, read cold
+# in ncu's replays), plus the move scratch block the kernels write, which
+# reaches DRAM at 4096 walkers (the blocks exceed L2).
+MOVE_DRAM_READ_PER_WALKER = (2.358528e6 + 2.234880e6 + 84.760064e6 + 14.224896e6) / 1184
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum of pairs_kernel + real_det_warp_kernel + real_s_kernel "
+                  "+ move_real_kernel (1184 walkers) x walkers/1184, + the move scratch written "
+                  "per walker")
 
 
 def move_scratch_bytes(N, nk, ns=()):
-    """Bytes of one walker's move scratch block (MoveScratch, backflow; with
-    ns, the spins' orbital counts, the orbitals-and-inversion region when
-    every spin has at most 32 orbitals)."""
-    pair = (14 * N + 3 + 4 * max(nk, 1) + 3) & ~3
-    end = pair + 3 * (N * (N - 1) // 2)
-    if ns and max(ns) <= 32:
-        end = (end + 1) & ~1
-        end += sum((2 * n * n + 2 * n * (n | 1) + 2 * n + 2 + 1) & ~1 for n in ns)
-    return 8 * ((end + 31) & ~31)
+    """Bytes a walker's move writes to its scratch over real orbitals
+    (MoveScratch and RealLayout): the per-particle sums and rho_k, the
+    Jacobian blocks of the pairs i <= j, and per spin of n orbitals F_x, F_y,
+    ln|det|, the singular flag, D2, and the drift and Laplacian shares."""
+    end = (14 * N + 3 + 4 * max(nk, 1) + 3) & ~3
+    end += 3 * (N * (N + 1) // 2)
+    end += sum(2 * n * n + 2 + 3 * n + 2 * N + 2 for n in ns)
+    return 8 * end
 
 
 def flops_per_sweep(N, ns, K):
@@ -83,6 +83,21 @@ def flops_per_sweep(N, ns, K):
     for n in ns:
         f += n * (26 * n + 60 * (N - 1) + 16 * n * n) + 25 * n * n
     return float(f + 60 * N * (N - 1) // 2 + 7 * N * K)
+
+
+def real_flops_per_move(N, ns, K, u3, backflow):
+    """As flops_per_move, over real orbitals (the route of Gamma-point decks):
+    per spin of n orbitals the real inverse 2 n^3 and, with backflow, F_x and
+    F_y 4 n^3, the symmetric S = J J^T 8 N n^2 and 13 n^2 for its contraction
+    with F; the rest as there."""
+    P = N * (N - 1) // 2
+    f = P * (16 + 32 + 12 + 110 * u3 + 80 * backflow) + 7 * N * K
+    for n in ns:
+        if backflow:
+            f += 6 * n ** 3 + 8 * N * n * n + 66 * n * n + 44 * N * n
+        else:
+            f += 2 * n ** 3 + 45 * n * n
+    return float(f)
 
 
 def flops_per_move(N, ns, K, u3, backflow):
@@ -484,17 +499,20 @@ def b200_arm(args, rank, world, local_rank):
     line = None
     if rank == 0:
         K = sysobj.s.nk
-        fpm = flops_per_move(N, ns, K, 0, 1)
-        # one walker-move of the population = one pairs_kernel, one
-        # orb_inv_kernel (where it applies) and one move_kernel launch; the
-        # roofline covers them all
+        # split orbital kernels with the default layout: the real-orbital route
+        real = oi_n > 0 and h.get_launch()[2] == 0
+        fpm = (real_flops_per_move if real else flops_per_move)(N, ns, K, 0, 1)
+        # one walker-move of the population = one pair kernel, the orbital
+        # kernels (one timing scope) and one end-of-move launch; the roofline
+        # covers them all
         achieved = fpm * nw / ((move_ms + pair_ms + oi_ms) / max(move_n, 1) * 1e-3) / 1e12
         peak = fp64_peak_tflops(torch)
         cpu = None
         if world == 1 and not args.no_cpu:
             rate, cores, sample = cpu_rate(d, args.cpu_seconds, rs=rs)
             cpu = {"value": rate, "unit": UNIT, "cores": cores, "kind": "port", "sample": sample}
-        launches = pair_n + oi_n + move_n + br_n + ga_n
+        # one orbital launch scope is two kernels (orbitals and F, then S)
+        launches = pair_n + 2 * oi_n + move_n + br_n + ga_n
         metric, config = workload_desc(args, world)
         line = {
             "metric": metric,
@@ -514,9 +532,10 @@ def b200_arm(args, rank, world, local_rank):
                          "traffic": ((MOVE_DRAM_READ_PER_WALKER + move_scratch_bytes(N, K, ns)) * nw
                                      if headline else None),
                          "traffic_source": TRAFFIC_SOURCE if headline else None,
-                         "kernel": ("pairs_kernel + orb_inv_kernel + move_kernel" if oi_n
+                         "kernel": ("pairs_kernel + real_det_warp_kernel + real_s_kernel + move_real_kernel" if oi_n
                                     else "pairs_kernel + move_kernel"),
                          "flops_per_move": fpm,
+                         "reference_flops_per_move": flops_per_move(N, ns, K, 0, 1),
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64)"},
             "cpu_baseline": cpu,
             "gpu_launches": launches,
@@ -706,7 +725,7 @@ def config_arm(args, rank, world, local_rank):
 
         def step():
             h.rmc(1)
-        kernels = (capi.KERNEL_PAIRS, capi.KERNEL_RMC)
+        kernels = (capi.KERNEL_PAIRS, capi.KERNEL_ORB_INV, capi.KERNEL_RMC)
     stream = torch.cuda.ExternalStream(h.stream())
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
     for _ in range(args.warmup):
@@ -790,8 +809,11 @@ def config_arm(args, rank, world, local_rank):
         # config 0's deck carries an eta = 0 backflow table (the reference
         # builds its determinant only in the backflow routine): counted as
         # the plain Slater-Jastrow algorithm it is
+        terms = (0, 0) if vmc else (1, 1)  # u3, backflow
+        # split orbital kernels: the real-orbital route
         fpm = (flops_per_sweep(N, ns, K) if vmc and args.single else
-               flops_per_move(N, ns, K, 0 if vmc else 1, 0 if vmc else 1))
+               real_flops_per_move(N, ns, K, *terms) if kms[capi.KERNEL_ORB_INV][1] else
+               flops_per_move(N, ns, K, *terms))
         kern_ms = sum(kms[k][0] for k in kernels)
         n_launch = max(kms[kernels[-1]][1], 1)
         achieved = fpm * nw * nw_moves / (kern_ms / n_launch * 1e-3) / 1e12
@@ -814,9 +836,10 @@ def config_arm(args, rank, world, local_rank):
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                          "kernel": ("single_kernel" if vmc and args.single else
-                                    "pairs_kernel + move_kernel" if vmc else
-                                    "rmc_pairs_kernel + rmc_det_kernel"),
+                                    "pair kernel + orbital kernels + end of the move" if vmc
+                                    else "rmc_pairs_kernel + orbital kernels + rmc_real_kernel"),
                          "flops_per_move": fpm,
+                         "reference_flops_per_move": flops_per_move(N, ns, K, *terms),
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64)"},
             "cpu_baseline": cpu,
             "gpu_launches": sum(kms[k][1] for k in kernels),

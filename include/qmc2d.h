@@ -219,9 +219,10 @@ int qmc2d_set_precision(qmc2d_handle *h, int precision);
 int qmc2d_set_dmc_ecut(qmc2d_handle *h, double ecut);
 
 /* Launch choices of the pair kernel (the proposal and pair passes of a
- * move): walker groups per CTA (1 or 2; 0 = the default, 2) and whether the
- * pair rows are staged in shared memory (stage 0: when they fit; 1: never,
- * read from global memory). Every choice computes the same values.
+ * move): walker groups per CTA (1 or 2; 0 = the default, by the population
+ * and N) and whether the pair rows are staged in shared memory (stage 0: when
+ * they fit and, with groups 0, when it pays; 1: never, read from global
+ * memory). Every choice computes the same values.
  * qmc2d_autotune times the four choices on the handle's current population
  * (three launches each after a warm-up; the population is not changed),
  * keeps the fastest and returns it with its time per launch. The reference
@@ -229,7 +230,9 @@ int qmc2d_set_dmc_ecut(qmc2d_handle *h, double ecut);
 int qmc2d_set_launch(qmc2d_handle *h, int groups, int stage);
 /* Inversion layout of the determinant section (compute_properties, VMC,
  * DMC, reptation) for determinants held in shared memory: 0 (the default)
- * the register-resident Gauss-Jordan over every warp of the CTA, 1 one warp
+ * real orbitals where the deck allows them (Gamma point, an odd number of
+ * plane waves per spin: orbitals, inverse and derivative matrices in kernels
+ * of their own), else the register-resident Gauss-Jordan over every warp of the CTA, 1 one warp
  * per spin in shared memory with rho_k on the other warps, 2 blocks of
  * eight pivot steps whose panels one warp factors in registers while the
  * spin's other warps wait for the block update (spins of at most 32
@@ -238,23 +241,28 @@ int qmc2d_set_launch(qmc2d_handle *h, int groups, int stage);
  * values up to round-off. The reference has no counterpart. */
 int qmc2d_set_inversion(qmc2d_handle *h, int layout);
 /* Lanes per particle in the pair kernel's two pair passes: 4, 8 or 16
- * (0: the default, 8). Each particle's sums over its partners are split
- * over that many lanes and meet in a fixed shuffle order, so a choice
- * other than 8 changes the sums' rounding (round-off only). qmc2d_autotune
+ * (0: the default, 4 or 8 by N; 8 in mixed precision). Each particle's sums
+ * over its partners are split over that many lanes and meet in a fixed
+ * shuffle order, so another choice changes the sums' rounding (round-off
+ * only). qmc2d_autotune
  * times the three after the groups and staging; qmc2d_get_pair_lanes
  * reports the choice in force. */
 int qmc2d_set_pair_lanes(qmc2d_handle *h, int lanes);
 int qmc2d_get_pair_lanes(qmc2d_handle *h, int *lanes);
-/* Where the moves (VMC, DMC) invert their determinants. The batched form
+/* Where the moves (VMC, DMC, reptation) form and invert their determinants.
+ * With mode 1 (the default), decks that allow real orbitals
+ * (qmc2d_set_inversion) take them, except up to 128 walkers of one spin of at
+ * most 29 electrons; modes 0 and 2 and all other decks take the complex
+ * kernels. Of those, the batched form
  * runs the orbitals and their inversion in a kernel of its own between the
  * pair kernel and the move kernel, one warp per spin matrix, for spins of
  * at most 32 orbitals held in shared memory; otherwise the move kernel
- * inverts with the inversion layout in force. mode 1 (the default): batched
- * when the population gives at least 10 spin matrices per SM (3 for a
+ * inverts with the inversion layout in force (reptation always does). mode 1:
+ * batched when the population gives at least 10 spin matrices per SM (3 for a
  * single spin): a fuller GPU hides the
  * pivot chains, small populations finish sooner inside the move kernel;
  * 2: batched whenever it fits; 0: never. Both pivot as zgefa does
- * and agree to round-off. get reports whether the next move is batched. The
+ * and agree to round-off. get reports whether the next complex move is batched. The
  * reference has no counterpart. */
 int qmc2d_set_move_inversion(qmc2d_handle *h, int mode);
 int qmc2d_get_move_inversion(qmc2d_handle *h, int *batched);
@@ -627,7 +635,9 @@ enum qmc2d_kernel {
   QMC2D_KERNEL_RMC = 4,     /* reptation moves */
   QMC2D_KERNEL_PAIRS = 5,   /* proposal + pair passes of a VMC/DMC move */
   QMC2D_KERNEL_SINGLE = 6,  /* single-electron VMC sweeps (qmc2d_vmc_single) */
-  QMC2D_KERNEL_ORB_INV = 7, /* orbitals and their inversion of a move (orb_inv_kernel) */
+  QMC2D_KERNEL_ORB_INV = 7, /* orbitals and their inversion of a move (orb_inv_kernel), or
+                               the real-orbital kernels of a move or bead growth (two or
+                               three launches, timed together) */
   QMC2D_NKERNELS = 8
 };
 /* The handle's CUDA stream (a cudaStream_t) so callers can order work and
