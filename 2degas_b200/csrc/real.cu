@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs
 // one barrier: before it every warp publishes its best candidate row (key,
 // reciprocal, columns), after it every thread takes the best key's row. Bound
 // by shared-memory wavefronts and the step's latency chain: a pivot-row value
-// read once serves kR rows: 2.19 ms for 768 matrices of 161, 0.73 for 1024 of
+// read once serves kR rows: 2.19 ms for 768 matrices of 161, 0.73 for 768 of
 // 113, where one row per four lanes with every value used once (shared-memory
 // pipe 61%, FP64 pipe 15% busy) took 3.53 and 1.94.
 // Above 128 orbitals the last kS columns of a lane, which the registers of
@@ -651,8 +651,8 @@ __global__ void __launch_bounds__(kFThreads, 1) real_f_kernel(RealArgs a, int nw
 // of both types, a tile pair's two types in one item, or (launch_s) those of
 // one type per CTA, up to about 96 orbitals; kB = 2 streams chunks of columns
 // through two buffers, one type after the other.
-// Measured on one B200: 29 + 29, 4096 walkers 0.25 ms (0.60 as 3 x 3 register
-// tiles of FMAs in the move's end); 161 polarised, 768 walkers 1.95 ms, 2.48
+// Measured on one B200: 29 + 29, 4096 walkers 0.25 ms (0.60 with the
+// move's end, as 3 x 3 register tiles of FMAs there); 161 polarised, 768 walkers 1.95 ms, 2.48
 // before the staging visited only the triangle rows of its chunk and the last
 // round's items were shared by several warps.
 __host__ __device__ inline int s_chunk(int n) {  // columns per chunk: two buffers in 176 KB
