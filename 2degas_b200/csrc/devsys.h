@@ -89,6 +89,10 @@ struct DevSys {
   // pair kernels form rho_k from per-particle tables of exp(2 pi i p x / L)
   // instead of a sincos per (k, particle).
   int rk_lat, rk_p1, rk_p2;
+  // The sums of every tile of 8 x 8 products of those tables have a place in a
+  // walker group's shared memory (set by each launch, pair_plan); 0: one tile
+  // after the other.
+  int rk_whole;
   // Determinants too large for one CTA's shared memory (gmat = 1): the
   // orbital, inversion, F and cross-term matrices of walker (CTA) b live at
   // gmat_base + b * gmat_stride (doubles) in global memory; everything

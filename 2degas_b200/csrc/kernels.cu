@@ -997,6 +997,9 @@ static size_t pair_rows_bytes(const DevSys &hs, bool no_u3 = false) {
   return row * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
 }
 
+// Shared memory of the launch's groups and rows together.
+static size_t pair_smem_limit(int optin) { return (size_t)optin - 1024; }
+
 // Groups, staging and lanes compute the same pair terms; groups and staging
 // leave every bit, the lanes the order of a particle's partial sums.
 //   groups and staging (FP64, us per launch, 148 SMs): one group per CTA
@@ -1014,7 +1017,7 @@ static size_t pair_rows_bytes(const DevSys &hs, bool no_u3 = false) {
 PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3) {
   PairLaunch p{hs.tune_groups, hs.tune_stage != 1, hs.tune_lanes};
   const size_t grp = pair_group_bytes(hs), rows = pair_rows_bytes(hs, no_u3),
-               lim = (size_t)optin - 1024;
+               lim = pair_smem_limit(optin);
   if (p.groups == 0) {
     if (2 * grp + rows > lim || nw <= nsm) {
       p.groups = 1;
@@ -1036,6 +1039,26 @@ PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3)
       if (c4 < c8) p.lanes = 4;
     }
   }
+  return p;
+}
+
+// The sums of rho_k's tiles get a place of their own where it costs the launch
+// neither a walker group, nor the staged rows, nor a second CTA on the SM: N =
+// 58, 4096 walkers 217 us, 224 with one tile after the other (N = 26: 110 and
+// 119). Where it does, 45 + 45 with u3, 1024 walkers, took 306 us in one group
+// and 230 in two with the tiles in turn; long k lists would not fit at all.
+PairLaunch pair_plan(DevSys &s, int nw, int nsm, int optin, bool no_u3) {
+  s.rk_whole = 0;
+  const PairLaunch p = pair_launch(s, nw, nsm, optin, no_u3);
+  if (!s.rk_lat) return p;
+  const size_t rows = p.stage ? pair_rows_bytes(s, no_u3) : 0, lim = pair_smem_limit(optin);
+  const size_t in_turn = p.groups * pair_group_bytes(s) + rows;
+  s.rk_whole = 1;
+  const PairLaunch w = pair_launch(s, nw, nsm, optin, no_u3);
+  const size_t whole = p.groups * pair_group_bytes(s) + rows;
+  if (w.groups != p.groups || w.stage != p.stage || whole > lim ||
+      (p.groups == 1 && 2 * whole > lim && 2 * in_turn <= lim))
+    s.rk_whole = 0;
   return p;
 }
 
@@ -1071,9 +1094,9 @@ static cudaError_t launch_pairs_g(const DevSys &hs, DevPop pop, const MoveArgs &
 }
 
 template <class R, bool kJ>
-static cudaError_t launch_pairs_r(const DevSys &hs, DevPop pop, const MoveArgs &a,
-                                  cudaStream_t st, int nsm, int optin, const double *xe) {
-  const PairLaunch p = pair_launch(hs, a.nw, nsm, optin, kJ && sizeof(R) == 8 && !hs.has_u3);
+static cudaError_t launch_pairs_r(DevSys hs, DevPop pop, const MoveArgs &a, cudaStream_t st,
+                                  int nsm, int optin, const double *xe) {
+  const PairLaunch p = pair_plan(hs, a.nw, nsm, optin, kJ && sizeof(R) == 8 && !hs.has_u3);
   switch (p.lanes) {
     case 4: return launch_pairs_g<R, 4, kJ>(hs, pop, a, st, nsm, p, xe);
     case 16: return launch_pairs_g<R, 16, kJ>(hs, pop, a, st, nsm, p, xe);

@@ -62,6 +62,8 @@ struct PairLaunch {
 };
 // no_u3: the kernel for systems without u3 (its staged rows are smaller).
 PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3);
+// The same, with hs.rk_whole set for that launch.
+PairLaunch pair_plan(DevSys &hs, int nw, int nsm, int optin, bool no_u3);
 
 // Raise (never lower) kernel fn's dynamic shared-memory limit on the current
 // device to bytes; safe to call from several host threads.

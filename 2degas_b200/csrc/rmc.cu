@@ -1048,7 +1048,7 @@ static cudaError_t launch_rmc_pairs(const q2d::DevSys &hs0, const q2d::RmcArgs &
       cudaSuccess)
     return e;
   const bool no_u3 = real && !hs.has_u3;
-  const q2d::PairLaunch p = q2d::pair_launch(hs, a.nrep, nsm, optin, no_u3);
+  const q2d::PairLaunch p = q2d::pair_plan(hs, a.nrep, nsm, optin, no_u3);
   if (no_u3)
     return p.groups == 1 ? launch_rmc_pairs_g<1, true, 0>(hs, a, scr, idelta, nsm, p, st)
                          : launch_rmc_pairs_g<2, true, 0>(hs, a, scr, idelta, nsm, p, st);

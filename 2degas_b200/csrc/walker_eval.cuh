@@ -250,9 +250,10 @@ __host__ __device__ inline size_t pair_carve(const DevSys &s, char *base, EvalSm
   t.rhok = (double *)take(sizeof(double) * 2 * (s.nk > 0 ? s.nk : 1) * 2);
   t.red = (double *)take(sizeof(double) * nthreads);
   t.rkt = s.rk_lat ? (double2 *)take(sizeof(double2) * (s.rk_p1 + s.rk_p2 + 2) * N) : nullptr;
-  t.rks = s.rk_lat ? (double *)take(sizeof(double) * 4 * s.nt * 64 * ((s.rk_p1 + 8) >> 3) *
-                                    ((s.rk_p2 + 8) >> 3))
-                   : nullptr;
+  t.rks = s.rk_lat && s.rk_whole
+              ? (double *)take(sizeof(double) * 256 * s.nt * ((s.rk_p1 + 8) >> 3) *
+                               ((s.rk_p2 + 8) >> 3))
+              : nullptr;
   if (m) *m = t;
   return off;
 }
@@ -1327,6 +1328,51 @@ __device__ inline void compute_rhok(const DevSys &S, const EvalSmem &m, int t, i
   }
 }
 
+// The end of compute_rhok_lattice where the group's shared memory has no place
+// for every tile's sums (DevSys::rk_whole): the tiles one after the other, each
+// through the reduction buffer, the same products in the same order. A
+// function of its own: inlined, the pair kernels lost 1%.
+template <class Sync>
+__device__ __noinline__ void rhok_tiles(const DevSys &S, const double2 *rkt, double *red,
+                                        double *rhok, int t, int nthr, Sync sync) {
+  static_assert(kThreads == 4 * 64, "a tile's four products fill the reduction buffer");
+  const int N = S.N, P1 = S.rk_p1, P2 = S.rk_p2, T1 = (P1 + 8) >> 3, T2 = (P2 + 8) >> 3;
+  const double *xd = reinterpret_cast<const double *>(rkt), *yd = xd + 2 * (size_t)(P1 + 1) * N;
+  const double c1 = S.el[0] * 0.15915494309189535, c2 = S.el[1] * 0.15915494309189535;
+  const int warp = t >> 5, lane = t & 31, lg = lane >> 2, lt = lane & 3;
+  for (int tile = 0; tile < T1 * T2 * S.nt; tile++) {
+    const int ty = tile / (T1 * T2), pq = tile % (T1 * T2);
+    if (S.irhok[ty] == 0) continue;
+    const int p0 = 8 * (pq / T2), q0 = 8 * (pq % T2), f0 = S.ipfrst[ty], n = S.np[ty];
+    for (int pr = warp; pr < 4; pr += nthr >> 5) {
+      // RR, II, RI, IR: component of X, component of Y
+      const double *xa = xd + 2 * ((size_t)min(p0 + lg, P1) * N + f0) + (pr == 1 || pr == 3);
+      const double *ya = yd + 2 * ((size_t)min(q0 + lg, P2) * N + f0) + (pr == 1 || pr == 2);
+      double acc[2] = {0.0, 0.0};
+      for (int k0 = 0; k0 < n; k0 += 4) {
+        const int k = k0 + lt;
+        dmma_m8n8k4(acc, k < n ? xa[2 * k] : 0.0, k < n ? ya[2 * k] : 0.0);
+      }
+      double *o = red + 64 * pr + 8 * lg + 2 * lt;
+      o[0] = acc[0];
+      o[1] = acc[1];
+    }
+    sync();
+    for (int k = t; k < S.nk; k += nthr) {
+      const int n1 = __double2int_rn(__ldg(S.kvec + 2 * k) * c1);
+      const int n2 = __double2int_rn(__ldg(S.kvec + 2 * k + 1) * c2);
+      const int p = abs(n1) - p0, q = abs(n2) - q0;
+      if ((p | q) & ~7) continue;
+      const double *r = red + 8 * p + q;
+      const double s1 = n1 < 0 ? -1.0 : 1.0, s2 = n2 < 0 ? -1.0 : 1.0;
+      const int slot = S.irhok[ty] - 1;
+      rhok[2 * (slot * S.nk + k)] = r[0] - s1 * s2 * r[64];
+      rhok[2 * (slot * S.nk + k) + 1] = s2 * r[128] + s1 * r[192];
+    }
+    sync();  // the buffer is the next tile's
+  }
+}
+
 // rho_k of the pair kernels when every k vector is on the reciprocal lattice
 // (DevSys::rk_lat): with k = 2 pi (n1 / Lx, n2 / Ly), exp(i k.x) =
 // X_{n1}(x) Y_{n2}(y), X_p(x) = exp(2 pi i p x / Lx), and each particle's
@@ -1357,8 +1403,9 @@ __device__ inline void compute_rhok_lattice(const DevSys &S, const EvalSmem &m, 
     }
   }
   sync();
-  const int T1 = (P1 + 8) >> 3, T2 = (P2 + 8) >> 3, ldt = 8 * T2, tab = 8 * T1 * ldt;
   double *R = m.rks;  // [type][RR, II, RI, IR][p][q]
+  if (!R) return rhok_tiles(S, m.rkt, m.red, m.rhok, t, nthr, sync);
+  const int T1 = (P1 + 8) >> 3, T2 = (P2 + 8) >> 3, ldt = 8 * T2, tab = 8 * T1 * ldt;
   {
     const int warp = t >> 5, lane = t & 31, lg = lane >> 2, lt = lane & 3;
     const double *xd = reinterpret_cast<const double *>(X), *yd = reinterpret_cast<const double *>(Y);
