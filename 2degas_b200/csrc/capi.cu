@@ -519,6 +519,17 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   }
   CK(cudaSetDevice(h->device));
   CK(join_side(h));
+  // the inversion layout in scope: real orbitals, which have none, where the
+  // moves would take them with layout 0
+  bool layouts = h->tune_scope & 4;
+  if (layouts && h->hs.real_orb) {
+    const int inv_in = h->hs.tune_inv;
+    h->hs.tune_inv = 0;
+    if (move_real(h, h->nw))
+      layouts = false;
+    else
+      h->hs.tune_inv = inv_in;
+  }
   q2d::MoveArgs a{};
   a.nw = h->nw;
   a.real = move_real(h, h->nw) ? 1 : 0;
@@ -535,9 +546,8 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   double best = 1e300;
-  int bg = h->hs.tune_groups ? h->hs.tune_groups : 2, bs = h->hs.tune_stage;
-  const int lanes_in = h->hs.tune_lanes;
-  h->hs.tune_lanes = 8;  // the groups and staging are compared at the default lanes
+  // groups and staging, compared at the lanes in force
+  int bg = h->hs.tune_groups, bs = h->hs.tune_stage;
   for (const auto &v : var) {
     if (!(h->tune_scope & 1)) break;
     h->hs.tune_groups = v[0];
@@ -557,7 +567,6 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   }
   h->hs.tune_groups = bg;
   h->hs.tune_stage = bs;
-  h->hs.tune_lanes = lanes_in;
   // lanes per particle of the pair passes, with the chosen groups and staging
   // (8 first: the other two must beat it)
   if (h->tune_scope & 2) {
@@ -583,9 +592,7 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   // inversion layout of the determinant section, timed on the evaluation
   // kernel over the population's configurations (into the staging buffers;
   // the population is not changed)
-  if ((h->tune_scope & 4) && h->hs.real_orb) {
-    h->hs.tune_inv = 0;  // the real-orbital route, which has no layouts
-  } else if ((h->tune_scope & 4) && h->hs.has_bf && !h->hs.gmat) {
+  if (layouts && h->hs.has_bf && !h->hs.gmat) {
     double best_inv = 1e300;
     int bi = 0;
     for (int layout = 0; layout < 3; layout++) {
@@ -614,7 +621,9 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
   CK(cudaStreamSynchronize(h->stream));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (groups) *groups = bg;
+  // groups left to the size: those of this population
+  const bool no_u3 = a.real && !h->hs.pair_f32 && !h->hs.has_u3;
+  if (groups) *groups = q2d::pair_launch(h->hs, h->nw, h->nsm, 232448, no_u3).groups;
   if (stage) *stage = bs;
   if (ms) *ms = best;
   return QMC2D_OK;

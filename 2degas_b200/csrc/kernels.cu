@@ -168,8 +168,8 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 // (stage_rows), made once per launch and shared by the groups; random rows
 // in global memory cost an L1 tag lookup per lane, shared memory a few bank
 // wavefronts per warp. G and the staging are the launch choices that
-// qmc2d_autotune times (DevSys::tune_groups, tune_stage); by default G = 2
-// with the rows staged. Both caps keep 128 registers a thread (G = 2: one
+// qmc2d_autotune times (DevSys::tune_groups, tune_stage); by default they go
+// by N and the population (pair_launch). Both caps keep 128 registers a thread (G = 2: one
 // 512-thread CTA per SM; G = 1: up to two 256-thread CTAs).
 
 //

@@ -6,6 +6,9 @@ tuning leaves the population and the random streams where they were. The
 autotuner also picks the inversion layout (qmc2d_set_inversion), whose
 choices agree to round-off: bit for bit when it keeps the defaults, to
 1e-12 otherwise."""
+import importlib
+import os
+
 import numpy as np
 import pytest
 
@@ -68,6 +71,41 @@ def test_autotune_scope_keeps_the_choices_outside_it(q, n26, n26_configs):
         assert h.get_pair_lanes() == 16 and h.get_launch()[2] == 1
         with pytest.raises(q.QMCError):
             h.set_autotune_scope(8)
+
+
+@pytest.mark.parametrize("scope", [0, 2, 4, 6])
+def test_autotune_leaves_groups_and_staging_outside_its_scope(q, n26, n26_configs, scope):
+    """Walker groups left to the size stay so (0), and the call returns those of
+    this population: one for at most one walker per SM."""
+    with q.Handle(n26, capacity=len(n26_configs), seed=4) as h:
+        h.population_set(n26_configs)
+        h.set_autotune_scope(scope)
+        assert h.autotune()[:2] == (1, 0)
+        assert h.get_launch()[:2] == (0, 0)
+        h.set_launch(2, 1)
+        assert h.autotune()[:2] == (2, 1)
+        assert h.get_launch()[:2] == (2, 1)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_autotune_times_the_layouts_that_moves_take(q, tmp_path, mode):
+    """Moves over real orbitals have no inversion layout (layout 0 is kept);
+    where the caller chose complex moves the layouts are timed, on the
+    evaluation kernel: its inversion phase has run."""
+    tables = importlib.import_module("2degas_b200.tables")
+    d = tables.make_run(os.path.join(tmp_path, "d"), "c", 13, 13, 3.0, nconf=8,
+                        backflow=(0.2, 3.0, 1.8))
+    s = q.System.read(d, "c")
+    with q.Handle(s, capacity=8, seed=4) as h:
+        h.population_set(s.read_configs(d, ".0", 0, 8))
+        h.set_inversion(1)
+        h.set_move_inversion(mode)
+        h.set_autotune_scope(4)
+        h.phase_timers(True)
+        h.autotune()
+        ran = h.phase_timers(False)["invert"] > 0
+        assert ran == (mode != 1)
+        assert mode != 1 or h.get_launch()[2] == 0
 
 
 def test_set_launch_rejects_bad_choices(q, n26, n26_configs):
