@@ -372,15 +372,6 @@ extern "C" int qmc2d_create(const qmc2d_system *sys, const qmc2d_options *opt,
   if ((e = dalloc(&h->ds, 1)) != cudaSuccess) return fail(cuda_fail(e, "alloc"));
   cudaMemcpy(h->ds, &h->hs, sizeof(q2d::DevSys), cudaMemcpyHostToDevice);
   int cap = h->cap, N = h->N, nt = h->nt, np = h->nprops;
-  // the move scratch, without room for real orbitals when that does not fit
-  // beside what is allocated
-  e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
-  if (e == cudaErrorMemoryAllocation && h->hs.real_room && !h->hs.gmat) {
-    cudaGetLastError();
-    h->hs.real_room = h->hs.real_orb = 0;
-    e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
-  }
-  if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
   for (int k = 0; k < 2; k++)
     if ((st = alloc_pop(&h->pop[k], cap, N, nt, np))) return fail(st);
   if ((e = dalloc(&h->d_blk, (size_t)cap * np)) != cudaSuccess ||
@@ -403,6 +394,15 @@ extern "C" int qmc2d_create(const qmc2d_system *sys, const qmc2d_options *opt,
       (e = dalloc(&h->d_blksum, (size_t)np + 1)) != cudaSuccess ||
       (e = dalloc(&h->d_sdrift, (size_t)cap)) != cudaSuccess)
     return fail(cuda_fail(e, "cudaMalloc"));
+  // the move scratch last: without room for real orbitals when that does not
+  // fit beside everything else (copied to the device below)
+  e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
+  if (e == cudaErrorMemoryAllocation && h->hs.real_room && !h->hs.gmat) {
+    cudaGetLastError();
+    h->hs.real_room = h->hs.real_orb = 0;
+    e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
+  }
+  if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
   const size_t status_bytes = (sizeof(int) * (size_t)cap + 255) & ~size_t(255);
   h->stage_doubles = std::min<size_t>(kHostStageBytes / sizeof(double),
                                       (size_t)cap * (4 * (size_t)N + nt + np + 1));
