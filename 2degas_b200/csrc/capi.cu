@@ -98,6 +98,27 @@ cudaError_t dalloc(T **p, size_t n) {
 // us with copies from and to pageable memory, 98 staged (256: 273 and 150).
 constexpr size_t kHostStageBytes = 4 << 20;
 
+// Whether `doubles` go through the staging memory, which the first such call
+// allocates (12 us; page-locking 4 MB with every handle took 1.5 to 3.4 of the 5.5
+// to 7.3 ms that creating one of 4096 walkers took, 3.9 without) and larger
+// ones replace by twice what they need. Without memory for it, the copies
+// are pageable.
+bool host_stage(qmc2d_handle *h, size_t doubles) {
+  if (doubles <= h->stage_doubles) return true;
+  const size_t most = kHostStageBytes / sizeof(double), n = std::min(most, 2 * doubles);
+  if (doubles > most) return false;
+  if (h->h_stage) cudaFreeHost(h->h_stage);
+  h->h_stage = nullptr;
+  h->stage_doubles = 0;
+  if (cudaMallocHost((void **)&h->h_stage, sizeof(double) * n) != cudaSuccess) {
+    cudaGetLastError();
+    h->h_stage = nullptr;
+    return false;
+  }
+  h->stage_doubles = n;
+  return true;
+}
+
 // The orbitals of every spin as real combinations (DevSys::real_orb): an odd
 // number of plane waves, k = 0 and exact pairs +-k.
 bool real_orbitals(const qmc2d_system *sys) {
@@ -403,13 +424,8 @@ extern "C" int qmc2d_create(const qmc2d_system *sys, const qmc2d_options *opt,
     e = dalloc(&h->d_mscr, (size_t)cap * q2d::move_scratch_doubles(h->hs));
   }
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc"));
-  const size_t status_bytes = (sizeof(int) * (size_t)cap + 255) & ~size_t(255);
-  h->stage_doubles = std::min<size_t>(kHostStageBytes / sizeof(double),
-                                      (size_t)cap * (4 * (size_t)N + nt + np + 1));
-  if ((e = cudaMallocHost((void **)&h->h_status,
-                          status_bytes + sizeof(double) * h->stage_doubles)) != cudaSuccess)
+  if ((e = cudaMallocHost((void **)&h->h_status, sizeof(int) * (size_t)cap)) != cudaSuccess)
     return fail(cuda_fail(e, "cudaMallocHost"));
-  h->h_stage = reinterpret_cast<double *>(reinterpret_cast<char *>(h->h_status) + status_bytes);
   // a backflow table of zeros only: the determinant of plain plane waves
   h->bf_zero = 0;
   if (h->hs.has_bf) {
@@ -679,6 +695,7 @@ extern "C" int qmc2d_destroy(qmc2d_handle *h) {
                   h->d_s, h->d_mscr, h->d_blksum, h->hs.phase, h->d_gmat, h->d_sdrift};
   for (void *b : bufs) cudaFree(b);
   if (h->h_status) cudaFreeHost(h->h_status);
+  if (h->h_stage) cudaFreeHost(h->h_stage);
   for (int k = 0; k < QMC2D_NKERNELS; k++)
     for (cudaEvent_t e : h->ev[k]) cudaEventDestroy(e);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -791,7 +808,7 @@ extern "C" int qmc2d_compute_properties(qmc2d_handle *h, int nw, const double *x
   CK(join_side(h));
   const size_t N2 = 2 * (size_t)h->N, w = nw;
   const size_t len[5] = {N2 * w, N2 * w, (size_t)h->nt * w, (size_t)h->nprops * w, w};
-  const bool staged = len[0] + len[1] + len[2] + len[3] + len[4] <= h->stage_doubles;
+  const bool staged = host_stage(h, len[0] + len[1] + len[2] + len[3] + len[4]);
   const double *src = x;
   if (staged) {
     std::memcpy(h->h_stage, x, sizeof(double) * len[0]);

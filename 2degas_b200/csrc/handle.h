@@ -22,8 +22,7 @@ struct qmc2d_handle {
   double *d_blk = nullptr, *d_norm = nullptr, *d_cnt = nullptr, *d_wate = nullptr;
   int *d_status = nullptr;
   int *h_status = nullptr;  // cap status words in pinned host memory (sync_status)
-  // behind them (256-byte aligned), staging of small host-buffer evaluations
-  // (qmc2d_compute_properties)
+  // pinned staging of small host-buffer evaluations (qmc2d_compute_properties)
   double *h_stage = nullptr;
   size_t stage_doubles = 0;
   double *d_mscr = nullptr;  // move scratch: cap * move_scratch_doubles(hs)

@@ -1,7 +1,8 @@
 """A handle on a nearly full device: where everything but the real-orbital room of
 the move scratch fits, the handle is made without that room, and its moves
 are those of the complex kernels (to 1e-9 of the largest value, as the routes
-agree elsewhere)."""
+agree elsewhere). Host memory is page-locked for the staging of host-buffer
+evaluations when a handle makes one, in the size that it needs."""
 import importlib
 import os
 
@@ -44,3 +45,30 @@ def test_create_falls_back_to_the_smaller_scratch(q, tmp_path):
         torch.cuda.empty_cache()
     for k in ("x", "g", "p"):
         assert np.abs(got[k] - want[k]).max() < 1e-9 * np.abs(want[k]).max(), k
+
+
+def _resident_shared():
+    with open("/proc/self/status") as f:
+        return sum(int(line.split()[1]) for line in f if line.startswith("RssShmem")) << 10
+
+
+def test_handles_page_lock_no_staging_that_they_do_not_use(q, n26):
+    q.Handle(n26, capacity=4096, seed=1).close()
+    before = _resident_shared()
+    hs = [q.Handle(n26, capacity=4096, seed=1) for _ in range(16)]
+    grown = _resident_shared() - before
+    for h in hs:
+        h.close()
+    assert grown < 16 * MB  # 16 x 4096 status words are 256 KB
+
+
+def test_staging_grows_with_the_calls(q, n26, n26_configs):
+    """Calls of every size, with those beyond the staging between them, return what
+    one configuration at a time does."""
+    x = np.tile(n26_configs, (64, 1))
+    with q.Handle(n26, capacity=len(x), seed=1) as h:
+        one = [h.compute_properties(x[k:k + 1]) for k in range(64)]
+        for n in (2, 64, 3, 640, 4096, 65):
+            for got, j in zip(h.compute_properties(x[:n]), range(4)):
+                want = np.concatenate([o[j] for o in one])[np.arange(n) % 64]
+                assert np.array_equal(got, want)
