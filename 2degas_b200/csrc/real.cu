@@ -772,13 +772,24 @@ __device__ __forceinline__ void s_contract(const double (&acc)[kN][kB][kB][4][2]
       if (kB > 1 && jt > kt) continue;  // inside a diagonal item: the other order counts
       const double wgt = jt == kt ? 1.0 : 2.0;
       const int j = 8 * jt + lg;
+      // the loads of both entries in flight together. They are plain ones: the
+      // read-only path is not for what a kernel before wrote that may still run
+      // when this one starts.
+      double f[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int jc = min(j, n - 1), kc = min(8 * kt + 2 * lq + e, n - 1);
+        const int kj = kc + jc * n, jk = jc + kc * n;
+        f[e][0] = FX[kj];
+        f[e][1] = FX[jk];
+        f[e][2] = FY[kj];
+        f[e][3] = FY[jk];
+      }
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int k = 8 * kt + 2 * lq + e;
         if (j < n && k < n) {
-          const int kj = k + j * n, jk = j + k * n;
-          const double xkj = wgt * __ldg(FX + kj), xjk = __ldg(FX + jk);
-          const double ykj = wgt * __ldg(FY + kj), yjk = __ldg(FY + jk);
+          const double xkj = wgt * f[e][0], xjk = f[e][1], ykj = wgt * f[e][2], yjk = f[e][3];
           double m0 = xkj * xjk, m1 = xkj * yjk, m2 = ykj * xjk, m3 = ykj * yjk;
           if (j == k) {
             m0 -= d2[3 * j];
@@ -865,8 +876,8 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   };
   stage(0, 0);
   for (int e = t; e < 2 * n; e += nthr)
-    fd[e] = __ldg(FX + (e & 1 ? n * n : 0) + (e >> 1) * (n + 1));
-  for (int e = t; e < 3 * n; e += nthr) d2[e] = __ldg(FX + 2 * n * n + 2 + e);
+    fd[e] = FX[(e & 1 ? n * n : 0) + (e >> 1) * (n + 1)];
+  for (int e = t; e < 3 * n; e += nthr) d2[e] = FX[2 * n * n + 2 + e];
   double lt[2] = {0.0, 0.0};
   // drift of the columns of a buffer: four lanes per electron
   auto drift = [&](const double *buf, int c0, int c1) {
@@ -956,8 +967,8 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   // - sum_j f_j . L_j
   const double *o = a.scr + w * a.stride;
   for (int e = t; e < 2 * n; e += nthr) {
-    if (!type) lt[0] -= fd[e] * __ldg(o + a.l_qbd + 2 * f0 + e);
-    if (split ? type : nt > 1) lt[1] -= fd[e] * __ldg(o + a.l_sb + 2 * f0 + e);
+    if (!type) lt[0] -= fd[e] * o[a.l_qbd + 2 * f0 + e];
+    if (split ? type : nt > 1) lt[1] -= fd[e] * o[a.l_sb + 2 * f0 + e];
   }
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) {

@@ -150,12 +150,11 @@ __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *
       const int n = S.np[t];
       const double *FX = base + R.f[t], *FY = FX + n * n;
       for (int j = tid; j < 2 * n; j += NT)
-        m.gd[2 * S.ipfrst[t] + j] = -__ldg((j & 1 ? FY : FX) + (j >> 1) * (n + 1));
+        m.gd[2 * S.ipfrst[t] + j] = -(j & 1 ? FY : FX)[(j >> 1) * (n + 1)];
       for (int e = tid; e < n * n; e += NT) {
         const int j = e / n, k = e - j * n;
         if (k > j)
-          s[t] -= 2.0 * (__ldg(FX + k + j * n) * __ldg(FX + j + k * n) +
-                         __ldg(FY + k + j * n) * __ldg(FY + j + k * n));
+          s[t] -= 2.0 * (FX[k + j * n] * FX[j + k * n] + FY[k + j * n] * FY[j + k * n]);
       }
     }
     block_sum_n<2, NT>(s, m.red);
@@ -164,8 +163,8 @@ __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *
   } else {
     // the determinants' drift: every spin's share
     for (int j = tid; j < 2 * N; j += NT) {
-      double g = __ldg(base + R.s[0] + j);
-      if (nt > 1) g += __ldg(base + R.s[1] + j);
+      double g = base[R.s[0] + j];
+      if (nt > 1) g += base[R.s[1] + j];
       m.gd[j] = g;
     }
   }
@@ -173,11 +172,11 @@ __device__ inline int eval_det_real(const DevSys &S, const EvalSmem &m, double *
   for (int t = 0; t < 2; t++) {
     if (t >= nt) continue;
     const double *f = base + R.f[t] + 2 * S.np[t] * S.np[t], *s = base + R.s[t] + 2 * N;
-    logdet_sum += __ldg(f);
-    if (__ldg(f + 1) != 0.0) status |= ST_SINGULAR;
+    logdet_sum += f[0];
+    if (f[1] != 0.0) status |= ST_SINGULAR;
     if (!S.bf_zero) {
-      l0 += __ldg(s);
-      l1 += __ldg(s + 1);
+      l0 += s[0];
+      l1 += s[1];
     }
   }
   cp_async_wait_all();
