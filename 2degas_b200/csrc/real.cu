@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs
   const int item = blockIdx.x * kRealWarps + wl;
   const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0], r = lane;
-  if (w >= nw || n > NM) return;  // whole warps; nothing below waits on other warps
+  if (w >= nw || n > NM || !real_on(a, w)) return;  // whole warps; nothing below waits on other warps
   double *Bs = reinterpret_cast<double *>(smem) + wl * real_warp_doubles(NM);
   double *Wt = Bs + NM * LD, *prow = Wt + NM * LD;
   double2 *sg = reinterpret_cast<double2 *>(prow + 64);
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, in
   pdl_wait();
   const int w = a.nt > 1 ? blockIdx.x >> 1 : blockIdx.x, spn = a.nt > 1 ? blockIdx.x & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0];
-  if (w >= nw || n <= 32) return;  // whole CTAs
+  if (w >= nw || n <= 32 || !real_on(a, w)) return;  // whole CTAs
   const int t = threadIdx.x, nthr = blockDim.x, G = nthr >> 5, lane = t & 31, wp = t >> 5;
   const int s = lane & (kL - 1), r0 = wp * RW + lane / kL * kR;  // first of its rows
   double *slots = reinterpret_cast<double *>(smem);                  // [2][G][SL]
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kFThreads, 1) real_f_kernel(RealArgs a, int nw
   const int bj = blockIdx.x % blocks, item = blockIdx.x / blocks;
   const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
   const int n = spn ? a.np[1] : a.np[0], j0 = 32 * bj;
-  if (w >= nw || n <= 32 || j0 >= n) return;  // whole CTAs
+  if (w >= nw || n <= 32 || j0 >= n || !real_on(a, w)) return;  // whole CTAs
   const int t = threadIdx.x, wp = t >> 5, lane = t & 31, lg = lane >> 2, lt = lane & 3;
   double *base = real_base(a, w);
   const int ldw = spn ? a.ldw[1] : a.ldw[0], ld = odd4(ldw), rows = (n + 15) / 16 * 16;
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
   // split (kB = 1, two types): one CTA per type of the columns
   const int item = blockIdx.x >> split, type = split ? blockIdx.x & 1 : 0;
   const int w = a.nt > 1 ? item >> 1 : item, spn = a.nt > 1 ? item & 1 : 0;
-  if (w >= nw) return;
+  if (w >= nw || !real_on(a, w)) return;  // whole CTAs
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nthr = blockDim.x, NW = nthr >> 5;
   const int nt = a.nt, n = spn ? a.np[1] : a.np[0], f0 = spn ? a.f0[1] : a.f0[0];
   double *base = real_base(a, w);
@@ -1079,9 +1079,10 @@ cudaError_t launch_orbitals_f(const DevSys &hs, const RealArgs &a, int nw, cudaS
 }  // namespace
 
 cudaError_t launch_real_det(const DevSys &hs, const DevSys *ds, int nw, double *scr,
-                            cudaStream_t st) {
+                            cudaStream_t st, bool some) {
   if (nw <= 0) return cudaSuccess;
-  const RealArgs a = real_args(hs, scr);
+  RealArgs a = real_args(hs, scr);
+  if (some) a.l_grows = move_scratch(hs).grows;
   const cudaError_t e = launch_orbitals_f(hs, a, nw, st);
   // a backflow of zeros needs no sums over Jacobian blocks (eval_det_real)
   if (e != cudaSuccess || hs.bf_zero) return e;

@@ -32,6 +32,7 @@ namespace q2d {
 struct RealArgs {
   int N, nt, np[2], f0[2], bf_zero, cols, pad0, jp;
   int l_q, l_qbd, l_sb, l_pair;
+  int l_grows;  // MoveScratch::grows where it is to be looked at, else -1
   size_t stride, f[2], s[2], w[2];
   int ldw[2];
   const double *gvec;
@@ -61,6 +62,7 @@ inline RealArgs real_args(const DevSys &hs, double *scr) {
   a.l_qbd = l.qbd;
   a.l_sb = l.sb;
   a.l_pair = l.pair;
+  a.l_grows = -1;
   a.stride = l.stride;
   a.gvec = hs.gvec;
   a.gbase = hs.gmat ? hs.gmat_base : nullptr;
@@ -73,6 +75,12 @@ inline RealArgs real_args(const DevSys &hs, double *scr) {
 // else in its move scratch behind the per-particle sums.
 __host__ __device__ inline double *real_base(const RealArgs &a, size_t w) {
   return a.gbase ? a.gbase + w * a.gstride : a.scr + w * a.stride + a.l_pair;
+}
+
+// Whether walker w has anything to evaluate (a reptile whose move has fewer bead
+// growths than this one has not).
+__device__ __forceinline__ bool real_on(const RealArgs &a, size_t w) {
+  return a.l_grows < 0 || a.scr[w * a.stride + a.l_grows] != 0.0;
 }
 
 // Shared memory of the evaluation's end: the per-particle arrays of EvalSmem
@@ -103,9 +111,10 @@ __host__ __device__ inline size_t real_carve(const DevSys &s, char *base, EvalSm
 
 // Between the pair passes and the evaluation's end, for nw walkers: orbitals,
 // inverse and F of every (walker, spin), then the S sums, drift and
-// Laplacian shares, all in the walkers' real regions.
+// Laplacian shares, all in the walkers' real regions. some: of the walkers marked
+// in their scratch (MoveScratch::grows) alone.
 cudaError_t launch_real_det(const DevSys &hs, const DevSys *ds, int nw, double *scr,
-                            cudaStream_t st);
+                            cudaStream_t st, bool some = false);
 
 // The pair passes' sums of walker w into shared memory, the determinant sums
 // zeroed (asynchronous 8-byte copies; the caller waits).

@@ -560,6 +560,8 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
   for (int r = blockIdx.x * G + grp; r < a.nrep; r += gridDim.x * G) {
     int idir, ndelta;
     rmc_dir(a, r, t, idir, ndelta);
+    double *o = scr + (size_t)r * L.stride;
+    if (kJ && tid == 0) o[L.grows] = idelta <= ndelta ? 1.0 : 0.0;
     if (idelta > ndelta) continue;  // the whole group: r is the group's
     long long tph = clock64();
     const int jstart = idir == 1 ? a.ends[2 * r + 1] : a.ends[2 * r];
@@ -582,7 +584,6 @@ __global__ void __launch_bounds__(G * kThreads, 2 / G) rmc_pairs_kernel(
     const double dold = block_sum_t<kThreads>(dd, m.red, sync, tid);
     const double lng = block_sum_t<kThreads>(wg, m.red, sync, tid);
     phase_mark(S, PH_PROPOSE, tph, tid == 0);
-    double *o = scr + (size_t)r * L.stride;
     double *pout = !S.has_bf || S.bf_zero ? nullptr
                    : kJ && S.gmat         ? S.gmat_base + (size_t)r * S.gmat_stride
                                           : o + L.pair;
@@ -1103,7 +1104,9 @@ extern "C" int qmc2d_rmc(qmc2d_handle *h, int nstp) {
         if (real) {
           {
             ProfScope ps(h, QMC2D_KERNEL_ORB_INV, h->stream);
-            RCK(q2d::launch_real_det(h->hs, h->ds, h->rmc.nrep, h->d_mscr, h->stream));
+            // every move has a first growth; later ones of some reptiles only
+            RCK(q2d::launch_real_det(h->hs, h->ds, h->rmc.nrep, h->d_mscr, h->stream,
+                                     idelta > 1));
           }
           ProfScope ps(h, QMC2D_KERNEL_RMC, h->stream);
           RCK(q2d::launch_pdl(q2d::rmc_real_kernel, h->rmc.nrep, q2d::kThreads, smr, h->stream, h->hs, a,

@@ -267,14 +267,15 @@ __host__ __device__ inline size_t pair_carve(const DevSys &s, char *base, EvalSm
 // P = N (N - 1) / 2 (the values are functions of r_ij alone, computed from
 // the same bits for (i, j) and (j, i), so one triangle serves both orders).
 // A reptile's bead growth also keeps its proposal's drift term (dold) and
-// the free-propagator sum (lng) of get_w_stack (reptation.f:1804-1851).
+// the free-propagator sum (lng) of get_w_stack (reptation.f:1804-1851), and
+// whether the reptile's move has this growth (grows: 1 or 0, real orbitals).
 __host__ __device__ inline size_t pair_count(int N) { return (size_t)N * (N - 1) / 2; }
 // Row-major upper triangle without the diagonal: (a, b), a < b.
 __host__ __device__ inline size_t pair_tri(int N, int a, int b) {
   return (size_t)a * (2 * N - a - 1) / 2 + (size_t)(b - a - 1);
 }
 struct MoveScratch {
-  int x, g, q, sb, qbd, lap, ltf, vp, wold, dold, lng, rhok, pair;
+  int x, g, q, sb, qbd, lap, ltf, vp, wold, dold, lng, grows, rhok, pair;
   size_t inv;  // orb_inv_kernel's output per spin (0: no such region)
   size_t stride;
 };
@@ -344,8 +345,9 @@ __host__ __device__ inline MoveScratch move_scratch(const DevSys &s, bool with_i
   l.wold = 14 * N;
   l.dold = 14 * N + 1;
   l.lng = 14 * N + 2;
-  l.rhok = 14 * N + 3;
-  l.pair = (14 * N + 3 + 4 * (s.nk > 0 ? s.nk : 1) + 3) & ~3;
+  l.grows = 14 * N + 3;
+  l.rhok = 14 * N + 4;
+  l.pair = (14 * N + 4 + 4 * (s.nk > 0 ? s.nk : 1) + 3) & ~3;
   size_t end = (size_t)l.pair + (s.has_bf ? 3 * pair_count(N) : 0);
   l.inv = 0;
   if (with_inv && orb_inv_fits(s)) {
