@@ -33,7 +33,8 @@
 // calls made handle by handle give the same walkers bit for bit.
 //
 // The graph is captured again when a call's parameters (time steps, trial
-// energies, population sizes, buffer parity) differ from the cached one.
+// energies, population sizes, buffer parity) or a handle's choices (route,
+// launch, precision, timers) differ from the cached one's.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -215,10 +216,18 @@ int run(qmc2d_batch *b, int n, int dmc, const double *delta, const double *etria
       key.push_back((double)b->h[k]->cur);
       key.push_back((double)(intptr_t)b->h[k]);
       key.push_back(b->h[k]->dmc_ecut);
-      key.push_back(move_real(b->h[k], b->h[k]->nw) ? 1.0 : 0.0);  // a twist may have changed it
+      // the launches' route and choices: a twist, the tuner or the caller may
+      // have changed them
+      const q2d::DevSys &hs = b->h[k]->hs;
+      const bool real = move_real(b->h[k], b->h[k]->nw);
+      key.push_back(real ? 1.0 : 0.0);
+      key.push_back(!real && move_orb_inv(b->h[k]) ? 1.0 : 0.0);
+      key.push_back((double)hs.tune_groups);
+      key.push_back((double)hs.tune_stage);
+      key.push_back((double)hs.tune_lanes);
       // kernels take the system by value: the timers' buffer and the precision
-      key.push_back((double)(intptr_t)b->h[k]->hs.phase);
-      key.push_back((double)b->h[k]->hs.pair_f32);
+      key.push_back((double)(intptr_t)hs.phase);
+      key.push_back((double)hs.pair_f32);
     }
     if (!b->exec || key != b->key) {
       if (b->exec) {

@@ -157,8 +157,9 @@ size_t move_smem_bytes_seq(const DevSys &s) {
 //
 // pairs_kernel and the real-orbital kernels take the system by value: its
 // fields are constant-bank operands, where a copy in shared memory costs a
-// load for every use. A captured graph keeps that value (its key holds what
-// can change: the timers' buffer, the precision, the time step).
+// load for every use. A captured graph keeps that value: its key holds what
+// can change between calls (route, launch choices, precision, timers' buffer,
+// time step), and what a twist changes is read from the wave vectors.
 //
 // pairs_kernel is persistent: its CTAs walk over the population with G
 // independent groups of kThreads threads each, every group on its own
