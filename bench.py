@@ -65,7 +65,7 @@ def move_scratch_bytes(N, nk, ns=()):
     (MoveScratch and RealLayout): the per-particle sums and rho_k, the
     Jacobian blocks of the pairs i <= j, and per spin of n orbitals F_x, F_y,
     ln|det|, the singular flag, D2, and the drift and Laplacian shares."""
-    end = (14 * N + 3 + 4 * max(nk, 1) + 3) & ~3
+    end = (14 * N + 4 + 4 * max(nk, 1) + 3) & ~3
     end += 3 * (N * (N + 1) // 2)
     end += sum(2 * n * n + 2 + 3 * n + 2 * N + 2 for n in ns)
     return 8 * end
@@ -117,6 +117,26 @@ def flops_per_move(N, ns, K, u3, backflow):
         else:
             f += 45 * n * n + 8 * n ** 3
     return float(f)
+
+
+def takes_real(orbital_scopes, mode, layout):
+    """Whether the moves timed ran over real orbitals, from the number of
+    orbital scopes (none when everything runs in the move kernel), the move
+    inversion mode (None: the default, 1) and the inversion layout in force.
+    Modes 0 and 2 keep complex orbitals, mode 2 with a scope of its own."""
+    return orbital_scopes > 0 and mode in (None, 1) and layout == 0
+
+
+def orbital_kernels(ns, real, backflow=1):
+    """The kernels of one orbital scope (qmc2d_profile's ORB_INV) of spins of ns
+    orbitals: spins above 32 in a CTA each, smaller ones in a warp, F in its
+    own kernel above 113, S when the backflow is not zero."""
+    if not real:
+        return ["orb_inv_kernel"]
+    return ((["real_det_warp_kernel"] if min(ns) <= 32 else []) +
+            (["real_inv_cta_kernel"] if max(ns) > 32 else []) +
+            (["real_f_kernel"] if max(ns) > 113 else []) +
+            (["real_s_kernel"] if backflow else []))
 
 
 def make_config(tmp, nconf, seed, shell=None, rs=None):
@@ -499,8 +519,8 @@ def b200_arm(args, rank, world, local_rank):
     line = None
     if rank == 0:
         K = sysobj.s.nk
-        # split orbital kernels with the default layout: the real-orbital route
-        real = oi_n > 0 and h.get_launch()[2] == 0
+        real = takes_real(oi_n, args.move_inversion, h.get_launch()[2])
+        orb = orbital_kernels(ns, real) if oi_n else []
         fpm = (real_flops_per_move if real else flops_per_move)(N, ns, K, 0, 1)
         # one walker-move of the population = one pair kernel, the orbital
         # kernels (one timing scope) and one end-of-move launch; the roofline
@@ -511,8 +531,7 @@ def b200_arm(args, rank, world, local_rank):
         if world == 1 and not args.no_cpu:
             rate, cores, sample = cpu_rate(d, args.cpu_seconds, rs=rs)
             cpu = {"value": rate, "unit": UNIT, "cores": cores, "kind": "port", "sample": sample}
-        # one orbital launch scope is two kernels (orbitals and F, then S)
-        launches = pair_n + 2 * oi_n + move_n + br_n + ga_n
+        launches = pair_n + len(orb) * oi_n + move_n + br_n + ga_n
         metric, config = workload_desc(args, world)
         line = {
             "metric": metric,
@@ -532,8 +551,8 @@ def b200_arm(args, rank, world, local_rank):
                          "traffic": ((MOVE_DRAM_READ_PER_WALKER + move_scratch_bytes(N, K, ns)) * nw
                                      if headline else None),
                          "traffic_source": TRAFFIC_SOURCE if headline else None,
-                         "kernel": ("pairs_kernel + real_det_warp_kernel + real_s_kernel + move_real_kernel" if oi_n
-                                    else "pairs_kernel + move_kernel"),
+                         "kernel": " + ".join(["pairs_kernel"] + orb +
+                                              ["move_real_kernel" if real else "move_kernel"]),
                          "flops_per_move": fpm,
                          "reference_flops_per_move": flops_per_move(N, ns, K, 0, 1),
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64)"},
@@ -810,10 +829,12 @@ def config_arm(args, rank, world, local_rank):
         # builds its determinant only in the backflow routine): counted as
         # the plain Slater-Jastrow algorithm it is
         terms = (0, 0) if vmc else (1, 1)  # u3, backflow
-        # split orbital kernels: the real-orbital route
+        oi_n = kms[capi.KERNEL_ORB_INV][1] if capi.KERNEL_ORB_INV in kms else 0
+        # (reptation keeps the default mode, and its complex route has no scope)
+        real = takes_real(oi_n, args.move_inversion if vmc else None, h.get_launch()[2])
+        orb = orbital_kernels(ns, real, terms[1]) if oi_n else []
         fpm = (flops_per_sweep(N, ns, K) if vmc and args.single else
-               real_flops_per_move(N, ns, K, *terms) if kms[capi.KERNEL_ORB_INV][1] else
-               flops_per_move(N, ns, K, *terms))
+               (real_flops_per_move if real else flops_per_move)(N, ns, K, *terms))
         kern_ms = sum(kms[k][0] for k in kernels)
         n_launch = max(kms[kernels[-1]][1], 1)
         achieved = fpm * nw * nw_moves / (kern_ms / n_launch * 1e-3) / 1e12
@@ -836,13 +857,15 @@ def config_arm(args, rank, world, local_rank):
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                          "kernel": ("single_kernel" if vmc and args.single else
-                                    "pair kernel + orbital kernels + end of the move" if vmc
-                                    else "rmc_pairs_kernel + orbital kernels + rmc_real_kernel"),
+                                    "rmc_move_kernel" if not kms[kernels[0]][1] else " + ".join(
+                             ["pairs_kernel" if vmc else "rmc_pairs_kernel"] + orb +
+                             [("move_" if vmc else "rmc_") +
+                              ("real_kernel" if real else "kernel" if vmc else "det_kernel")])),
                          "flops_per_move": fpm,
                          "reference_flops_per_move": flops_per_move(N, ns, K, *terms),
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64)"},
             "cpu_baseline": cpu,
-            "gpu_launches": sum(kms[k][1] for k in kernels),
+            "gpu_launches": sum(kms[k][1] for k in kernels) + (len(orb) - 1) * oi_n,
             "kernel_ms": {str(k): kms[k][0] for k in kernels},
             "acceptance": acc["accepted"] / max(acc["proposed"], 1),
             "e_mean": blk[0] / norm,
