@@ -292,7 +292,8 @@ __host__ __device__ inline size_t orb_inv_warp_doubles(int n) {
 }
 
 template <int NM>
-__global__ void __launch_bounds__(32 * kOrbWarps) orb_inv_kernel(const DevSys *sp, MoveArgs a) {
+__global__ void __launch_bounds__(32 * kOrbWarps) orb_inv_kernel(const DevSys *sp, MoveArgs a,
+                                                                 MoveScratch L) {
   static_assert(NM <= 32, "one lane per row");
   __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
@@ -307,7 +308,6 @@ __global__ void __launch_bounds__(32 * kOrbWarps) orb_inv_kernel(const DevSys *s
   double2 *tile = reinterpret_cast<double2 *>(base);
   double *qs = base + 2 * (size_t)n * ld;
   double2 *prow = reinterpret_cast<double2 *>(qs + 2 * n);  // 2 x 32, double-buffered
-  const MoveScratch L = move_scratch(S);
   double *o = a.scr + (size_t)w * L.stride;
   size_t off = L.inv;
   for (int t = 0; t < spn; t++) off += inv_spin_doubles(S.np[t]);
@@ -396,9 +396,12 @@ __global__ void __launch_bounds__(32 * kOrbWarps) orb_inv_kernel(const DevSys *s
 
 // kSeq: the one-buffer form for moves whose orbitals and inverses come from
 // orb_inv_kernel (smaller shared memory, 80 registers: three CTAs per SM).
+// The scratch's offsets L come from the host, here and in orb_inv_kernel: formed
+// by every thread they took 13 + 13, twisted, 1024 walkers from 116 to 127 us and
+// from 20.9 to 23.0.
 template <bool kGmat, bool kSeq>
 __global__ void __launch_bounds__(kThreads, kSeq ? 3 : 2) move_kernel(const DevSys *sp, DevPop pop,
-                                                                      MoveArgs a) {
+                                                                      MoveArgs a, MoveScratch L) {
   __shared__ DevSys S;
   extern __shared__ __align__(16) char smem[];
   load_sys(S, sp);
@@ -411,7 +414,6 @@ __global__ void __launch_bounds__(kThreads, kSeq ? 3 : 2) move_kernel(const DevS
   const int w = blockIdx.x, tid = threadIdx.x;
   if (w >= a.nw) return;
   const int N = S.N, N2 = 2 * N, np = S.nprops, nt = S.nt;
-  const MoveScratch L = move_scratch(S);
   const double *o = a.scr + (size_t)w * L.stride;
   // the pair values are read by the Jacobian build long after this point,
   // the orbitals and inverse of orb_inv_kernel at the start of the
@@ -1170,7 +1172,7 @@ cudaError_t launch_orb_inv(const DevSys &hs, const DevSys *ds, const MoveArgs &a
                       : orb_inv_kernel<32>;
   cudaError_t e = set_smem((const void *)k, sm);
   if (e != cudaSuccess) return e;
-  k<<<grid, 32 * kOrbWarps, sm, st>>>(ds, a);
+  k<<<grid, 32 * kOrbWarps, sm, st>>>(ds, a, move_scratch(hs));
   return cudaGetLastError();
 }
 
@@ -1190,7 +1192,7 @@ cudaError_t launch_move(const DevSys &hs, const DevSys *ds, DevPop pop, const Mo
                    : (seq ? move_kernel<false, true> : move_kernel<false, false>);
   cudaError_t e = set_smem((const void *)k, sm);
   if (e != cudaSuccess) return e;
-  k<<<a.nw, kThreads, sm, st>>>(ds, pop, a);
+  k<<<a.nw, kThreads, sm, st>>>(ds, pop, a, move_scratch(hs));
   return cudaGetLastError();
 }
 

@@ -313,7 +313,9 @@ __host__ __device__ inline RealLayout real_layout(const DevSys &s) {
   RealLayout r{};
   r.jp = s.N * (s.N + 1) / 2;
   size_t o = s.has_bf && !s.bf_zero ? ((size_t)3 * r.jp + 1) & ~size_t(1) : 0;
-  for (int t = 0; t < s.nt; t++) {
+#pragma unroll
+  for (int t = 0; t < 2; t++) {  // unrolled: in kernels the arrays stay in registers
+    if (t >= s.nt) continue;
     const size_t n = s.np[t];
     r.f[t] = o;
     o += (2 * n * n + 2 + 3 * n + 1) & ~size_t(1);
