@@ -1005,14 +1005,22 @@ static size_t pair_smem_limit(int optin) { return (size_t)optin - 1024; }
 
 // Groups, staging and lanes compute the same pair terms; groups and staging
 // leave every bit, the lanes the order of a particle's partial sums.
-//   groups and staging (FP64, us per launch, 148 SMs): one group per CTA
-//   when two and the rows do not fit a CTA's shared memory (N = 122 with 144-byte
-//   rows, 1024 walkers: 321 against 344; N = 161, 148: 95 against 173) and when every SM
-//   has at most one walker (N = 58, 148: 25 against 29); rows of small
-//   systems stay in global memory up to seven walkers per SM, where copying
-//   them costs more than it saves (N = 26: 17.0 against 19.4 at 64 walkers, 29.5
-//   against 31.4 at 512, equal at 1024); else two groups with staged rows
-//   (N = 58, 4096: 312 against 355).
+//   groups and staging (us per launch, 148 SMs):
+//   - N <= 32: one group per CTA and the rows in global memory while copying
+//     them costs more than it saves, up to 7 walkers per SM at N = 26 (16.7
+//     against 18.7 in two groups at 200 walkers, 32.0 and 33.0 at 888, 39.7 and
+//     39.6 at 1184) and 4 at N = 32 (24.9 and 24.9 at 444, 34.4 and 33.1 at
+//     740), one less with u3 (N = 26: 41.8 and 41.2 at 888; N = 32: 33.2 and
+//     32.0 at 592, 57.3 and 53.7 at 1024).
+//   - Two groups and the rows do not fit a CTA: one group with them, a walker per
+//     SM and round, where its rounds take less than rounds of two walkers
+//     per SM without, which last 1.8 to 2.0 times as long (61 + 61 with u3:
+//     211 against 258 at 444, 411 and 383 at 768, 478 and 508 at 1024, 947
+//     and 889 at 2048; 81 + 81: 234 and 299 at 444), 1.55 times without
+//     backflow sums (61 + 61 with u3: 423 and 373 at 1024, 832 and 652 at 2048).
+//   - At most one walker per SM: one group with the rows (N = 58, 148: 25
+//     against 29).
+//   - Else two groups with the rows (N = 58, 4096: 312 against 355).
 //   lanes: the fewest sweeps, ceil(N / particles per round) rounds of
 //   ceil(N / lanes) partners and the round's reductions (N = 58: four lanes 273,
 //   eight 312; N = 122: 344 against 360; N = 74: eight 209, four 230). Eight in
@@ -1022,14 +1030,18 @@ PairLaunch pair_launch(const DevSys &hs, int nw, int nsm, int optin, bool no_u3)
   const size_t grp = pair_group_bytes(hs), rows = pair_rows_bytes(hs, no_u3),
                lim = pair_smem_limit(optin);
   if (p.groups == 0) {
-    if (2 * grp + rows > lim || nw <= nsm) {
-      p.groups = 1;
-      if (hs.N <= 32) p.stage = 0;
-    } else if (hs.N <= 32 && nw < 7 * nsm) {
+    // walkers per SM up to which small systems take one group without rows
+    const double few =
+        7.0 - std::max(0.0, 0.5 * (hs.N - 26)) - (hs.has_u3 && hs.N > 24 ? 1.0 : 0.0);
+    if (hs.N <= 32 && nw < few * nsm) {
       p.groups = 1;
       p.stage = 0;
+    } else if (2 * grp + rows > lim) {
+      const int one = (nw + nsm - 1) / nsm, two = (one + 1) / 2;
+      p.groups = 1;
+      if (2 * grp <= lim && one >= (hs.has_bf && !hs.bf_zero ? 1.9 : 1.55) * two) p.stage = 0;
     } else {
-      p.groups = 2;
+      p.groups = nw <= nsm ? 1 : 2;
     }
   }
   if (p.groups * grp + rows > lim) p.stage = 0;
