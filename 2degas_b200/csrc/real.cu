@@ -54,7 +54,8 @@ __device__ __forceinline__ void orbital_rows(const RealArgs &a, const double *q,
     at(2 * p, j) = kSqrt2 * cv;
     at(2 * p + 1, j) = kSqrt2 * sv;
   }
-  for (int j = t; j < n; j += nthr) at(n - 1, j) = 1.0;
+  // (NaN where the coordinates are not finite, as exp(i 0.q) is)
+  for (int j = t; j < n; j += nthr) at(n - 1, j) = fma(0.0, q[2 * j], fma(0.0, q[2 * j + 1], 1.0));
 }
 
 // F_x and F_y of kR row tiles (from l0) and kT column tiles (from j0) of 8 x 8

@@ -1399,7 +1399,7 @@ __device__ inline void compute_rhok_lattice(const DevSys &S, const EvalSmem &m, 
     double sb, cb;
     sincospi(2.0 * (m.x[2 * i + ax] * S.eli[ax]), &sb, &cb);
     const double2 b = make_double2(cb, sb);
-    double2 p = make_double2(1.0, 0.0);
+    double2 p = make_double2(fma(0.0, cb, 1.0), 0.0);  // 1; NaN where the coordinate is not finite
     T[0] = p;
     for (int k = 1; k <= P; k++) {
       p = cmul(p, b);
