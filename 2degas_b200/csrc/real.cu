@@ -202,6 +202,9 @@ __global__ void __launch_bounds__(32 * kRealWarps) real_det_warp_kernel(RealArgs
   double ld = r < n ? log(my_d) : 0.0;
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) ld += __shfl_xor_sync(0xffffffffu, ld, q);
+  // where a spin has more than 32 orbitals a NaN pivot counts as none, as in
+  // real_inv_cta_kernel
+  if (max(a.np[0], a.np[1]) > 32) sing |= __any_sync(0xffffffffu, r < n && my_d != my_d);
   __syncwarp();
   if (r < n)
 #pragma unroll
@@ -391,8 +394,9 @@ __global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, in
       perm[k] = p;
       rowl[p] = k;
       rinv[p] = inv;
-      dk[k] = ps[kL * LS + 1];
-      if ((best >> 8) == 0u) singular = 1;
+      const double d = ps[kL * LS + 1];
+      dk[k] = d;
+      if ((best >> 8) == 0u || d != d) singular = 1;  // as the complex kernels of these spins
     }
     double fac[kR];
 #pragma unroll
