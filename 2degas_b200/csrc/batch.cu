@@ -104,7 +104,7 @@ cudaError_t enqueue(qmc2d_batch *b, int k, int g0, int ngen, int dmc, double del
     a.real = move_real(h, h->nw) ? 1 : 0;
     a.orb_inv = !a.real && move_orb_inv(h) ? 1 : 0;
     a.ctr = ctr;
-    if ((e = q2d::launch_pairs(h->hs, h->ds, h->pop[cur], a, st)) != cudaSuccess) return e;
+    if ((e = q2d::launch_pairs(h->hs, h->pop[cur], a, st)) != cudaSuccess) return e;
     if ((e = q2d::launch_orb_inv(h->hs, h->ds, a, st)) != cudaSuccess) return e;
     if ((e = q2d::launch_move(h->hs, h->ds, h->pop[cur], a, st)) != cudaSuccess) return e;
     if (dmc) {

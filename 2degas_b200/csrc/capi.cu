@@ -568,9 +568,9 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
     if (!(h->tune_scope & 1)) break;
     h->hs.tune_groups = v[0];
     h->hs.tune_stage = v[1];
-    CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));  // warm-up
+    CK(q2d::launch_pairs(h->hs, h->pop[h->cur], a, h->stream));  // warm-up
     CK(cudaEventRecord(e0, h->stream));
-    for (int r = 0; r < 3; r++) CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));
+    for (int r = 0; r < 3; r++) CK(q2d::launch_pairs(h->hs, h->pop[h->cur], a, h->stream));
     CK(cudaEventRecord(e1, h->stream));
     CK(cudaEventSynchronize(e1));
     float t = 0.f;
@@ -590,10 +590,10 @@ extern "C" int qmc2d_autotune(qmc2d_handle *h, int *groups, int *stage, double *
     int bl = 8;
     for (int l : lanes) {
       h->hs.tune_lanes = l;
-      CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));  // warm-up
+      CK(q2d::launch_pairs(h->hs, h->pop[h->cur], a, h->stream));  // warm-up
       CK(cudaEventRecord(e0, h->stream));
       for (int r = 0; r < 3; r++)
-        CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));
+        CK(q2d::launch_pairs(h->hs, h->pop[h->cur], a, h->stream));
       CK(cudaEventRecord(e1, h->stream));
       CK(cudaEventSynchronize(e1));
       float t = 0.f;
@@ -1016,7 +1016,7 @@ static int run_moves(qmc2d_handle *h, int nstp, int dmc, double delta, double et
     a.first = istp == 0;
     {
       ProfScope ps(h, QMC2D_KERNEL_PAIRS, h->stream);
-      CK(q2d::launch_pairs(h->hs, h->ds, h->pop[h->cur], a, h->stream));
+      CK(q2d::launch_pairs(h->hs, h->pop[h->cur], a, h->stream));
     }
     if (a.orb_inv || a.real) {
       ProfScope ps(h, QMC2D_KERNEL_ORB_INV, h->stream);

@@ -79,7 +79,8 @@ struct DevSys {
   // of plane waves per spin that are k = 0 and pairs +-k, gvec rows 2 p + 1
   // and 2 p + 2 exact negatives (the Gamma point). Moves and evaluations
   // then take the real-orbital kernels (real_det.cuh) unless the caller has
-  // chosen a complex layout (qmc2d_set_inversion, qmc2d_set_move_inversion).
+  // chosen an inversion layout (qmc2d_set_inversion) or, for moves alone, a move
+  // inversion mode (qmc2d_set_move_inversion).
   int real_orb;
   // The scratch has room for them (odd spins, fixed at create time: a twist
   // can be set and taken back later).

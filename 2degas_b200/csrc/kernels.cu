@@ -995,7 +995,8 @@ static size_t pair_group_bytes(const DevSys &hs) {
   return (pair_carve(hs, nullptr, nullptr, kThreads) + 127) & ~size_t(127);
 }
 static size_t pair_rows_bytes(const DevSys &hs, bool no_u3 = false) {
-  const size_t row = no_u3 && !hs.pair_f32 ? sizeof(double) * RowLayoutNoU3::sstride : hs.pair_f32 ? sizeof(float) * RowLayout<float>::sstride
+  const size_t row = hs.pair_f32 ? sizeof(float) * RowLayout<float>::sstride
+                     : no_u3     ? sizeof(double) * RowLayoutNoU3::sstride
                                  : sizeof(double) * RowLayout<double>::sstride;
   return row * (size_t)hs.cmb_nblk * (hs.cmb_ng + 1);
 }
@@ -1092,7 +1093,8 @@ static cudaError_t launch_pairs_t(const DevSys &hs, DevPop pop, const MoveArgs &
   const int need = (a.nw + G - 1) / G;
   const int cap = nsm * (per_sm > 0 ? per_sm : 1);
   const int grid = need < cap ? need : cap;
-  return launch_pdl(pairs_kernel<R, G, LG, kJ, kU3>, grid, G * kThreads, sm, st, hs, pop, a, stage, xe);
+  return launch_pdl(pairs_kernel<R, G, LG, kJ, kU3>, grid, G * kThreads, sm, st, hs, pop, a,
+                    stage, xe);
 }
 
 template <class R, int LG, bool kJ>
@@ -1137,9 +1139,7 @@ static cudaError_t launch_pairs_x(const DevSys &hs, DevPop pop, const MoveArgs &
                      : launch_pairs_r<double, false>(hs, pop, a, st, nsm, optin, nullptr);
 }
 
-cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
-                         cudaStream_t st) {
-  (void)ds;
+cudaError_t launch_pairs(const DevSys &hs, DevPop pop, const MoveArgs &a, cudaStream_t st) {
   return launch_pairs_x(hs, pop, a, st, nullptr);
 }
 

@@ -84,8 +84,7 @@ cudaError_t launch_eval_real(const DevSys &hs, const DevSys *ds, int nw, const d
 // move scratch when MoveArgs::orb_inv is set (launch_orb_inv, otherwise
 // nothing), then the rest of the evaluation, the acceptance and the
 // averages (launch_move).
-cudaError_t launch_pairs(const DevSys &hs, const DevSys *ds, DevPop pop, const MoveArgs &a,
-                         cudaStream_t st);
+cudaError_t launch_pairs(const DevSys &hs, DevPop pop, const MoveArgs &a, cudaStream_t st);
 cudaError_t launch_orb_inv(const DevSys &hs, const DevSys *ds, const MoveArgs &a,
                            cudaStream_t st);
 // launch_orb_inv can run (DevSys::split_inv and a scratch region for it),

@@ -999,7 +999,12 @@ __global__ void __launch_bounds__(kB == 1 ? kSMaxThreads : 512, 1)
 // 45 + 45, 1024: 8 374, 10 364, 12 384; 61 + 61, a type per CTA: 8 749, 10 710, 12 698).
 int s_warps(int n, size_t smem) {
   const int ctas = 227 * 1024 / (int)(smem + 1024);
-  return ctas >= 8 ? 3 : ctas >= 5 ? 4 : ctas == 4 ? 6 : ctas == 3 || n <= 40 ? 8 : ctas == 2 ? n <= 45 ? 10 : 12 : 20;
+  if (ctas >= 8) return 3;
+  if (ctas >= 5) return 4;
+  if (ctas == 4) return 6;
+  if (ctas == 3 || n <= 40) return 8;
+  if (ctas == 2) return n <= 45 ? 10 : 12;
+  return 20;
 }
 
 cudaError_t launch_s(const DevSys &hs, const DevSys *ds, const RealArgs &a, int nw,
