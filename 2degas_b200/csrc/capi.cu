@@ -93,9 +93,11 @@ cudaError_t dalloc(T **p, size_t n) {
 }
 
 
-// Host-buffer evaluations whose configurations and results fit this go
-// through pinned staging memory: a call of 64 configurations of N = 26 took 148
-// us with copies from and to pageable memory, 98 staged (256: 273 and 150).
+// Host-buffer evaluations whose pageable buffers fit this go through pinned
+// staging memory: a call of 64 configurations of N = 26 with u3 took 132 us with
+// copies from and to pageable memory, 85 staged (256: 171 and 126). Buffers that
+// the caller has pinned are copied directly (78 and 96; staged all the same they
+// took 85 and 127).
 constexpr size_t kHostStageBytes = 4 << 20;
 
 // Whether `doubles` go through the staging memory, which the first such call
@@ -116,6 +118,14 @@ bool host_stage(qmc2d_handle *h, size_t doubles) {
     return false;
   }
   h->stage_doubles = n;
+  return true;
+}
+
+// Whether p is memory that CUDA does not know (a copy would stage it itself).
+bool pageable(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
   return true;
 }
 
@@ -807,36 +817,41 @@ extern "C" int qmc2d_compute_properties(qmc2d_handle *h, int nw, const double *x
   CK(cudaSetDevice(h->device));
   CK(join_side(h));
   const size_t N2 = 2 * (size_t)h->N, w = nw;
+  const double *const host[5] = {x, g, hl, props, s};
+  double *const dst[5] = {nullptr, g, hl, props, s};
+  double *const dev[5] = {h->d_x, h->d_g, h->d_h, h->d_p, h->d_s};
   const size_t len[5] = {N2 * w, N2 * w, (size_t)h->nt * w, (size_t)h->nprops * w, w};
-  const bool staged = host_stage(h, len[0] + len[1] + len[2] + len[3] + len[4]);
-  const double *src = x;
-  if (staged) {
-    std::memcpy(h->h_stage, x, sizeof(double) * len[0]);
-    src = h->h_stage;
+  // the pageable buffers' places in the staging memory, if that takes them all
+  double *at[5] = {};
+  bool paged[5];
+  size_t total = 0;
+  for (int k = 0; k < 5; k++) {
+    paged[k] = host[k] && pageable(host[k]);
+    if (paged[k]) total += len[k];
   }
+  if (total > 0 && host_stage(h, total)) {
+    double *next = h->h_stage;
+    for (int k = 0; k < 5; k++)
+      if (paged[k]) {
+        at[k] = next;
+        next += len[k];
+      }
+  }
+  if (at[0]) std::memcpy(at[0], x, sizeof(double) * len[0]);
   CK(cudaMemsetAsync(h->d_status, 0, sizeof(int) * nw, h->stream));
-  CK(cudaMemcpyAsync(h->d_x, src, sizeof(double) * len[0], cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->d_x, at[0] ? at[0] : x, sizeof(double) * len[0], cudaMemcpyHostToDevice,
+                     h->stream));
   {
     ProfScope ps(h, QMC2D_KERNEL_EVAL, h->stream);
     CK(evaluate(h, nw, h->d_x, h->d_g, h->d_h, h->d_p, h->d_s, h->stream));
   }
-  double *const dst[5] = {nullptr, g, hl, props, s};
-  const double *const dev[5] = {nullptr, h->d_g, h->d_h, h->d_p, h->d_s};
-  double *at = h->h_stage + len[0];
-  for (int k = 1; k < 5; k++) {
+  for (int k = 1; k < 5; k++)
     if (dst[k])
-      CK(cudaMemcpyAsync(staged ? at : dst[k], dev[k], sizeof(double) * len[k],
+      CK(cudaMemcpyAsync(at[k] ? at[k] : dst[k], dev[k], sizeof(double) * len[k],
                          cudaMemcpyDeviceToHost, h->stream));
-    at += len[k];
-  }
   const int st = sync_status(h, nw);
-  if (staged) {
-    at = h->h_stage + len[0];
-    for (int k = 1; k < 5; k++) {
-      if (dst[k]) std::memcpy(dst[k], at, sizeof(double) * len[k]);
-      at += len[k];
-    }
-  }
+  for (int k = 1; k < 5; k++)
+    if (at[k]) std::memcpy(dst[k], at[k], sizeof(double) * len[k]);
   return st;
 }
 
