@@ -817,26 +817,13 @@ extern "C" int qmc2d_compute_properties(qmc2d_handle *h, int nw, const double *x
   CK(cudaSetDevice(h->device));
   CK(join_side(h));
   const size_t N2 = 2 * (size_t)h->N, w = nw;
-  const double *const host[5] = {x, g, hl, props, s};
   double *const dst[5] = {nullptr, g, hl, props, s};
   double *const dev[5] = {h->d_x, h->d_g, h->d_h, h->d_p, h->d_s};
   const size_t len[5] = {N2 * w, N2 * w, (size_t)h->nt * w, (size_t)h->nprops * w, w};
-  // the pageable buffers' places in the staging memory, if that takes them all
+  // the pageable buffers' places in the staging memory
   double *at[5] = {};
-  bool paged[5];
-  size_t total = 0;
-  for (int k = 0; k < 5; k++) {
-    paged[k] = host[k] && pageable(host[k]);
-    if (paged[k]) total += len[k];
-  }
-  if (total > 0 && host_stage(h, total)) {
-    double *next = h->h_stage;
-    for (int k = 0; k < 5; k++)
-      if (paged[k]) {
-        at[k] = next;
-        next += len[k];
-      }
-  }
+  const bool paged = pageable(x);
+  if (paged && host_stage(h, len[0] + len[1] + len[2] + len[3] + len[4])) at[0] = h->h_stage;
   if (at[0]) std::memcpy(at[0], x, sizeof(double) * len[0]);
   CK(cudaMemsetAsync(h->d_status, 0, sizeof(int) * nw, h->stream));
   CK(cudaMemcpyAsync(h->d_x, at[0] ? at[0] : x, sizeof(double) * len[0], cudaMemcpyHostToDevice,
@@ -844,6 +831,22 @@ extern "C" int qmc2d_compute_properties(qmc2d_handle *h, int nw, const double *x
   {
     ProfScope ps(h, QMC2D_KERNEL_EVAL, h->stream);
     CK(evaluate(h, nw, h->d_x, h->d_g, h->d_h, h->d_p, h->d_s, h->stream));
+  }
+  // the results' buffers are looked at while the kernels run (0.4 us each); with
+  // x staged there is room for all, else none of it is in use
+  bool stage[5] = {};
+  size_t total = 0;
+  for (int k = 1; k < 5; k++) {
+    stage[k] = dst[k] && (!paged || at[0]) && pageable(dst[k]);
+    if (stage[k]) total += len[k];
+  }
+  if (total > 0 && (at[0] || host_stage(h, total))) {
+    double *next = h->h_stage + (at[0] ? len[0] : 0);
+    for (int k = 1; k < 5; k++)
+      if (stage[k]) {
+        at[k] = next;
+        next += len[k];
+      }
   }
   for (int k = 1; k < 5; k++)
     if (dst[k])
