@@ -394,9 +394,8 @@ __global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, in
       perm[k] = p;
       rowl[p] = k;
       rinv[p] = inv;
-      const double d = ps[kL * LS + 1];
-      dk[k] = d;
-      if ((best >> 8) == 0u || d != d) singular = 1;  // as the complex kernels of these spins
+      dk[k] = ps[kL * LS + 1];
+      if ((best >> 8) == 0u) singular = 1;
     }
     double fac[kR];
 #pragma unroll
@@ -505,6 +504,9 @@ __global__ void __launch_bounds__(kMaxT, kMB) real_inv_cta_kernel(RealArgs a, in
       Wt[k * ld + n + e - k * (ld - n)] = 0.0;
     }
   }
+  // a NaN pivot counts as none, as in the complex kernels of these spins (looked
+  // at here, off the chain of the pivot steps)
+  if (t < n && dk[t] != dk[t]) singular = 1;
   double lg = t < n ? log(dk[t]) : 0.0;
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) lg += __shfl_xor_sync(0xffffffffu, lg, q);
